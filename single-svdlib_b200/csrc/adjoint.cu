@@ -20,6 +20,7 @@
 #include <cstring>
 #include <vector>
 
+#include "dense_tall.cuh"
 #include "device_common.cuh"
 #include "ops.cuh"
 #include "svdb_internal.h"
@@ -128,93 +129,9 @@ static const DevCompressed& pattern_of(const svdb_matrix* a, bool& swapped) {
 }
 
 // ------------------------------------------------------- tall-skinny dense ----
-// C (p x q) = X^T Y for X (rows x p, ld ldx), Y (rows x q, ld ldy): blocks
-// take row chunks staged through shared memory; a 16 x 16 thread grid keeps
-// an NC x NC tile of C.  Block partials are summed in block order.
-constexpr int kAtbRows = 32;
-template <int NC>
-__global__ void __launch_bounds__(256) k_atb_part(const double* __restrict__ X, int64_t ldx,
-                                                  const double* __restrict__ Y, int64_t ldy, int64_t rows, int p,
-                                                  int q, int64_t chunk, double* __restrict__ part) {
-    extern __shared__ double sm[];
-    double* xs = sm;                 // kAtbRows x p
-    double* ys = sm + kAtbRows * p;  // kAtbRows x q
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int64_t r0 = blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
-    double acc[NC][NC];
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[i][j] = 0.0;
-    for (int64_t rb = r0; rb < r1; rb += kAtbRows) {
-        const int nr = (int)min((int64_t)kAtbRows, r1 - rb);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * p; t += blockDim.x) xs[t] = X[(rb + t / p) * ldx + t % p];
-        for (int t = threadIdx.x; t < nr * q; t += blockDim.x) ys[t] = Y[(rb + t / q) * ldy + t % q];
-        __syncthreads();
-        for (int r = 0; r < nr; ++r) {
-            double xa[NC], yb[NC];
-#pragma unroll
-            for (int i = 0; i < NC; ++i) {
-                const int a = ty + 16 * i, b = tx + 16 * i;
-                xa[i] = a < p ? xs[r * p + a] : 0.0;
-                yb[i] = b < q ? ys[r * q + b] : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < NC; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j) acc[i][j] = fma(xa[i], yb[j], acc[i][j]);
-        }
-    }
-    double* o = part + (int64_t)blockIdx.x * p * q;
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            const int a = ty + 16 * i, b = tx + 16 * j;
-            if (a < p && b < q) o[a * q + b] = acc[i][j];
-        }
-}
-
-__global__ void k_sum_parts(const double* __restrict__ part, int nblocks, int count, double* __restrict__ out) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
-        double s0 = 0.0, s1 = 0.0;
-        int b = 0;
-        for (; b + 2 <= nblocks; b += 2) {
-            s0 += part[(int64_t)b * count + e];
-            s1 += part[(int64_t)(b + 1) * count + e];
-        }
-        if (b < nblocks) s0 += part[(int64_t)b * count + e];
-        out[e] = s0 + s1;
-    }
-}
-
-// Out (rows x q, ld ldo) = beta * Y + alpha * X diag(d) C, X: rows x p (ld
-// ldx), C: p x q row-major, d: p values or null (= 1), Y null when beta = 0.
-// Out may be Y (each element is read, then written, by one thread).
-constexpr int kGtRows = 32;
-__global__ void __launch_bounds__(256) k_gemm_tall(const double* __restrict__ X, int64_t ldx, int64_t rows, int p,
-                                                   const double* __restrict__ C, const double* __restrict__ d, int q,
-                                                   double alpha, const double* Y, int64_t ldy, double beta,
-                                                   double* Out, int64_t ldo) {
-    extern __shared__ double sm[];
-    double* cs = sm;          // p x q, rows scaled by d
-    double* xs = sm + p * q;  // kGtRows x p
-    for (int t = threadIdx.x; t < p * q; t += blockDim.x) cs[t] = d ? d[t / q] * C[t] : C[t];
-    for (int64_t r0 = (int64_t)blockIdx.x * kGtRows; r0 < rows; r0 += (int64_t)gridDim.x * kGtRows) {
-        const int nr = (int)min((int64_t)kGtRows, rows - r0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * p; t += blockDim.x) xs[t] = X[(r0 + t / p) * ldx + t % p];
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * q; t += blockDim.x) {
-            const int rr = t / q, j = t % q;
-            double s = 0.0;
-            for (int k = 0; k < p; ++k) s = fma(xs[rr * p + k], cs[k * q + j], s);
-            const int64_t row = r0 + rr;
-            const double y = (beta != 0.0) ? beta * Y[row * ldy + j] : 0.0;
-            Out[row * ldo + j] = y + alpha * s;
-        }
-    }
+// column of flat index t of a k-column matrix (32-bit division where it fits)
+__device__ __forceinline__ int col_of(int64_t t, int k) {
+    return t < ((int64_t)1 << 32) ? (int)((uint32_t)t % (uint32_t)k) : (int)(t % k);
 }
 
 // Out[r][j] = ca[j] A[r][j] + sb cb[j] B[r][j]; ca / cb null mean 1, B null
@@ -224,83 +141,98 @@ __global__ void k_axpby_cols(int64_t rows, int k, double* Out, int64_t ldo, cons
                              const double* __restrict__ cb, double sb) {
     const int64_t total = rows * k;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / k;
-        const int j = (int)(t % k);
+        const int j = col_of(t, k);
+        const int64_t r = t < ((int64_t)1 << 32) ? (int64_t)((uint32_t)t / (uint32_t)k) : t / k;
         double v = A[r * lda + j] * (ca ? ca[j] : 1.0);
         if (B) v += sb * (cb ? cb[j] : 1.0) * B[r * ldb + j];
         Out[r * ldo + j] = v;
     }
 }
 
-__global__ void k_diag(const double* __restrict__ C, int k, double* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < k) out[j] = C[j * k + j];
+// X += P diag(alpha), R -= W diag(alpha), one pass
+__global__ void k_cg_step(int64_t rows, int k, double* __restrict__ X, const double* __restrict__ P,
+                          double* __restrict__ R, const double* __restrict__ W, const double* __restrict__ alpha) {
+    const int64_t total = rows * k;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const double al = alpha[col_of(t, k)];
+        X[t] += al * P[t];
+        R[t] += -1.0 * al * W[t];
+    }
 }
 
-// CG scalars per column.  A column is frozen (alpha = beta = 0) once its
-// residual norm is below freeze * ||rhs||, or when a denominator is not positive.
-__global__ void k_cg_alpha(const double* __restrict__ rr, const double* __restrict__ pw,
-                           const double* __restrict__ rhs_norm, double freeze, int k, double* __restrict__ alpha) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    const bool live = rr[j] > 0.0 && pw[j] > 0.0 && sqrt(rr[j]) > freeze * rhs_norm[j];
-    alpha[j] = live ? rr[j] / pw[j] : 0.0;
-}
-__global__ void k_cg_beta(const double* __restrict__ rr_new, double* __restrict__ rr, const double* __restrict__ alpha,
-                          int k, double* __restrict__ beta) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    beta[j] = (alpha[j] != 0.0 && rr[j] > 0.0) ? rr_new[j] / rr[j] : 0.0;
-    rr[j] = rr_new[j];
+// The column sums `tot` of the CTAs' partials dots (nb x k), one warp per
+// column in a fixed order, then the CG scalars of the column.  A column is
+// frozen (alpha = beta = 0) once its residual norm is below freeze * ||rhs||,
+// or when a denominator is not positive.
+//   CG_INIT   rr = tot
+//   CG_ALPHA  alpha = rr / tot (tot = p . w)
+//   CG_BETA   beta = tot / rr, rr = tot (tot = r . r)
+enum { CG_INIT, CG_ALPHA, CG_BETA };
+template <int WHAT>
+__global__ void k_cg_scalars(const double* __restrict__ dots, int nb, int k, double* __restrict__ rr,
+                             const double* __restrict__ rhs_norm, double freeze, double* __restrict__ alpha,
+                             double* __restrict__ beta) {
+    const int lane = threadIdx.x & 31, nw = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < k; j += nw) {
+        double tot = 0.0;
+        for (int b = lane; b < nb; b += 32) tot += dots[(int64_t)b * k + j];
+        tot = warp_sum(tot);
+        if (lane) continue;
+        if (WHAT == CG_INIT) {
+            rr[j] = tot;
+        } else if (WHAT == CG_ALPHA) {
+            const bool live = rr[j] > 0.0 && tot > 0.0 && sqrt(rr[j]) > freeze * rhs_norm[j];
+            alpha[j] = live ? rr[j] / tot : 0.0;
+        } else {
+            beta[j] = (alpha[j] != 0.0 && rr[j] > 0.0) ? tot / rr[j] : 0.0;
+            rr[j] = tot;
+        }
+    }
 }
 
+// The tall products of an iteration go through dense_tall.cuh (FP64 matrix
+// instruction).  What it measured on 50,000 x 20,000, k = 32, per launch
+// before and after: X^T Y 25-37 -> 8-12 us, the sum of its partials 75 -> 5 us
+// (eight blocks of one thread per element, held by load latency), X C 25 ->
+// 13-18 us; the k x k Grams formed for their diagonals became column sums in
+// the products' epilogues.  Adjoint 37.7 -> 22.2 ms.
 struct TallCtx {
     cudaStream_t s;
-    DevBuf<double> part;
+    DevBuf<double> part, dots;
+    int nb = 0;  // CTAs that wrote dots
 };
 
+// C (p x q) = X^T Y, X: rows x p (ld ldx), Y: rows x q (ld ldy)
 static void atb(TallCtx& cx, const double* X, int64_t ldx, const double* Y, int64_t ldy, int64_t rows, int p, int q,
                 double* C) {
-    const int nc = (std::max(p, q) + 15) / 16;
-    if (nc > 8) throw Error(SVDB_ERR_UNSUPPORTED, "adjoint: more than 128 triplets");
-    const int sms = device_props().sms;
-    const int64_t chunk = std::max<int64_t>(kAtbRows * 4, (rows + sms * 2 - 1) / (sms * 2));
-    const int nblk = (int)std::max<int64_t>(1, (rows + chunk - 1) / chunk);
-    if ((int64_t)cx.part.n < (int64_t)nblk * p * q) cx.part.alloc((size_t)nblk * p * q, cx.s);
-    const size_t smem = (size_t)kAtbRows * (p + q) * sizeof(double);
-#define SVDB_ATB_CASE(N)                                                                                     \
-    case N:                                                                                                  \
-        if (smem > 48 * 1024)                                                                                \
-            SVDB_CUDA(cudaFuncSetAttribute(k_atb_part<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
-                                           (int)smem));                                                      \
-        k_atb_part<N><<<nblk, 256, smem, cx.s>>>(X, ldx, Y, ldy, rows, p, q, chunk, cx.part.p);               \
-        break;
-    switch (nc) {
-        SVDB_ATB_CASE(1)
-        SVDB_ATB_CASE(2)
-        SVDB_ATB_CASE(3)
-        SVDB_ATB_CASE(4)
-        SVDB_ATB_CASE(5)
-        SVDB_ATB_CASE(6)
-        SVDB_ATB_CASE(7)
-        SVDB_ATB_CASE(8)
-    }
-#undef SVDB_ATB_CASE
-    k_sum_parts<<<grid_for_work((int64_t)p * q, 128), 128, 0, cx.s>>>(cx.part.p, nblk, p * q, C);
-    SVDB_CHECK_LAUNCH_N(2);
+    if (std::max(p, q) > 128) throw Error(SVDB_ERR_UNSUPPORTED, "adjoint: more than 128 triplets");
+    const TnShape h = tn_shape(rows, p, q, false, device_props().sms);
+    if ((int64_t)cx.part.n < (int64_t)h.blocks * p * q) cx.part.alloc((size_t)h.blocks * p * q, cx.s);
+    tn_launch(h, X, ldx, p, Y, ldy, q, rows, cx.part.p, C, nullptr, cx.s);
 }
 
-static void gemm_tall(const double* X, int64_t ldx, int64_t rows, int p, const double* C, const double* d, int q,
-                      double alpha, const double* Y, int64_t ldy, double beta, double* Out, int64_t ldo,
-                      cudaStream_t s) {
-    if (rows == 0) return;
-    const size_t smem = ((size_t)p * q + (size_t)kGtRows * p) * sizeof(double);
-    if (smem > 200 * 1024) throw Error(SVDB_ERR_UNSUPPORTED, "adjoint: factor wider than the shared-memory tile");
-    if (smem > 48 * 1024)
-        SVDB_CUDA(cudaFuncSetAttribute(k_gemm_tall, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int blocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>((rows + kGtRows - 1) / kGtRows, (int64_t)device_props().sms * 4));
-    k_gemm_tall<<<blocks, 256, smem, s>>>(X, ldx, rows, p, C, d, q, alpha, Y, ldy, beta, Out, ldo);
+// Out (rows x q, ld ldo) = beta * Y + alpha * X diag(d) C + E diag(es), X: rows x p
+// (ld ldx), C: p x q row-major, d: p values or null (= 1), Y / E null: no such
+// term.  Out may be Y.  DOT 1 / 2: the column sums of Out * Out / Out * E are
+// left as cx.nb partials in cx.dots.
+template <int DOT = 0>
+static void gemm_tall(TallCtx& cx, const double* X, int64_t ldx, int64_t rows, int p, const double* C, const double* d,
+                      int q, double alpha, const double* Y, int64_t ldy, double beta, double* Out, int64_t ldo,
+                      const double* E = nullptr, int64_t lde = 0, const double* es = nullptr) {
+    const int sms = device_props().sms;
+    if (DOT) {
+        cx.nb = nn_blocks(rows, sms);
+        if ((int64_t)cx.dots.n < (int64_t)cx.nb * q) cx.dots.alloc((size_t)cx.nb * q, cx.s);
+    }
+    nn_launch<DOT>(NnArgs<double, double>{X, ldx, rows, p, C, q, d, q, 0, alpha, beta != 0.0 ? Y : nullptr, ldy, beta,
+                                          E, lde, es, Out, ldo, 0, cx.dots.p, nullptr},
+                   sms, cx.s);
+}
+
+template <int WHAT>
+static void cg_scalars(TallCtx& cx, int k, double* rr, const double* rhs_norm, double freeze, double* alpha,
+                       double* beta) {
+    k_cg_scalars<WHAT><<<(k + 7) / 8, 256, 0, cx.s>>>(cx.dots.p, cx.nb, k, rr, rhs_norm, freeze, alpha, beta);
     SVDB_CHECK_LAUNCH();
 }
 
@@ -385,16 +317,14 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     SVDB_CUDA(cudaMemcpyAsync(hJ.data(), JU, 2 * k * k * 8, cudaMemcpyDeviceToHost, s));
 
     // per-column vectors on the device: s, s^2, 1/s and CG scalars
-    DevBuf<double> colv(9 * k, s);
+    DevBuf<double> colv(7 * k, s);
     double* d_s = colv.p;
     double* d_s2 = colv.p + k;
     double* d_si = colv.p + 2 * k;
     double* d_rr = colv.p + 3 * k;
-    double* d_rrn = colv.p + 4 * k;
-    double* d_pw = colv.p + 5 * k;
-    double* d_al = colv.p + 6 * k;
-    double* d_be = colv.p + 7 * k;
-    double* d_rhsn = colv.p + 8 * k;
+    double* d_al = colv.p + 4 * k;
+    double* d_be = colv.p + 5 * k;
+    double* d_rhsn = colv.p + 6 * k;
     std::vector<double> hcol(3 * k);
     for (int i = 0; i < kk; ++i) {
         hcol[i] = sv[i];
@@ -405,8 +335,8 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
 
     // a = (I - U U^T) g_U,  b = (I - V V^T) g_V
     DevBuf<double> Aa(m * k, s), Bb(n * k, s);
-    gemm_tall(U.p, k, m, kk, JU, nullptr, kk, -1.0, GU.p, k, 1.0, Aa.p, k, s);
-    gemm_tall(V.p, k, n, kk, JV, nullptr, kk, -1.0, GV.p, k, 1.0, Bb.p, k, s);
+    gemm_tall(cx, U.p, k, m, kk, JU, nullptr, kk, -1.0, GU.p, k, 1.0, Aa.p, k);
+    gemm_tall(cx, V.p, k, n, kk, JV, nullptr, kk, -1.0, GV.p, k, 1.0, Bb.p, k);
 
     const DevCompressed& Ar = csr_of(A);  // rows of A
     const DevCompressed& Ac = csc_of(A);  // rows of A^T
@@ -414,30 +344,25 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     DevBuf<double> Rhs(n * k, s), Z(n * k, s), T(m * k, s);
     spmm_dev<double, double>(Ac, false, Aa.p, kk, Z.p, s);
     atb(cx, V.p, k, Z.p, k, n, kk, kk, C1);
-    gemm_tall(V.p, k, n, kk, C1, nullptr, kk, -1.0, Z.p, k, 1.0, Z.p, k, s);
-    axpby_cols(n, kk, Rhs.p, k, Bb.p, k, d_s, Z.p, k, nullptr, 1.0, s);
+    gemm_tall(cx, V.p, k, n, kk, C1, nullptr, kk, -1.0, Z.p, k, 1.0, Rhs.p, k, Bb.p, k, d_s);
 
-    // W = (S^2 - A_p^T A_p) P
-    auto apply_op = [&](const double* P, double* W) {
-        spmm_dev<double, double>(Ar, false, P, kk, T.p, s);                        // T = A P
-        atb(cx, V.p, k, P, k, n, kk, kk, C1);                                       // C1 = V^T P
-        gemm_tall(U.p, k, m, kk, C1, d_s, kk, -1.0, T.p, k, 1.0, T.p, k, s);        // T -= U S C1
-        spmm_dev<double, double>(Ac, false, T.p, kk, Z.p, s);                       // Z = A^T T
-        atb(cx, U.p, k, T.p, k, m, kk, kk, C2);                                     // C2 = U^T T
-        gemm_tall(V.p, k, n, kk, C2, d_s, kk, -1.0, Z.p, k, 1.0, Z.p, k, s);        // Z -= V S C2
-        axpby_cols(n, kk, W, k, P, k, d_s2, Z.p, k, nullptr, -1.0, s);              // W = P S^2 - Z
-    };
-
-    // block CG, X = 0, R = P = rhs
+    // block CG on S^2 - A_p^T A_p: X = 0, R = P = rhs
     DevBuf<double> X(n * k, s), R(n * k, s), P(n * k, s), W(n * k, s);
     SVDB_CUDA(cudaMemsetAsync(X.p, 0, n * k * 8, s));
     SVDB_CUDA(cudaMemcpyAsync(R.p, Rhs.p, n * k * 8, cudaMemcpyDeviceToDevice, s));
     SVDB_CUDA(cudaMemcpyAsync(P.p, Rhs.p, n * k * 8, cudaMemcpyDeviceToDevice, s));
-    atb(cx, R.p, k, R.p, k, n, kk, kk, C1);
-    k_diag<<<(kk + 127) / 128, 128, 0, s>>>(C1, kk, d_rr);
-    SVDB_CHECK_LAUNCH();
-    std::vector<double> rhs_norm(k), rr(k);
-    SVDB_CUDA(cudaMemcpyAsync(rr.data(), d_rr, k * 8, cudaMemcpyDeviceToHost, s));
+    // page-locked: the residual's copy does not hold the host, which enqueues on
+    struct HostBuf {
+        double* p;
+        ~HostBuf() { host_result_free(p); }
+    } hrr{(double*)host_result_alloc(64 << 10)};
+    double* rr = hrr.p;
+    // column norms of rhs as the dots of R with itself (C1 = 0: the product adds nothing)
+    SVDB_CUDA(cudaMemsetAsync(C1, 0, k * k * 8, s));
+    gemm_tall<1>(cx, V.p, k, n, kk, C1, nullptr, kk, 0.0, R.p, k, 1.0, W.p, k);
+    cg_scalars<CG_INIT>(cx, kk, d_rr, nullptr, 0.0, nullptr, nullptr);
+    std::vector<double> rhs_norm(k);
+    SVDB_CUDA(cudaMemcpyAsync(rr, d_rr, k * 8, cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
     for (int j = 0; j < kk; ++j) rhs_norm[j] = std::sqrt(rr[j]);
     SVDB_CUDA(cudaMemcpyAsync(d_rhsn, rhs_norm.data(), k * 8, cudaMemcpyHostToDevice, s));
@@ -451,26 +376,33 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     };
     double res = residual();
     uint64_t it = 0;
+    cudaEvent_t got;  // the residual's copy
+    SVDB_CUDA(cudaEventCreateWithFlags(&got, cudaEventDisableTiming));
+    if (res > tol && it < max_it) spmm_dev<double, double>(Ar, false, P.p, kk, T.p, s);  // T = A P
     while (res > tol && it < max_it) {
-        apply_op(P.p, W.p);
-        atb(cx, P.p, k, W.p, k, n, kk, kk, C1);
-        k_diag<<<(kk + 127) / 128, 128, 0, s>>>(C1, kk, d_pw);
-        k_cg_alpha<<<(kk + 127) / 128, 128, 0, s>>>(d_rr, d_pw, d_rhsn, 0.25 * tol, kk, d_al);
-        SVDB_CHECK_LAUNCH_N(2);
-        axpby_cols(n, kk, X.p, k, X.p, k, nullptr, P.p, k, d_al, 1.0, s);   // X += P alpha
-        axpby_cols(n, kk, R.p, k, R.p, k, nullptr, W.p, k, d_al, -1.0, s);  // R -= W alpha
-        atb(cx, V.p, k, R.p, k, n, kk, kk, C2);                               // keep R off span(V)
-        gemm_tall(V.p, k, n, kk, C2, nullptr, kk, -1.0, R.p, k, 1.0, R.p, k, s);
-        atb(cx, R.p, k, R.p, k, n, kk, kk, C1);
-        k_diag<<<(kk + 127) / 128, 128, 0, s>>>(C1, kk, d_rrn);
-        k_cg_beta<<<(kk + 127) / 128, 128, 0, s>>>(d_rrn, d_rr, d_al, kk, d_be);
-        SVDB_CHECK_LAUNCH_N(2);
-        axpby_cols(n, kk, P.p, k, R.p, k, nullptr, P.p, k, d_be, 1.0, s);   // P = R + P beta
-        SVDB_CUDA(cudaMemcpyAsync(rr.data(), d_rr, k * 8, cudaMemcpyDeviceToHost, s));
-        SVDB_CUDA(cudaStreamSynchronize(s));
+        atb(cx, V.p, k, P.p, k, n, kk, kk, C1);                                           // C1 = V^T P
+        gemm_tall(cx, U.p, k, m, kk, C1, d_s, kk, -1.0, T.p, k, 1.0, T.p, k);             // T -= U S C1
+        spmm_dev<double, double>(Ac, false, T.p, kk, Z.p, s);                             // Z = A^T T
+        atb(cx, U.p, k, T.p, k, m, kk, kk, C2);                                           // C2 = U^T T
+        // W = P S^2 - (Z - V S C2), with the sums of P * W
+        gemm_tall<2>(cx, V.p, k, n, kk, C2, d_s, kk, 1.0, Z.p, k, -1.0, W.p, k, P.p, k, d_s2);
+        cg_scalars<CG_ALPHA>(cx, kk, d_rr, d_rhsn, 0.25 * tol, d_al, nullptr);
+        k_cg_step<<<grid_for_work(n * k, 256), 256, 0, s>>>(n, kk, X.p, P.p, R.p, W.p, d_al);
+        SVDB_CHECK_LAUNCH();
+        atb(cx, V.p, k, R.p, k, n, kk, kk, C2);                                           // keep R off span(V)
+        gemm_tall<1>(cx, V.p, k, n, kk, C2, nullptr, kk, -1.0, R.p, k, 1.0, R.p, k);
+        cg_scalars<CG_BETA>(cx, kk, d_rr, nullptr, 0.0, d_al, d_be);
+        axpby_cols(n, kk, P.p, k, R.p, k, nullptr, P.p, k, d_be, 1.0, s);                 // P = R + P beta
+        SVDB_CUDA(cudaMemcpyAsync(rr, d_rr, k * 8, cudaMemcpyDeviceToHost, s));
+        SVDB_CUDA(cudaEventRecord(got, s));
+        // the next iteration's first product (of the last one after the end:
+        // T = A X below overwrites it) runs while the host looks at the residual
+        spmm_dev<double, double>(Ar, false, P.p, kk, T.p, s);
+        SVDB_CUDA(cudaEventSynchronize(got));
         ++it;
         res = residual();
     }
+    cudaEventDestroy(got);
     o.cg_iterations = it;
     o.cg_residual = res;
 
@@ -478,9 +410,9 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     DevBuf<double> Gm(m * k, s);
     spmm_dev<double, double>(Ar, false, X.p, kk, T.p, s);
     atb(cx, V.p, k, X.p, k, n, kk, kk, C1);
-    gemm_tall(U.p, k, m, kk, C1, d_s, kk, -1.0, T.p, k, 1.0, T.p, k, s);
+    gemm_tall(cx, U.p, k, m, kk, C1, d_s, kk, -1.0, T.p, k, 1.0, T.p, k);
     atb(cx, U.p, k, T.p, k, m, kk, kk, C2);  // A_p Delta lies off span(U): drop the rounding residue
-    gemm_tall(U.p, k, m, kk, C2, nullptr, kk, -1.0, T.p, k, 1.0, T.p, k, s);
+    gemm_tall(cx, U.p, k, m, kk, C2, nullptr, kk, -1.0, T.p, k, 1.0, T.p, k);
     axpby_cols(m, kk, Gm.p, k, Aa.p, k, d_si, T.p, k, d_si, 1.0, s);
 
     // M on the host
@@ -488,8 +420,6 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     {
         const double* hJU = hJ.data();
         const double* hJV = hJ.data() + k * k;
-        double smax2 = 0.0;
-        for (int i = 0; i < kk; ++i) smax2 = std::max(smax2, sv[i] * sv[i]);
         for (int i = 0; i < kk; ++i)
             for (int j = 0; j < kk; ++j) {
                 if (i == j) { M[i * k + j] = gs[i]; continue; }
@@ -499,7 +429,6 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
                 const double avv = hJV[i * k + j] - hJV[j * k + i];
                 M[i * k + j] = f * au * sv[j] + sv[i] * f * avv;
             }
-        (void)smax2;
     }
     DevBuf<double> dM(k * k, s);
     SVDB_CUDA(cudaMemcpyAsync(dM.p, M.data(), k * k * 8, cudaMemcpyHostToDevice, s));
@@ -507,7 +436,7 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     // factors: Lf = [U M + Gamma | U] (m x 2k), Rf = [V | Delta] (n x 2k)
     const int rank = 2 * kk;
     DevBuf<double> Lf(m * rank, s), Rf(n * rank, s);
-    gemm_tall(U.p, k, m, kk, dM.p, nullptr, kk, 1.0, Gm.p, k, 1.0, Lf.p, rank, s);
+    gemm_tall(cx, U.p, k, m, kk, dM.p, nullptr, kk, 1.0, Gm.p, k, 1.0, Lf.p, rank);
     axpby_cols(m, kk, Lf.p + k, rank, U.p, k, nullptr, nullptr, 0, nullptr, 0.0, s);
     axpby_cols(n, kk, Rf.p, rank, V.p, k, nullptr, nullptr, 0, nullptr, 0.0, s);
     axpby_cols(n, kk, Rf.p + k, rank, X.p, k, nullptr, nullptr, 0, nullptr, 0.0, s);
