@@ -27,7 +27,7 @@ int group_for(double avg) {
 
 // --------------------------------------------------------------- SpMV ----
 // One launch: every block first takes its share of the rows of more than
-// kSegNnz entries (one block per row, the plan's multi rows), then its warps
+// kSegNnz entries (one block per row, the plan's long rows), then its warps
 // take the other rows through the length bins.  The grid is one wave of
 // resident blocks, so the two parts overlap and no partial wave trails.
 template <typename VT>
@@ -76,15 +76,15 @@ void spmv(const DevCompressed& m, bool fp32, const double* x, double* y, cudaStr
     if (m.nmajor == 0) return;
     const bool f = fp32 && m.val32.p;
     if (allow_sliced && !sliced_off() && spmv_sliced(m, f, x, y, s)) return;
-    const int64_t work = std::max<int64_t>(m.plan.bins.items[kSpmvBins] / 8, m.plan.nmulti);
+    const int64_t work = std::max<int64_t>(m.plan.bins.items[kSpmvBins] / 8, m.plan.nlong);
     if (f) {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<float>()));
-        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, m.plan.multi_rows.p,
-                                             m.plan.nmulti, x, y);
+        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, m.plan.long_rows.p,
+                                             m.plan.nlong, x, y);
     } else {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<double>()));
-        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, m.plan.multi_rows.p,
-                                              m.plan.nmulti, x, y);
+        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, m.plan.long_rows.p,
+                                              m.plan.nlong, x, y);
     }
     SVDB_CHECK_LAUNCH();
 }

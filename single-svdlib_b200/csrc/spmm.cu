@@ -2,7 +2,7 @@
 // dense products of randomized_svd (masked.rs:265-733) and the sigma/u step
 // of ritvec (mod.rs:1197-1210).
 //
-// Work unit: a row segment of at most kSegNnz entries (SegPlan), so rows of
+// Work unit: a row segment (SegPlan, at most kSegNnz entries), so rows of
 // any length spread over warps evenly; rows cut into several segments write
 // per-segment partials that a second kernel adds in segment order, keeping
 // the result deterministic.  Inside a warp, H groups of 32/H lanes each take
@@ -168,195 +168,197 @@ __global__ void __launch_bounds__(256, sizeof(XT) == 4 ? 4 : 3) k_spmm_seg(const
 }
 
 // Lean gather kernel: values and dense operand of one type T (float or
-// double), l <= 64 (H = 2) or <= 32 (H = 4), rows of X 16-byte aligned: the
-// same segments, lane groups and summation order as k_spmm_seg (group g takes
-// entries g, g + H, ... of a 32-entry chunk; FP32 sums within a chunk and
-// FP64 across chunks for float, FP64 throughout for double), with fewer
-// instructions per entry.  k_spmm_seg spent about 21 warp instructions per
-// nonzero at FP32 (its shuffles, 64-bit address arithmetic and per-entry
-// bounds tests), and with X resident in L1 it was bound by instruction issue,
-// not by memory.  Here a chunk's (row offset, value) pairs are written once to
-// a per-warp shared buffer and read back by broadcast, offsets are 32-bit, and
-// full chunks run without bounds tests with U gathers in flight per lane.
-constexpr int kF32Warps = 8;
+// double), rows of X 16-byte aligned and a multiple of 16 bytes apart.  A warp
+// takes a segment; its H groups of GL = 32 / H lanes take entries g, g + H, ...
+// of each 32-entry chunk, and a lane owns NL vectors of VEC = 16 / sizeof(T)
+// columns, GL * VEC columns apart, so that every gather instruction reads
+// contiguous bytes of a row.  FP32 sums within a chunk and FP64 across chunks
+// for float, FP64 throughout for double: the summation order of k_spmm_seg.
+//
+// What bounds it: the gathered rows, through L1 and L2 (15-17 TB/s of rows).
+// At FP64 a lane that owned four neighbouring columns read them as two 16-byte
+// loads at a 32-byte stride, so each load touched every sector of the row: L1
+// at 97 % of its peak, half of it for bytes already read.  With the vectors
+// GL * VEC apart the same loads are dense: 1,133 -> 914 us for A X of
+// 50,000 x 30,000, 28 M nonzeros, l = 60.
+//
+// A chunk's row offsets and values are written once to per-warp shared
+// buffers, a group's entries side by side, and read back four at a time by
+// broadcast (a 16-byte struct per entry took an LDS.128 each, 914 -> 812 us).
+// Offsets are 32-bit byte offsets from X where X is below 4 GB (BYTES: one add
+// per gather), else element offsets.  A chunk runs U gathers per lane at a
+// time, all issued before they are used; the last chunk of a segment runs
+// masked batches of four (one entry after another, a short last chunk cost
+// as much as a full one).  Tried and not kept: loading the next segment's
+// bounds and first chunk ahead (928 us), and segments ordered by length with a
+// CTA's warps starting together, which raised the L1 hits from 7 to 26 % and
+// gained 3 % on long rows but lost 10 % on A^T X.
+constexpr int kLeanWarps = 8;
 template <typename T>
-struct LeanEntry;
+struct LeanVec;
 template <>
-struct alignas(8) LeanEntry<float> { int32_t off; float v; };
+struct alignas(16) LeanVec<float> { float v[4]; };
 template <>
-struct alignas(16) LeanEntry<double> { int32_t off; int32_t pad; double v; };
-
-// four consecutive elements of a row (16-byte aligned)
-__device__ __forceinline__ void load4(const float* p, float (&x)[4]) {
-    const float4 t = *reinterpret_cast<const float4*>(p);
-    x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+struct alignas(16) LeanVec<double> { double v[2]; };
+template <typename T>
+__device__ __forceinline__ void lean_values4(const T* p, T (&v)[4]) {  // four consecutive shared values
+    constexpr int VEC = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int i = 0; i < 4 / VEC; ++i) {
+        const LeanVec<T> t = reinterpret_cast<const LeanVec<T>*>(p)[i];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) v[i * VEC + e] = t.v[e];
+    }
 }
-__device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
-    const double2 t0 = reinterpret_cast<const double2*>(p)[0], t1 = reinterpret_cast<const double2*>(p)[1];
-    x[0] = t0.x; x[1] = t0.y; x[2] = t1.x; x[3] = t1.y;
-}
 
-template <typename T, typename OT, int H, int U, int MINB>
-__global__ void __launch_bounds__(kF32Warps * 32, MINB)
+template <typename T, typename OT, int H, int NL, int U, int MINB, bool BYTES>
+__global__ void __launch_bounds__(kLeanWarps * 32, MINB)
     k_spmm_lean(const int32_t* __restrict__ ci, const T* __restrict__ val, const int32_t* __restrict__ seg_row,
                 const int64_t* __restrict__ seg_beg, const int64_t* __restrict__ seg_end, int64_t nseg,
-                const T* __restrict__ X, int32_t ldx, int l, OT* __restrict__ Y, int64_t ldy,
+                const T* __restrict__ X, uint32_t ldx, int l, OT* __restrict__ Y, int64_t ldy, int yvec,
                 double* __restrict__ part) {
     using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
-    constexpr int GL = 32 / H;           // lanes per group
-    constexpr int PER = 32 / H;          // entries of a chunk per group
-    __shared__ LeanEntry<T> s_ent[kF32Warps][32];
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int GL = 32 / H;   // lanes per group
+    constexpr int PER = 32 / H;  // entries of a chunk per group
+    constexpr int VS = PER + (sizeof(T) == 8 && H > 1 ? 2 : 0);  // a group's values, off the others' banks
+    static_assert(U % 4 == 0 && U <= PER, "batches of whole quads");
+    __shared__ __align__(16) uint32_t s_off[kLeanWarps][32];
+    __shared__ __align__(16) T s_val[kLeanWarps][H * VS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int g = lane / GL, gl = lane % GL;
-    const int col0 = gl * 4;
-    const int ncols_here = (l - col0) < 4 ? (l - col0) : 4;
-    const bool active = ncols_here > 0;
-    const uint32_t c0a = active ? (uint32_t)col0 : 0u;  // gathers at X + a 32-bit offset
-    LeanEntry<T>* E = s_ent[w];
+    bool active[NL];
+    uint32_t col[NL];
+#pragma unroll
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * VEC;
+        active[j] = c < l;
+        col[j] = active[j] ? (uint32_t)c : 0u;
+    }
+    const uint32_t scale = BYTES ? ldx * (uint32_t)sizeof(T) : ldx;
+    uint32_t* const oput = s_off[w] + (lane % H) * PER + lane / H;
+    T* const vput = s_val[w] + (lane % H) * VS + lane / H;
+    const uint32_t* const og = s_off[w] + g * PER;
+    const T* const vg = s_val[w] + g * VS;
+    auto gather = [&](uint32_t off, int j) {
+        if constexpr (BYTES)
+            return *reinterpret_cast<const LeanVec<T>*>(reinterpret_cast<const char*>(X) +
+                                                        (off + col[j] * (uint32_t)sizeof(T)));
+        else
+            return *reinterpret_cast<const LeanVec<T>*>(X + (off + col[j]));
+    };
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t sg = gwarp; sg < nseg; sg += nwarps) {
         const int32_t rr = __ldg(seg_row + sg);
-        const int64_t a = __ldg(seg_beg + sg), b = __ldg(seg_end + sg);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        const int64_t a = __ldg(seg_beg + sg);
+        int left = (int)(__ldg(seg_end + sg) - a);
+        const int32_t* cp = ci + a + lane;
+        const T* vp = val + a + lane;
+        double acc[NL][VEC];
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[j][e] = 0.0;
         int32_t myc = 0;
         T myv = T(0);
-        if (a + lane < b) { myc = __ldg(ci + a + lane); myv = __ldg(val + a + lane); }
-        for (int64_t k0 = a; k0 < b; k0 += 32) {
-            const int cnt = (b - k0) < 32 ? (int)(b - k0) : 32;
+        if (lane < left) { myc = __ldg(cp); myv = __ldg(vp); }
+        for (; left > 0; left -= 32) {
             __syncwarp();  // the previous chunk's entries have been read
-            LeanEntry<T> en;
-            en.off = myc * ldx;
-            en.v = myv;
-            E[lane] = en;
+            *oput = (uint32_t)myc * scale;
+            *vput = myv;
             __syncwarp();
-            if (k0 + 32 + lane < b) {  // the next chunk's pairs, while this one is used
-                myc = __ldg(ci + k0 + 32 + lane);
-                myv = __ldg(val + k0 + 32 + lane);
-            }
-            CT c4[4] = {CT(0), CT(0), CT(0), CT(0)};
-            if (cnt == 32) {
+            cp += 32;
+            vp += 32;
+            if (lane + 32 < left) { myc = __ldg(cp); myv = __ldg(vp); }  // the next chunk's, while this one is used
+            CT cs[NL][VEC];
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
+            if (left >= 32) {
 #pragma unroll 1
-                for (int qb = 0; qb < PER; qb += U) {  // batches of U gathers, one batch live at a time
-                    T xv[U][4];
+                for (int qb = 0; qb < PER; qb += U) {  // one batch live at a time
+                    LeanVec<T> xv[U][NL];
                     T vv[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const LeanEntry<T> e = E[(qb + u) * H + g];
-                        vv[u] = e.v;
-                        if (active) load4(X + ((uint32_t)e.off + c0a), xv[u]);
-                        else xv[u][0] = xv[u][1] = xv[u][2] = xv[u][3] = T(0);
+                    for (int q = 0; q < U; q += 4) {
+                        const uint4 o = *reinterpret_cast<const uint4*>(og + qb + q);
+                        T v4[4];
+                        lean_values4(vg + qb + q, v4);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            vv[q + u] = v4[u];
+                            const uint32_t off = u == 0 ? o.x : u == 1 ? o.y : u == 2 ? o.z : o.w;
+#pragma unroll
+                            for (int j = 0; j < NL; ++j) {
+                                if (active[j]) xv[q + u][j] = gather(off, j);
+                                else xv[q + u][j] = LeanVec<T>{};
+                            }
+                        }
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) c4[j] = fma((CT)vv[u], (CT)xv[u][j], c4[j]);
+                        for (int j = 0; j < NL; ++j)
+#pragma unroll
+                            for (int e = 0; e < VEC; ++e) cs[j][e] = fma((CT)vv[u], (CT)xv[u][j].v[e], cs[j][e]);
                 }
             } else {
-                for (int q = g; q < cnt; q += H) {
-                    const LeanEntry<T> e = E[q];
-                    T x[4] = {T(0), T(0), T(0), T(0)};
-                    if (active) load4(X + ((uint32_t)e.off + c0a), x);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) c4[j] = fma((CT)e.v, (CT)x[j], c4[j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += (double)c4[j];
-        }
-#pragma unroll
-        for (int o = GL; o < 32; o <<= 1)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-        if (g == 0 && active) {
-            if (rr >= 0) store_cols<OT, 4>(Y + (int64_t)rr * ldy + col0, ncols_here, acc);
-            else store_cols<double, 4>(part + sg * (int64_t)l + col0, ncols_here, acc);
-        }
-    }
-}
-
-// The FP32 form, kept apart from the template: its own instruction schedule
-// measured 7 % faster than k_spmm_lean<float> on the 100k x 30k workload.
-template <typename OT, int H>
-__global__ void __launch_bounds__(kF32Warps * 32, 4)
-    k_spmm_f32(const int32_t* __restrict__ ci, const float* __restrict__ val, const int32_t* __restrict__ seg_row,
-               const int64_t* __restrict__ seg_beg, const int64_t* __restrict__ seg_end, int64_t nseg,
-               const float* __restrict__ X, int32_t ldx, int l, OT* __restrict__ Y, int64_t ldy,
-               double* __restrict__ part) {
-    constexpr int GL = 32 / H;        // lanes per group
-    constexpr int PER = 32 / H;       // entries of a chunk per group
-    constexpr int U = 8;              // gathers in flight per lane
-    __shared__ int2 s_ent[kF32Warps][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane / GL, gl = lane % GL;
-    const int col0 = gl * 4;
-    const int ncols_here = (l - col0) < 4 ? (l - col0) : 4;
-    const bool active = ncols_here > 0;
-    // gathers address X + (32-bit offset): the base is the same for every
-    // lane, which saves the 64-bit per-lane address arithmetic (4 % per pass)
-    const uint32_t c0a = active ? (uint32_t)col0 : 0u;
-    int2* E = s_ent[w];
-    const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t sg = gwarp; sg < nseg; sg += nwarps) {
-        const int32_t rr = __ldg(seg_row + sg);
-        const int64_t a = __ldg(seg_beg + sg), b = __ldg(seg_end + sg);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        int32_t myc = 0;
-        float myv = 0.f;
-        if (a + lane < b) { myc = __ldg(ci + a + lane); myv = __ldg(val + a + lane); }
-        for (int64_t k0 = a; k0 < b; k0 += 32) {
-            const int cnt = (b - k0) < 32 ? (int)(b - k0) : 32;
-            __syncwarp();  // the previous chunk's entries have been read
-            E[lane] = make_int2(myc * ldx, __float_as_int(myv));
-            __syncwarp();
-            if (k0 + 32 + lane < b) {  // the next chunk's pairs, while this one is used
-                myc = __ldg(ci + k0 + 32 + lane);
-                myv = __ldg(val + k0 + 32 + lane);
-            }
-            float c4[4] = {0.f, 0.f, 0.f, 0.f};
-            if (cnt == 32) {
+                const int mine = (left - g + H - 1) / H;  // entries of this group
 #pragma unroll 1
-                for (int qb = 0; qb < PER; qb += U) {  // batches of U gathers, one batch live at a time
-                    float4 xv[U];
-                    float vv[U];
+                for (int qb = 0; qb * H < left; qb += 4) {
+                    LeanVec<T> xv[4][NL];
+                    T vv[4];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int2 e = E[(qb + u) * H + g];
-                        vv[u] = __int_as_float(e.y);
-                        xv[u] = active ? *reinterpret_cast<const float4*>(X + ((uint32_t)e.x + c0a))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int u = 0; u < 4; ++u) {
+                        const bool ok = qb + u < mine;
+                        vv[u] = ok ? vg[qb + u] : T(0);
+                        const uint32_t off = og[qb + u];
+#pragma unroll
+                        for (int j = 0; j < NL; ++j) {
+                            if (ok && active[j]) xv[u][j] = gather(off, j);
+                            else xv[u][j] = LeanVec<T>{};
+                        }
                     }
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        c4[0] = fmaf(vv[u], xv[u].x, c4[0]);
-                        c4[1] = fmaf(vv[u], xv[u].y, c4[1]);
-                        c4[2] = fmaf(vv[u], xv[u].z, c4[2]);
-                        c4[3] = fmaf(vv[u], xv[u].w, c4[3]);
-                    }
-                }
-            } else {
-                for (int q = g; q < cnt; q += H) {
-                    const int2 e = E[q];
-                    const float v = __int_as_float(e.y);
-                    const float4 x = active ? *reinterpret_cast<const float4*>(X + ((uint32_t)e.x + c0a))
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
-                    c4[0] = fmaf(v, x.x, c4[0]);
-                    c4[1] = fmaf(v, x.y, c4[1]);
-                    c4[2] = fmaf(v, x.z, c4[2]);
-                    c4[3] = fmaf(v, x.w, c4[3]);
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int j = 0; j < NL; ++j)
+#pragma unroll
+                            for (int e = 0; e < VEC; ++e) cs[j][e] = fma((CT)vv[u], (CT)xv[u][j].v[e], cs[j][e]);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += (double)c4[j];
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += (double)cs[j][e];
         }
 #pragma unroll
         for (int o = GL; o < 32; o <<= 1)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-        if (g == 0 && active) {
-            if (rr >= 0) store_cols<OT, 4>(Y + (int64_t)rr * ldy + col0, ncols_here, acc);
-            else store_cols<double, 4>(part + sg * (int64_t)l + col0, ncols_here, acc);
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += __shfl_xor_sync(0xffffffffu, acc[j][e], o);
+        if (g != 0) continue;
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+            if (!active[j]) continue;
+            const int here = l - (int)col[j];
+            if (rr >= 0) {
+                OT* o = Y + (int64_t)rr * ldy + col[j];
+                if (yvec && here >= VEC) {
+                    struct alignas(sizeof(OT) * VEC > 16 ? 16 : sizeof(OT) * VEC) Row { OT v[VEC]; };
+                    Row t;
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) t.v[e] = (OT)acc[j][e];
+                    *reinterpret_cast<Row*>(o) = t;
+                } else {
+                    store_cols<OT, VEC>(o, here, acc[j]);
+                }
+            } else {
+                store_cols<double, VEC>(part + sg * (int64_t)l + col[j], here, acc[j]);
+            }
         }
     }
 }
@@ -381,26 +383,39 @@ __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_
 }
 
 // ------------------------------------------------------------- the plan --
-__global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_t* __restrict__ cnt) {
+// SpMM segment length of a structure: the power of two at which the resident
+// warps (148 SMs x 24) get at least four segments' worth of entries each, so
+// that one long row does not outlast the rest of the product.  At 2,048
+// throughout, A^T X of a 30,011 x 8,009 matrix (3.1 M nonzeros, columns up to
+// a few thousand entries, l = 40) took 196 us; 85 us at 128.
+static int64_t seg_len_for(int64_t nnz) {
+    int64_t len = nnz < 200000 ? 512 : 128;  // small products: the merge's launch costs more than a long row
+    while (len < kSegNnz && len * 4 * 148 * 24 < nnz) len *= 2;
+    return len;
+}
+__global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, int64_t* __restrict__ cnt) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r <= rows; r += (int64_t)gridDim.x * blockDim.x) {
         if (r == rows) { cnt[r] = 0; continue; }
         const int64_t len = rp[r + 1] - rp[r];
-        cnt[r] = len <= kSegNnz ? 1 : (len + kSegNnz - 1) / kSegNnz;
+        cnt[r] = len <= seg ? 1 : (len + seg - 1) / seg;
     }
 }
 __global__ void k_seg_fill(const int64_t* __restrict__ rp, const int64_t* __restrict__ first, int64_t rows,
-                           int32_t* __restrict__ seg_row, int64_t* __restrict__ seg_beg, int64_t* __restrict__ seg_end,
-                           int32_t* __restrict__ multi_rows, unsigned long long* __restrict__ nmulti) {
+                           int64_t seg, int32_t* __restrict__ seg_row, int64_t* __restrict__ seg_beg,
+                           int64_t* __restrict__ seg_end, int32_t* __restrict__ multi_rows,
+                           int32_t* __restrict__ long_rows, unsigned long long* __restrict__ counts) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t f = first[r], f1 = first[r + 1], e = rp[r + 1];
         const bool multi = f1 - f > 1;
         for (int64_t s = f; s < f1; ++s) {
-            const int64_t a = rp[r] + (s - f) * kSegNnz;
+            const int64_t a = rp[r] + (s - f) * seg;
             seg_row[s] = multi ? -(int32_t)r - 1 : (int32_t)r;
             seg_beg[s] = a;
-            seg_end[s] = (a + kSegNnz < e) ? a + kSegNnz : e;
+            seg_end[s] = (a + seg < e) ? a + seg : e;
         }
-        if (multi) multi_rows[atomicAdd(nmulti, 1ull)] = (int32_t)r;  // order is irrelevant to the sums
+        // the lists' order is irrelevant to the sums
+        if (multi) multi_rows[atomicAdd(counts, 1ull)] = (int32_t)r;
+        if (e - rp[r] > kSegNnz) long_rows[atomicAdd(counts + 1, 1ull)] = (int32_t)r;
     }
 }
 
@@ -424,11 +439,12 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.seg_first.alloc(rows + 1, s);
     if (rows == 0) {
         SVDB_CUDA(cudaMemsetAsync(p.seg_first.p, 0, sizeof(int64_t), s));
-        p.nseg = p.nmulti = 0;
+        p.nseg = p.nmulti = p.nlong = 0;
         return;
     }
     DevBuf<int64_t> cnt(rows + 1, s);
-    k_seg_count<<<nblk(rows + 1, 256, 16), 256, 0, s>>>(m.ptr.p, rows, cnt.p);
+    const int64_t seg = seg_len_for(m.nnz);
+    k_seg_count<<<nblk(rows + 1, 256, 16), 256, 0, s>>>(m.ptr.p, rows, seg, cnt.p);
     SVDB_CHECK_LAUNCH();
     size_t tb = 0;
     SVDB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.p, p.seg_first.p, rows + 1, s));
@@ -442,15 +458,17 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.seg_beg.alloc(std::max<int64_t>(nseg, 1), s);
     p.seg_end.alloc(std::max<int64_t>(nseg, 1), s);
     p.multi_rows.alloc(std::max<int64_t>(rows, 1), s);
-    DevBuf<unsigned long long> nm(1, s);
-    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, sizeof(unsigned long long), s));
-    k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, p.seg_row.p, p.seg_beg.p,
-                                                   p.seg_end.p, p.multi_rows.p, nm.p);
+    p.long_rows.alloc(std::max<int64_t>(m.nnz / kSegNnz, 1), s);
+    DevBuf<unsigned long long> nm(2, s);
+    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, 2 * sizeof(unsigned long long), s));
+    k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, seg, p.seg_row.p, p.seg_beg.p,
+                                                   p.seg_end.p, p.multi_rows.p, p.long_rows.p, nm.p);
     SVDB_CHECK_LAUNCH();
-    unsigned long long hm = 0;
-    SVDB_CUDA(cudaMemcpyAsync(&hm, nm.p, sizeof(hm), cudaMemcpyDeviceToHost, s));
+    unsigned long long hm[2] = {0, 0};
+    SVDB_CUDA(cudaMemcpyAsync(hm, nm.p, sizeof(hm), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
-    p.nmulti = (int64_t)hm;
+    p.nmulti = (int64_t)hm[0];
+    p.nlong = (int64_t)hm[1];
 
     // SpMV bins: a stable partition of the rows by length
     p.bin_rows.alloc(std::max<int64_t>(rows, 1), s);
@@ -497,52 +515,95 @@ static void launch_seg(const DevCompressed& m, const VT* v, const XT* X, int64_t
     SVDB_CHECK_LAUNCH();
 }
 
-// k_spmm_lean applies: values and operand of one type, l <= 64 and a
-// multiple of 4, a 16-byte aligned operand with rows of a 16-byte multiple,
-// 32-bit element offsets (nminor * ldx < 2^31), and SVDB_SPMM=seg not set
-// (that keeps k_spmm_seg, for comparisons)
-template <typename VT, typename XT>
-static bool lean_eligible(const DevCompressed& m, const XT* X, int l, int64_t ldx) {
-    if constexpr (!std::is_same<VT, XT>::value) {
-        return false;
+// SVDB_SPMM=seg keeps k_spmm_seg, for comparisons
+static bool lean_off() {
+    const char* e = getenv("SVDB_SPMM");
+    return e && std::string(e) == "seg";
+}
+
+// k_spmm_lean takes X as it is: rows 16-byte aligned, 32-bit element offsets
+template <typename T>
+static bool lean_aligned(const DevCompressed& m, const T* X, int64_t ldx) {
+    return (ldx * (int64_t)sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(X) % 16) == 0 &&
+           m.nminor * ldx < ((int64_t)1 << 31);
+}
+
+template <typename T, typename OT, int H, int NL, int U, int MINB>
+static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
+                    double* part, cudaStream_t s) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    // 8x the resident blocks: timed against the resident blocks only, 1.10
+    // against 1.20 ms for A X of the 100k x 30k workload
+    const int blocks = nblk(m.plan.nseg * 32, kLeanWarps * 32, MINB * 8);
+    const int yvec = ldy % VEC == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
+    auto go = [&](auto kern) {
+        kern<<<blocks, kLeanWarps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p,
+                                                m.plan.nseg, X, (uint32_t)ldx, l, Y, ldy, yvec, part);
+    };
+    if (m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32)) go(k_spmm_lean<T, OT, H, NL, U, MINB, true>);
+    else go(k_spmm_lean<T, OT, H, NL, U, MINB, false>);
+    SVDB_CHECK_LAUNCH();
+}
+
+// l <= 128 columns of X (ldx apart) into Y (ldy apart).  Lane groups as narrow
+// as the columns allow, so that few lanes idle.
+template <typename T, typename OT>
+static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
+                        double* part, cudaStream_t s) {
+    if (m.plan.nseg <= 0) return;
+    if constexpr (std::is_same<T, float>::value) {
+        if (l <= 16) lean_go<T, OT, 8, 1, 4, 4>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
     } else {
-        const char* e = getenv("SVDB_SPMM");
-        if (e && std::string(e) == "seg") return false;
-        return l >= 1 && l <= 64 && l % 4 == 0 && ldx >= l && (ldx * (int64_t)sizeof(XT)) % 16 == 0 &&
-               (reinterpret_cast<uintptr_t>(X) % 16) == 0 && m.nminor * ldx < ((int64_t)1 << 31);
+        if (l <= 8) lean_go<T, OT, 8, 1, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 16) lean_go<T, OT, 4, 1, 8, 3>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 48) lean_go<T, OT, 4, 3, 4, 2>(m, v, X, l, ldx, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
     }
 }
 
-// FP32: 64 registers and four blocks per SM with eight gathers in flight per
-// lane (1.10 ms for A X of the 100k x 30k workload, against 1.64 ms at two
-// blocks and 1.33-1.36 ms at three); FP64: four gathers in flight, three blocks.
-template <typename T, typename OT>
-static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, OT* Y, double* part,
-                        cudaStream_t s, int64_t ldx = 0) {
-    if (ldx == 0) ldx = l;
-    const int64_t ns = m.plan.nseg;
-    if (ns <= 0) return;
-    constexpr bool f32 = std::is_same<T, float>::value;
-    constexpr int U = f32 ? 8 : 4, MINB = f32 ? 4 : 3;
-    // 8x the resident blocks: timed against the resident blocks only, 1.10
-    // against 1.20 ms for A X of the 100k x 30k workload
-    const int blocks = nblk(ns * 32, kF32Warps * 32, MINB * 8);
-    if constexpr (f32) {
-        if (l <= 32)
-            k_spmm_f32<OT, 4><<<blocks, kF32Warps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p,
-                                                                m.plan.seg_end.p, ns, X, (int32_t)ldx, l, Y, l, part);
-        else
-            k_spmm_f32<OT, 2><<<blocks, kF32Warps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p,
-                                                                m.plan.seg_end.p, ns, X, (int32_t)ldx, l, Y, l, part);
-    } else {
-        if (l <= 32)
-            k_spmm_lean<T, OT, 4, U, MINB><<<blocks, kF32Warps * 32, 0, s>>>(
-                m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p, ns, X, (int32_t)ldx, l, Y, l, part);
-        else
-            k_spmm_lean<T, OT, 2, U, MINB><<<blocks, kF32Warps * 32, 0, s>>>(
-                m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p, ns, X, (int32_t)ldx, l, Y, l, part);
+// out (rows x ldx) = in (rows x l), zero past column l; rows * ldx < 2^31
+template <typename T>
+__global__ void k_pad_rows(const T* __restrict__ in, T* __restrict__ out, uint32_t n, uint32_t l, uint32_t ldx) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t r = i / ldx, c = i - r * ldx;
+        out[i] = c < l ? in[r * l + c] : T(0);
     }
+}
+
+template <typename OT>
+static void merge_rows(const DevCompressed& m, const double* part, int l, OT* Y, int64_t ldy, cudaStream_t s) {
+    if (!m.plan.nmulti) return;
+    k_spmm_merge<OT><<<nblk(m.plan.nmulti * 32, 256, 16), 256, 0, s>>>(m.plan.seg_first.p, m.plan.multi_rows.p,
+                                                                      m.plan.nmulti, part, l, Y, ldy);
     SVDB_CHECK_LAUNCH();
+}
+
+// The operand k_spmm_lean reads: X itself, or a copy in `buf` whose rows are
+// whole 16-byte vectors (odd l, unaligned X).  Null where it does not apply:
+// 2^31 elements or more, or fewer entries than rows of X (the copy would cost
+// more than the gathers); k_spmm_seg takes those as they are.  Rows padded
+// further, to whole 128-byte lines, were no faster (50,000 x 30,000, 28 M
+// nonzeros, l = 60: 805 against 812 us FP64, 865 against 870 FP32 at 100,000
+// rows): the gathers run at 15-17 TB/s of rows, near what L2 delivers.
+template <typename T>
+static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t& ldx, DevBuf<T>& buf,
+                             cudaStream_t s) {
+    if (lean_off()) return nullptr;
+    ldx = l;
+    if (lean_aligned(m, X, ldx)) return X;
+    constexpr int64_t VEC = 16 / (int64_t)sizeof(T);
+    ldx = (l + VEC - 1) / VEC * VEC;
+    if (m.nnz < m.nminor || m.nminor * ldx >= ((int64_t)1 << 31)) return nullptr;
+    buf.alloc(std::max<int64_t>(m.nminor * ldx, 1), s);
+    k_pad_rows<T><<<nblk(m.nminor * ldx, 256, 16), 256, 0, s>>>(X, buf.p, (uint32_t)(m.nminor * ldx), (uint32_t)l,
+                                                               (uint32_t)ldx);
+    SVDB_CHECK_LAUNCH();
+    return buf.p;
 }
 
 template <typename VT, typename XT, typename OT>
@@ -550,12 +611,14 @@ static void spmm_impl(const DevCompressed& m, const VT* v, const XT* X, int l, O
     DevBuf<double> part;
     if (m.plan.nmulti) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
     if constexpr (std::is_same<VT, XT>::value) {
-        if (lean_eligible<VT, XT>(m, X, l, l)) {
-            launch_lean<VT, OT>(m, v, X, l, Y, part.p, s);
-            if (m.plan.nmulti) {
-                k_spmm_merge<OT><<<nblk(m.plan.nmulti * 32, 256, 16), 256, 0, s>>>(
-                    m.plan.seg_first.p, m.plan.multi_rows.p, m.plan.nmulti, part.p, l, Y, l);
-                SVDB_CHECK_LAUNCH();
+        DevBuf<XT> buf;
+        int64_t ldx = 0;
+        const XT* Xa = lean_operand(m, X, l, ldx, buf, s);
+        if (Xa) {
+            for (int c0 = 0; c0 < l; c0 += 128) {
+                const int lc = std::min(128, l - c0);
+                launch_lean<VT, OT>(m, v, Xa + c0, lc, ldx, Y + c0, l, part.p, s);
+                merge_rows(m, part.p, lc, Y + c0, l, s);
             }
             return;
         }
@@ -567,11 +630,7 @@ static void spmm_impl(const DevCompressed& m, const VT* v, const XT* X, int l, O
         if (lc <= 32) launch_seg<VT, XT, OT, 2, 2>(m, v, Xc, l, lc, Yc, l, part.p, s);
         else if (lc <= 64) launch_seg<VT, XT, OT, 4, 2>(m, v, Xc, l, lc, Yc, l, part.p, s);
         else launch_seg<VT, XT, OT, 4, 1>(m, v, Xc, l, lc, Yc, l, part.p, s);
-        if (m.plan.nmulti) {
-            k_spmm_merge<OT><<<nblk(m.plan.nmulti * 32, 256, 16), 256, 0, s>>>(
-                m.plan.seg_first.p, m.plan.multi_rows.p, m.plan.nmulti, part.p, lc, Yc, l);
-            SVDB_CHECK_LAUNCH();
-        }
+        merge_rows(m, part.p, lc, Yc, l, s);
     }
 }
 
@@ -850,12 +909,8 @@ void spmm_f32_strided(const DevCompressed& m, const float* X, int l, int64_t ldx
         throw Error(SVDB_ERR_ARG, "spmm_f32_strided: operand layout not supported");
     DevBuf<double> part;
     if (m.plan.nmulti) part.alloc(m.plan.nseg * (int64_t)l, s);
-    launch_lean<float, double>(m, m.val32.p, X, l, Y, part.p, s, ldx);
-    if (m.plan.nmulti) {
-        k_spmm_merge<double><<<nblk(m.plan.nmulti * 32, 256, 16), 256, 0, s>>>(m.plan.seg_first.p, m.plan.multi_rows.p,
-                                                                              m.plan.nmulti, part.p, l, Y, l);
-        SVDB_CHECK_LAUNCH();
-    }
+    launch_lean<float, double>(m, m.val32.p, X, l, ldx, Y, l, part.p, s);
+    merge_rows(m, part.p, l, Y, l, s);
 }
 
 template <typename XT, typename OT>

@@ -79,15 +79,16 @@ struct DevBuf {
 // a CSC, i.e. rows of the transpose).  Column indices are int32 (minor
 // dimension < 2^31), offsets int64.
 // Load-balancing plan for the row gathers of SpMM: every row is cut into
-// segments of at most kSegNnz entries; seg_first[r] .. seg_first[r+1] are the
+// segments of at most kSegNnz entries (fewer in small structures,
+// seg_len_for); seg_first[r] .. seg_first[r+1] are the
 // segments of row r; segment s covers entries [seg_beg[s], seg_end[s]) of row
 // seg_row[s], stored as -(row + 1) when the row has several segments; those
 // rows are listed in multi_rows and merged by a second, ordered pass.
 constexpr int64_t kSegNnz = 2048;
 // SpMV row bins: bin b (< kSpmvBins) holds the rows of at most
 // kSpmvBinLen[b] entries (and more than kSpmvBinLen[b-1]), ascending, taken
-// by groups of (2 << b) lanes; rows of more than kSegNnz entries are the
-// multi rows, one block each.
+// by groups of (2 << b) lanes; rows of more than kSegNnz entries are
+// long_rows, one block each.
 constexpr int kSpmvBins = 5;
 constexpr int64_t kSpmvBinLen[kSpmvBins] = {8, 16, 32, 64, kSegNnz};
 struct SpmvBins {
@@ -96,13 +97,13 @@ struct SpmvBins {
     int64_t items[kSpmvBins + 1];    // warp items before bin b (32 / (2 << b) rows per item)
 };
 struct SegPlan {
-    int64_t nseg = 0, nmulti = 0;
+    int64_t nseg = 0, nmulti = 0, nlong = 0;
     DevBuf<int32_t> bin_rows;
     SpmvBins bins{};
     DevBuf<int64_t> seg_first;
     DevBuf<int32_t> seg_row;
     DevBuf<int64_t> seg_beg, seg_end;
-    DevBuf<int32_t> multi_rows;
+    DevBuf<int32_t> multi_rows, long_rows;
 };
 
 // Panel plan of the FP32 SpMM (spmm_panel.cu), built on first use.  Rows
