@@ -34,89 +34,150 @@ static int grid_for_work(int64_t work, int threads, int per_sm = 8) {
 
 // ------------------------------------------------------------------ SDDMM ----
 // One warp per segment of the load-balancing plan (at most kSegNnz entries of
-// one row).  Lane t keeps left[r][t + 32 j] (j < SLOTS) in registers.  The
-// segment is taken 32 entries at a time: for entry q every lane forms its
-// partial product with right[c_q] (coalesced row reads), and a butterfly
-// transpose reduction (16 + 8 + 4 + 2 + 1 shuffles for all 32 entries) leaves
-// lane q holding the dot product of entry q, in a fixed order.
-template <typename T, int SLOTS>
-__global__ void __launch_bounds__(256) k_sddmm(const int32_t* __restrict__ idx, const int32_t* __restrict__ seg_row,
-                                               const int64_t* __restrict__ seg_beg,
-                                               const int64_t* __restrict__ seg_end, int64_t nseg,
-                                               const T* __restrict__ left, const T* __restrict__ right, int rank,
-                                               T* __restrict__ out) {
+// one row).  H = 32 / GL groups of GL lanes take every H-th entry of a
+// 32-entry chunk; a lane keeps NL 16-byte vectors of the left row, GL vectors
+// apart, and reads the same columns of the right rows (dense 16-byte loads).
+// A batch of U entries is reduced over the group's lanes by a butterfly
+// transpose (U - 1 shuffles, then log2(GL / U) for the lanes that share an
+// entry), in a fixed order; the batches run one at a time so that only U rows
+// are live (unrolled, the compiler hoisted their loads and spilled).
+// The gathered rows through L1 and L2 bound it.  A lane per column (4-byte
+// loads, a 31-shuffle transpose with two selects each over the whole warp,
+// about 20 warp instructions per entry) took 313 us for 4.3 M entries of
+// rank 64 at FP32.
+template <typename T>
+struct alignas(16) SdVec { T v[16 / sizeof(T)]; };
+
+template <typename T, int GL, int NL, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__ idx, const int32_t* __restrict__ seg_row,
+                                                     const int64_t* __restrict__ seg_beg,
+                                                     const int64_t* __restrict__ seg_end, int64_t nseg,
+                                                     const T* __restrict__ left, const T* __restrict__ right, int rank,
+                                                     T* __restrict__ out) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int H = 32 / GL;
+    static_assert(GL % U == 0, "whole batches");
+    constexpr int SH = GL / U;  // lanes that end up with one entry of a batch; batches of a chunk
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, g = lane / GL, gl = lane % GL;
     const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    bool active[NL];
+    int col[NL];
+#pragma unroll
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * VEC;
+        active[j] = c < rank;
+        col[j] = active[j] ? c : 0;
+    }
     for (int64_t sg = warp0; sg < nseg; sg += nwarps) {
-        int32_t r = seg_row[sg];
+        int32_t r = __ldg(seg_row + sg);
         if (r < 0) r = -r - 1;
-        const int64_t beg = seg_beg[sg], end = seg_end[sg];
-        T lv[SLOTS];
+        const int64_t beg = __ldg(seg_beg + sg);
+        int left_n = (int)(__ldg(seg_end + sg) - beg);
+        const int32_t* ip = idx + beg + lane;
+        int32_t cm = lane < left_n ? __ldg(ip) : 0;
+        SdVec<T> lv[NL];
 #pragma unroll
-        for (int j = 0; j < SLOTS; ++j) {
-            const int t = lane + 32 * j;
-            lv[j] = t < rank ? left[(int64_t)r * rank + t] : T(0);
-        }
-        for (int64_t p0 = beg; p0 < end; p0 += 32) {
-            const int cnt = (int)min((int64_t)32, end - p0);
-            const int cmine = lane < cnt ? idx[p0 + lane] : 0;
-            T p[32];
+        for (int j = 0; j < NL; ++j)
+            lv[j] = active[j] ? *reinterpret_cast<const SdVec<T>*>(left + (int64_t)r * rank + col[j]) : SdVec<T>{};
+        for (T* op = out + beg; left_n > 0; left_n -= 32, op += 32) {
+            const int cnt = left_n < 32 ? left_n : 32;
+            ip += 32;
+            const int32_t cnext = lane + 32 < left_n ? __ldg(ip) : 0;  // the next chunk's columns
+            T res = T(0);
+#pragma unroll 1
+            for (int b = 0; b < SH && b * U * H < cnt; ++b) {
+                SdVec<T> x[U][NL];
 #pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                const int c = __shfl_sync(full, cmine, q);
-                T acc = T(0);
-                if (q < cnt) {
-                    const T* rr = right + (int64_t)c * rank;
+                for (int u = 0; u < U; ++u) {
+                    const int q = (b * U + u) * H + g;
+                    const uint32_t c = (uint32_t)__shfl_sync(full, cm, q);
+                    const T* row = right + (uint64_t)c * (uint32_t)rank;
 #pragma unroll
-                    for (int j = 0; j < SLOTS; ++j) {
-                        const int t = lane + 32 * j;
-                        if (t < rank) acc = fma(lv[j], __ldg(rr + t), acc);
+                    for (int j = 0; j < NL; ++j) {
+                        if (q < cnt && active[j]) x[u][j] = *reinterpret_cast<const SdVec<T>*>(row + col[j]);
+                        else x[u][j] = SdVec<T>{};
                     }
                 }
-                p[q] = acc;
-            }
+                T p[U];
 #pragma unroll
-            for (int w = 16; w >= 1; w >>= 1) {
-                const bool upper = (lane & w) != 0;
+                for (int u = 0; u < U; ++u) {
+                    p[u] = T(0);
 #pragma unroll
-                for (int i = 0; i < w; ++i) {
-                    const T send = upper ? p[i] : p[i + w];
-                    const T keep = upper ? p[i + w] : p[i];
-                    p[i] = keep + __shfl_xor_sync(full, send, w);
+                    for (int j = 0; j < NL; ++j)
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) p[u] = fma(lv[j].v[e], x[u][j].v[e], p[u]);
                 }
+#pragma unroll
+                for (int n = U / 2, w = GL / 2; w >= 1; w >>= 1, n >>= 1) {
+                    if (n >= 1) {  // transpose: the upper lanes take the later entries
+                        const bool upper = (gl & w) != 0;
+#pragma unroll
+                        for (int i = 0; i < n; ++i) {
+                            const T send = upper ? p[i] : p[i + n];
+                            const T keep = upper ? p[i + n] : p[i];
+                            p[i] = keep + __shfl_xor_sync(full, send, w);
+                        }
+                    } else {
+                        p[0] += __shfl_xor_sync(full, p[0], w);
+                    }
+                }
+                if (gl % SH == b) res = p[0];
             }
-            if (lane < cnt) out[p0 + lane] = p[0];
+            const int mine = ((gl % SH) * U + gl / SH) * H + g;
+            if (mine < cnt) op[mine] = res;
+            cm = cnext;
         }
+    }
+}
+
+// out (rows x ldo) = in (rows x rank), zero past column rank
+template <typename T>
+__global__ void k_sddmm_pad(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int rank, int ldo) {
+    const int64_t n = rows * ldo;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / ldo;
+        const int c = (int)(i - r * ldo);
+        out[i] = c < rank ? in[r * rank + c] : T(0);
     }
 }
 
 template <typename T>
 static void sddmm_launch(const DevCompressed& m, const T* left, const T* right, int rank, T* out, cudaStream_t s) {
     if (m.nnz == 0) return;
+    if (rank > 256) throw Error(SVDB_ERR_UNSUPPORTED, "sddmm: rank above 256");
+    // factors whose rows are not whole 16-byte vectors are copied to rows that are
+    constexpr int VEC = 16 / (int)sizeof(T);
+    DevBuf<T> lbuf, rbuf;
+    const int ld = (rank + VEC - 1) / VEC * VEC;
+    auto whole = [&](const T* x, int64_t rows, DevBuf<T>& buf) -> const T* {
+        if (ld == rank && reinterpret_cast<uintptr_t>(x) % 16 == 0) return x;
+        buf.alloc(rows * ld, s);
+        k_sddmm_pad<T><<<grid_for_work(rows * ld, 256, 16), 256, 0, s>>>(x, buf.p, rows, rank, ld);
+        SVDB_CHECK_LAUNCH();
+        return buf.p;
+    };
+    left = whole(left, m.nmajor, lbuf);
+    right = whole(right, m.nminor, rbuf);
     const SegPlan& pl = m.plan;
-    const int blocks = grid_for_work(pl.nseg * 32, 256, 8);
-    const int slots = (rank + 31) / 32;
-#define SVDB_SDDMM_CASE(S)                                                                                  \
-    case S:                                                                                                 \
-        k_sddmm<T, S><<<blocks, 256, 0, s>>>(m.idx.p, pl.seg_row.p, pl.seg_beg.p, pl.seg_end.p, pl.nseg, left, \
-                                             right, rank, out);                                             \
-        break;
-    switch (slots) {
-        SVDB_SDDMM_CASE(1)
-        SVDB_SDDMM_CASE(2)
-        SVDB_SDDMM_CASE(3)
-        SVDB_SDDMM_CASE(4)
-        SVDB_SDDMM_CASE(6)
-        SVDB_SDDMM_CASE(8)
-        case 5: k_sddmm<T, 6><<<blocks, 256, 0, s>>>(m.idx.p, pl.seg_row.p, pl.seg_beg.p, pl.seg_end.p, pl.nseg,
-                                                     left, right, rank, out); break;
-        case 7: k_sddmm<T, 8><<<blocks, 256, 0, s>>>(m.idx.p, pl.seg_row.p, pl.seg_beg.p, pl.seg_end.p, pl.nseg,
-                                                     left, right, rank, out); break;
-        default: throw Error(SVDB_ERR_UNSUPPORTED, "sddmm: rank above 256");
-    }
-#undef SVDB_SDDMM_CASE
+    const int blocks = grid_for_work(pl.nseg * 32, 256, 24);
+    auto go = [&](auto kern) {
+        kern<<<blocks, 256, 0, s>>>(m.idx.p, pl.seg_row.p, pl.seg_beg.p, pl.seg_end.p, pl.nseg, left, right, ld, out);
+    };
+    // At least 64 contiguous bytes per load, two vectors per lane before the
+    // group widens, and as many warps as the registers allow: warps count more
+    // than entries in flight per warp (5.4 M entries, rank 64, FP32: 126 us with
+    // two entries and six CTAs per SM, 144-174 with eight and two or three;
+    // FP64: 240 us with four entries and four CTAs, 291 with (8, 4, 2) and three).
+    const int nv = ld / VEC;  // vectors per row
+    if (nv <= 4) go(k_sddmm<T, 4, 1, 4, 4>);
+    else if (nv <= 8) go(k_sddmm<T, 8, 1, 8, 4>);
+    else if (nv <= 16) go(k_sddmm<T, 8, 2, 2, 6>);
+    else if (nv <= 24) go(k_sddmm<T, 8, 3, 2, 4>);
+    else if (nv <= 32) go(k_sddmm<T, 16, 2, 4, 4>);
+    else if (nv <= 64) go(k_sddmm<T, 32, 2, 4, 4>);
+    else go(k_sddmm<T, 32, 4, 2, 3>);
     SVDB_CHECK_LAUNCH();
 }
 
