@@ -495,7 +495,7 @@ __global__ void k_b_gram_reduce(const double* __restrict__ part, int nchunk, int
     }
 }
 
-__global__ void k_b_chol_inv(const double* __restrict__ G, int c, SubLayout L, const int64_t* __restrict__ coff,
+__global__ void __launch_bounds__(256) k_b_chol_inv(const double* __restrict__ G, int c, SubLayout L, const int64_t* __restrict__ coff,
                              double* __restrict__ R, double* __restrict__ Ri, int* __restrict__ flags,
                              int* __restrict__ shifted, const int* __restrict__ cond) {
     const int64_t b = blockIdx.x;
@@ -504,7 +504,7 @@ __global__ void k_b_chol_inv(const double* __restrict__ G, int c, SubLayout L, c
     const int64_t rows = sub_rows(L, coff, b);
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
     const int64_t cc = (int64_t)c * c;
-    chol_inv_body(G + b * cc, c, shift_scale, R + b * cc, Ri + b * cc, flags + b, shifted + b, 1, sm);
+    chol_inv_body(G + b * cc, 0, c, shift_scale, R + b * cc, Ri + b * cc, flags + b, shifted + b, sm);
 }
 
 // Out_b (rows x cout) = X_b (rows x c) S_b (c x lds, first cout columns),
@@ -784,8 +784,8 @@ static void right_mul(svdb_batch& B, const TI* X, SubLayout L, const double* S, 
 
 static void chol(svdb_batch& B, SubLayout L, double* R, const int* cond) {
     const int c = (int)B.l;
-    const size_t smem = 2 * (size_t)c * c * sizeof(double);
-    // chol_inv_body also holds about 1 KB of static shared memory
+    const size_t smem = chol_smem(c);
+    // chol_inv_body also holds some static shared memory
     if (smem > 40 * 1024)
         SVDB_CUDA(cudaFuncSetAttribute(k_b_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_b_chol_inv<<<(unsigned)B.count, 256, smem, B.s>>>(B.G.p, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,

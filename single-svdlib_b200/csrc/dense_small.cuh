@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "dense_tall.cuh"
 #include "device_common.cuh"
 
 namespace svdb {
@@ -29,129 +30,152 @@ __device__ __forceinline__ double omega_value(uint64_t key, int64_t i) {
     return sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
 }
 
-// One block: G = R^T R (upper R) in shared memory, then R^-1.  A non-positive
-// pivot restarts the factorisation on G + shift I with shift =
-// shift_scale * trace(G) (shifted CholeskyQR); that sets bit 1 of *flags and
-// *shifted (which enables the third pass).  A second breakdown sets bit 2 and
-// leaves R = R^-1 = I.  R and R^-1 are written to global memory.
-// The factorisation runs on the first 128 threads with one named barrier per
-// step: step k updates a_ij -= a_ki a_kj / a_kk with the unscaled pivot row,
-// and every row is scaled by 1/sqrt(a_kk) at the end.
-// sm: c*c doubles of shared memory (2*c*c when ri_in_smem); c <= 128; at
-// least 128 threads.
-__device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int c, double shift_scale,
+// One block: G = R^T R (upper R), and R^-1, in one sweep over panels of eight
+// rows.  The forward elimination of [G | I] leaves [R | R^-T], so R^-1 has no
+// dependent chain of its own.  Per panel K:
+//   - every warp that owns columns factors the 8 x 8 diagonal block in
+//     registers (redundantly: no broadcast, no barrier) and eliminates one
+//     column per thread;
+//   - the trailing tiles are updated with the FP64 matrix instruction.
+// What bounds it is the chain of c pivots (a reciprocal square root and two
+// multiply-adds each, about 90 cycles) and two barriers per eight of them.  The
+// form before it (a barrier and a division per pivot, then a forward
+// substitution per row of R^-1) took 70 us at c = 60, 36 at 40 and 15 at 20;
+// this one 22, 13 and 11 (ncu, cold caches).
+//
+// Layout: rows of 8 x 8 tiles, row tile I: tiles 0 .. I hold R^-T (I, 0 .. I)
+// (the identity before panel I), tiles I + 1 .. nt hold G / R (I, I .. nt - 1);
+// padded to whole tiles with the identity.  The factored diagonal tiles go to
+// their own buffer, since other warps may still be reading the unfactored one.
+//
+// A pivot that is not positive and finite restarts the factorisation on
+// G + shift I with shift = shift_scale * trace(G) (shifted CholeskyQR); that
+// sets bit 1 of *flags and *shifted (which enables the third pass).  A second
+// breakdown sets bit 2 and leaves R = R^-1 = I.
+// G: c x c, or with nparts > 0 the sum of nparts such matrices, in order (only
+// the tiles on and above the diagonal are read).  c <= 128; blockDim.x a
+// multiple of 32, at least 160.  sm: chol_smem(c) bytes.
+__host__ __device__ inline int chol_ld(int c) { return ((c + 7) / 8 + 1) * 8 + 4; }  // = 4 or 12 mod 16: no conflicts
+__host__ __device__ inline size_t chol_smem(int c) {
+    const int nt = (c + 7) / 8;
+    return ((size_t)nt * 8 * chol_ld(c) + (size_t)nt * 64) * sizeof(double);
+}
+__device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int nparts, int c, double shift_scale,
                                               double* __restrict__ R, double* __restrict__ Ri,
-                                              int* __restrict__ flags, int* __restrict__ shifted, int ri_in_smem,
-                                              double* sm) {
+                                              int* __restrict__ flags, int* __restrict__ shifted, double* sm) {
     __shared__ int s_fail;
-    __shared__ double s_shift;
-    __shared__ double s_rd[128];  // 1 / sqrt(a_kk)
-    const int cc = c * c;
-    double* ri = ri_in_smem ? sm + cc : Ri;
-    if (blockDim.x < 128 || c > 128) {  // the named barrier needs 128 threads; s_rd holds 128 pivots
+    __shared__ double s_red[32];
+    const int nt = (c + 7) / 8, c8 = nt * 8, ld = chol_ld(c), cc = c * c;
+    double* const dg = sm + (size_t)c8 * ld;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (blockDim.x < 160 || c > 128) {  // one thread per column of the widest row
         if (threadIdx.x == 0) atomicOr(flags, 2);
         for (int t = threadIdx.x; t < cc; t += blockDim.x) R[t] = Ri[t] = (t / c == t % c) ? 1.0 : 0.0;
         return;
     }
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        for (int t = threadIdx.x; t < cc; t += blockDim.x)
-            sm[t] = G[t] + ((attempt == 1 && t / c == t % c) ? s_shift : 0.0);
-        if (threadIdx.x == 0) s_fail = 0;
-        __syncthreads();
-        if (threadIdx.x < 128) {
-            for (int k = 0; k < c; ++k) {
-                const double d = sm[k * c + k];
-                if (!(d > 0.0 && isfinite(d))) {  // the same value for all 128 threads
-                    if (threadIdx.x == 0) s_fail = 1;
-                    break;
-                }
-                const double inv = 1.0 / d;
-                // upper triangle i <= j of the trailing block: 8 rows x 16 columns of
-                // threads, no index division
-                const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-                for (int i = k + 1 + ty; i < c; i += 8) {
-                    const double aki = sm[k * c + i];
-                    for (int j = i + tx; j < c; j += 16) sm[i * c + j] -= aki * sm[k * c + j] * inv;
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+    auto g_at = [&](int i, int j) {
+        if (nparts <= 0) return G[i * c + j];
+        double v = 0.0;
+#pragma unroll 8
+        for (int b = 0; b < nparts; ++b) v += G[(int64_t)b * cc + i * c + j];
+        return v;
+    };
+    double shift = 0.0;
+    for (int attempt = 0;; ++attempt) {
+        for (int i = warp; i < c8; i += nw) {
+            const int i8 = i & ~7;
+            for (int j = lane; j < i8; j += 32) sm[i * ld + j] = 0.0;
+            for (int j = i8 + lane; j < c8; j += 32) {
+                double v = i == j ? 1.0 : 0.0;
+                if (i < c && j < c) v = g_at(i, j) + (i == j ? shift : 0.0);
+                sm[i * ld + 8 + j] = v;
             }
         }
+        if (threadIdx.x == 0) s_fail = 0;
         __syncthreads();
-        if (!s_fail) break;
-        if (attempt == 0) {
-            if (threadIdx.x == 0) {
-                double tr = 0.0;
-                for (int i = 0; i < c; ++i) tr += G[i * c + i];
-                s_shift = shift_scale * tr > 0.0 ? shift_scale * tr : 1e-300;
-                atomicOr(flags, 1);
-                *shifted = 1;
+        bool failed = false;
+        for (int K = 0; K < nt; ++K) {
+            if (warp * 32 < c8 + 8) {
+                double d[8][8], r[8];
+                const double* blk = sm + 8 * K * ld + 8 * (K + 1);
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+#pragma unroll
+                    for (int i = k; i < 8; ++i) d[k][i] = blk[k * ld + i];
+                bool ok = true;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    ok = ok && d[k][k] > 0.0 && isfinite(d[k][k]);
+                    r[k] = rsqrt(d[k][k]);
+#pragma unroll
+                    for (int i = k; i < 8; ++i) d[k][i] *= r[k];
+#pragma unroll
+                    for (int i = k + 1; i < 8; ++i)
+#pragma unroll
+                        for (int j = i; j < 8; ++j) d[i][j] = fma(-d[k][i], d[k][j], d[i][j]);
+                }
+                if (!ok && lane == 0) s_fail = 1;
+                const int j = threadIdx.x, tile = j >> 3;
+                if (j < c8 + 8) {
+                    double a[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        a[k] = tile == K ? ((j & 7) == k ? 1.0 : 0.0) : sm[(8 * K + k) * ld + j];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        a[k] *= r[k];
+#pragma unroll
+                        for (int i = k + 1; i < 8; ++i) a[i] = fma(-d[k][i], a[k], a[i]);
+                    }
+                    if (tile == K + 1) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) dg[(8 * K + k) * 8 + (j & 7)] = (j & 7) < k ? 0.0 : a[k];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) sm[(8 * K + k) * ld + j] = a[k];
+                    }
+                }
             }
             __syncthreads();
+            if (s_fail) {  // the same value for every thread
+                failed = true;
+                break;
+            }
+            // row tiles I > K: tiles 0 .. K of R^-T and I .. nt - 1 of G
+            const int kl = lane & 3, il = lane >> 2;
+            const double* pk = sm + (8 * K + kl) * ld + il;
+            for (int q = warp; q < (nt - 1 - K) * (nt + 1); q += nw) {
+                const int I = K + 1 + q / (nt + 1), t = q % (nt + 1);
+                if (t > K && t <= I) continue;
+                double* cp = sm + (8 * I + il) * ld + 8 * t + 2 * kl;
+                double acc[2] = {cp[0], cp[1]};
+                dmma(acc, -pk[8 * (I + 1)], pk[8 * t]);
+                dmma(acc, -pk[4 * ld + 8 * (I + 1)], pk[4 * ld + 8 * t]);
+                cp[0] = acc[0];
+                cp[1] = acc[1];
+            }
+            __syncthreads();
+        }
+        if (!failed || attempt == 1) break;
+        double tr = 0.0;
+        for (int i = threadIdx.x; i < c; i += blockDim.x) tr += g_at(i, i);
+        shift = shift_scale * block_sum(tr, s_red);  // also orders this attempt's reads before the next one's writes
+        if (!(shift > 0.0)) shift = 1e-300;
+        if (threadIdx.x == 0) {
+            atomicOr(flags, 1);
+            *shifted = 1;
         }
     }
     if (s_fail) {
         if (threadIdx.x == 0) atomicOr(flags, 2);
-        for (int t = threadIdx.x; t < cc; t += blockDim.x) {
-            const double v = (t / c == t % c) ? 1.0 : 0.0;
-            R[t] = v;
-            Ri[t] = v;
-        }
+        for (int t = threadIdx.x; t < cc; t += blockDim.x) R[t] = Ri[t] = (t / c == t % c) ? 1.0 : 0.0;
         return;
     }
-    for (int k = threadIdx.x; k < c; k += blockDim.x) s_rd[k] = 1.0 / sqrt(sm[k * c + k]);
-    __syncthreads();
-    for (int t = threadIdx.x; t < cc; t += blockDim.x) {
-        const int i = t / c, j = t % c;
-        double v = 0.0;
-        if (i == j) v = sqrt(sm[t]);
-        else if (i < j) v = sm[t] * s_rd[i];
-        ri[t] = v;  // staged: sm still holds the pivots other threads read
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < cc; t += blockDim.x) {
-        sm[t] = ri[t];
-        R[t] = ri[t];
-        ri[t] = 0.0;
-    }
-    __syncthreads();
-    // R^-1 row i, one warp per row: x^T R = e_i^T by forward substitution in
-    // axpy form.  Lane l holds x_l, x_{l+32}, x_{l+64}, x_{l+96}; step k scales
-    // x_k by 1 / R_kk and subtracts x_k R[k, k+1..] from the later entries,
-    // reading row k of R (contiguous, no bank conflicts).  No reductions: the
-    // dependent path of a step is one shuffle, one multiply and one FMA.
-    for (int k = threadIdx.x; k < c; k += blockDim.x) s_rd[k] = 1.0 / sm[k * c + k];
-    __syncthreads();
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        for (int i = warp; i < c; i += nwarps) {
-            double x[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) x[q] = (lane + 32 * q == i) ? 1.0 : 0.0;
-            for (int k = i; k < c; ++k) {
-                const int ks = k >> 5, kl = k & 31;
-                double own = x[0];
-#pragma unroll
-                for (int q = 1; q < 4; ++q)
-                    if (ks == q) own = x[q];
-                const double xk = __shfl_sync(0xffffffffu, own, kl) * s_rd[k];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int e = lane + 32 * q;
-                    if (e == k) x[q] = xk;
-                    else if (e > k && e < c) x[q] = fma(-xk, sm[k * c + e], x[q]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = lane + 32 * q;
-                if (e < c) ri[i * c + e] = e >= i ? x[q] : 0.0;
-            }
+    for (int i = warp; i < c; i += nw)
+        for (int j = lane; j < c; j += 32) {
+            R[i * c + j] = (j >> 3) == (i >> 3) ? dg[i * 8 + (j & 7)] : j > i ? sm[i * ld + 8 + j] : 0.0;
+            Ri[i * c + j] = j >= i ? sm[j * ld + i] : 0.0;
         }
-    }
-    if (ri_in_smem) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < cc; t += blockDim.x) Ri[t] = ri[t];
-    }
 }
 
 // Lanes per column pair in jacobi_svd_body (about eight elements of a column

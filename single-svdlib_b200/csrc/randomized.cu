@@ -28,11 +28,6 @@
 
 namespace svdb {
 
-static bool getenv_is(const char* name, const char* value) {
-    const char* e = getenv(name);
-    return e && std::strcmp(e, value) == 0;
-}
-
 static int nb(int64_t work, int threads, int per_sm = 16) {
     int64_t b = (work + threads - 1) / threads;
     return (int)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)device_props().sms * per_sm));
@@ -46,175 +41,28 @@ __global__ void k_omega(uint64_t seed, int64_t total, T* __restrict__ out) {
         out[i] = (T)omega_value(key, i);
 }
 
-// ---------------------------------------------------------------- Gram ----
-// G (c x c) = X^T X for X (rows x c) row-major.  Blocks take row chunks
-// (staged through shared memory); a 16 x 16 thread grid holds an NC x NC
-// register tile of G per thread (entries (ty + 16 i, tx + 16 j)).  G[a][b]
-// and G[b][a] see the same products in the same order, so G is exactly
-// symmetric.  Block partials are reduced in block order.  Every kernel of a
-// CholeskyQR pass takes `cond`: when it points to 0 the kernel returns at
-// once (the conditional third pass of shifted CholeskyQR).
-constexpr int kGramRows = 32;
-template <typename T, int NC>
-__global__ void __launch_bounds__(256) k_gram_part(const T* __restrict__ X, int64_t rows, int c, int64_t chunk,
-                                                   double* __restrict__ part, const int* __restrict__ cond) {
-    if (cond && *cond == 0) return;
-    extern __shared__ double xs[];  // kGramRows x c
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int64_t r0 = blockIdx.x * chunk, r1 = std::min<int64_t>(rows, r0 + chunk);
-    double acc[NC][NC];
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[i][j] = 0.0;
-    for (int64_t rb = r0; rb < r1; rb += kGramRows) {
-        const int nr = (int)std::min<int64_t>(kGramRows, r1 - rb);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * c; t += blockDim.x) xs[t] = (double)X[(rb + t / c) * c + t % c];
-        __syncthreads();
-        for (int r = 0; r < nr; ++r) {
-            double xa[NC], xb[NC];
-#pragma unroll
-            for (int i = 0; i < NC; ++i) {
-                const int a = ty + 16 * i, b = tx + 16 * i;
-                xa[i] = a < c ? xs[r * c + a] : 0.0;
-                xb[i] = b < c ? xs[r * c + b] : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < NC; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j) acc[i][j] = fma(xa[i], xb[j], acc[i][j]);
-        }
-    }
-    double* out = part + (int64_t)blockIdx.x * c * c;
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            const int a = ty + 16 * i, b = tx + 16 * j;
-            if (a < c && b < c) out[a * c + b] = acc[i][j];
-        }
-}
-// G[p] = sum over blocks of part[b][p].  A block covers 32 elements; its 8
-// warps sum fixed slices of the blocks, and the slices are added in slice
-// order, so G[a][b] and G[b][a] still see the same operations (G symmetric).
-constexpr int kRedSlices = 8;
-__global__ void __launch_bounds__(256) k_gram_reduce(const double* __restrict__ part, int nblocks, int c,
-                                                     double* __restrict__ G, const int* __restrict__ cond) {
-    if (cond && *cond == 0) return;
-    __shared__ double sh[kRedSlices][32];
-    const int cc = c * c;
-    const int e = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int sl = threadIdx.x >> 5;
-    double acc = 0.0;
-    if (e < cc) {
-        const int per = (nblocks + kRedSlices - 1) / kRedSlices;
-        const int b0 = sl * per, b1 = min(nblocks, b0 + per);
-        for (int bq = b0; bq < b1; ++bq) acc += part[(int64_t)bq * cc + e];
-    }
-    sh[sl][threadIdx.x & 31] = acc;
-    __syncthreads();
-    if (sl == 0 && e < cc) {
-        double t = 0.0;
-#pragma unroll
-        for (int k = 0; k < kRedSlices; ++k) t += sh[k][threadIdx.x];
-        G[e] = t;
-    }
-}
-
 // ------------------------------------------------------ small dense ops ----
-__global__ void __launch_bounds__(1024) k_chol_inv(const double* __restrict__ G, int c, double shift_scale,
-                                                   double* __restrict__ R, double* __restrict__ Ri,
-                                                   int* __restrict__ flags, int* __restrict__ shifted,
-                                                   const int* __restrict__ cond, int ri_in_smem) {
+// Every kernel of a CholeskyQR pass takes `cond`: when it points to 0 the
+// kernel returns at once (the conditional third pass of shifted CholeskyQR).
+__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int nparts, int c, double shift_scale,
+                                                  double* __restrict__ R, double* __restrict__ Ri,
+                                                  int* __restrict__ flags, int* __restrict__ shifted,
+                                                  const int* __restrict__ cond) {
     if (cond && *cond == 0) return;
-    extern __shared__ double sm[];  // R work (c*c) | R^-1 (c*c) when ri_in_smem
-    chol_inv_body(G, c, shift_scale, R, Ri, flags, shifted, ri_in_smem, sm);
+    extern __shared__ double sm[];
+    chol_inv_body(G, nparts, c, shift_scale, R, Ri, flags, shifted, sm);
 }
 
-// C (c x c) = A (c x c) B (c x c), one block
+// C (c x c) = A (c x c) B (c x c), one thread per element
 __global__ void k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int c,
                              double* __restrict__ C, const int* __restrict__ cond) {
     if (cond && *cond == 0) return;
-    for (int t = threadIdx.x; t < c * c; t += blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < c * c; t += gridDim.x * blockDim.x) {
         const int i = t / c, j = t % c;
         double s = 0.0;
         for (int k = 0; k < c; ++k) s = fma(A[i * c + k], B[k * c + j], s);
         C[t] = s;
     }
-}
-
-// Out (rows x cout) = X (rows x c) S (c x lds, first cout columns).  S and
-// 64-row tiles of X are staged in shared memory; a 16 x 16 thread grid gives
-// every thread a 4 x NJ register tile (rows ty + 16 i, columns tx + 16 j).
-// With nbuf = 2 the next tile of X is copied (cp.async) while the current one
-// is multiplied; nbuf = 1 when two tiles do not fit.
-constexpr int kRmRows = 64;
-__device__ __forceinline__ void rm_cp_async(void* dst, const void* src, int bytes) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-template <typename TI, typename TO, int NJ>
-__global__ void __launch_bounds__(256) k_right_mul(const TI* __restrict__ X, int64_t rows, int c,
-                                                   const double* __restrict__ S, int lds, int cout,
-                                                   TO* __restrict__ Out, const int* __restrict__ cond, int nbuf) {
-    if (cond && *cond == 0) return;
-    extern __shared__ double sm[];  // S: c*cout doubles | nbuf X tiles of kRmRows*c TI
-    double* ss = sm;
-    TI* xbuf = reinterpret_cast<TI*>(sm + c * cout);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int t = threadIdx.x; t < c * cout; t += blockDim.x) ss[t] = S[(t / cout) * lds + t % cout];
-    auto load = [&](int64_t r0, int b) {  // tile at row r0 into buffer b (asynchronous)
-        const int nr = (int)std::min<int64_t>(kRmRows, rows - r0);
-        TI* xs = xbuf + (size_t)b * kRmRows * c;
-        for (int t = threadIdx.x; t < nr * c; t += blockDim.x) rm_cp_async(xs + t, X + r0 * c + t, (int)sizeof(TI));
-    };
-    const int64_t step = (int64_t)gridDim.x * kRmRows;
-    int64_t r0 = (int64_t)blockIdx.x * kRmRows;
-    if (r0 < rows) load(r0, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int it = 0; r0 < rows; r0 += step, ++it) {
-        const int b = nbuf == 2 ? (it & 1) : 0;
-        if (nbuf == 2 && r0 + step < rows) load(r0 + step, b ^ 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");  // possibly empty: one group per iteration
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // this tile's group has landed
-        __syncthreads();
-        const TI* xs = xbuf + (size_t)b * kRmRows * c;
-        const int nr = (int)std::min<int64_t>(kRmRows, rows - r0);
-        double acc[4][NJ];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) acc[i][j] = 0.0;
-        for (int k = 0; k < c; ++k) {
-            double xv[4], sv[NJ];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) xv[i] = (ty + 16 * i < nr) ? (double)xs[(ty + 16 * i) * c + k] : 0.0;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) sv[j] = (tx + 16 * j < cout) ? ss[k * cout + tx + 16 * j] : 0.0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) acc[i][j] = fma(xv[i], sv[j], acc[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int rr = ty + 16 * i;
-            if (rr >= nr) continue;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const int col = tx + 16 * j;
-                if (col < cout) Out[(r0 + rr) * cout + col] = (TO)acc[i][j];
-            }
-        }
-        __syncthreads();  // this buffer is read; it may be refilled
-        if (nbuf == 1 && r0 + step < rows) {
-            load(r0 + step, 0);
-            asm volatile("cp.async.commit_group;" ::: "memory");  // older than the next iteration's group
-        }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 __global__ void k_copy_cond(const double* __restrict__ src, double* __restrict__ dst, int64_t n,
@@ -364,8 +212,6 @@ void center_product(const double* X, int64_t xrows, int c, const double* mu, dou
 // ------------------------------------------------------ host helpers ----
 struct RandCtx {
     cudaStream_t s;
-    bool tensor_gram = false;  // first CholeskyQR pass on the tensor cores (SVDB_MIXED)
-    int cmax = 0;
     DevBuf<double> part, G, R1, R2, R3, Ri, Rtmp, T;
     DevBuf<int> flags, shifted;
     int64_t part_cap = 0;
@@ -373,78 +219,51 @@ struct RandCtx {
 
 // G = X^T X on the tensor cores (3xTF32, FP32 accumulation; gram_tc.cu), the
 // CTA partials summed in FP64 in block order
-static void gram_tensor(RandCtx& cx, const double* X, int64_t rows, int c, double* G, const int* cond) {
+static void gram_tensor(RandCtx& cx, const double* X, int64_t rows, int c, double* G) {
     const int nblk = gram_tc_blocks(rows);
     if ((int64_t)nblk * c * c > cx.part_cap) {
         cx.part_cap = (int64_t)nblk * c * c;
         cx.part.alloc(cx.part_cap, cx.s);
     }
-    gram_tc_launch(X, rows, c, cx.part.p, cx.part_cap, cond, cx.s);
-    k_gram_reduce<<<(c * c + 31) / 32, 32 * kRedSlices, 0, cx.s>>>(cx.part.p, nblk, c, G, cond);
+    gram_tc_launch(X, rows, c, cx.part.p, cx.part_cap, nullptr, cx.s);
+    k_tn_reduce<<<(c * c + 31) / 32, 32 * kTnSlices, 0, cx.s>>>(cx.part.p, nblk, c, c, c, 0, G, nullptr);
     SVDB_CHECK_LAUNCH();
 }
 
-static void gram(RandCtx& cx, const double* X, int64_t rows, int c, double* G, const int* cond) {
+// X^T X on the FP64 matrix instruction.  Returns G, or (parts > 0) the
+// partials that chol_inv adds itself: below kCholParts elements in all the
+// one-block factorisation reads them faster than another launch.
+constexpr int64_t kCholParts = 16384;
+static const double* gram(RandCtx& cx, const double* X, int64_t rows, int c, double* G, const int* cond, int& parts) {
     if (c > 128) throw Error(SVDB_ERR_UNSUPPORTED, "randomized_svd: more than 128 sample columns");
-    const int sms = device_props().sms;
-    int64_t chunk = std::max<int64_t>(kGramRows * 4, (rows + sms * 2 - 1) / (sms * 2));
-    int nblk = (int)std::max<int64_t>(1, (rows + chunk - 1) / chunk);
-    if ((int64_t)nblk * c * c > cx.part_cap) {
-        cx.part_cap = (int64_t)nblk * c * c;
+    const TnShape h = tn_shape(rows, c, c, true, device_props().sms);
+    const int64_t n = (int64_t)h.blocks * c * c;
+    if (n > cx.part_cap) {
+        cx.part_cap = n;
         cx.part.alloc(cx.part_cap, cx.s);
     }
-    const size_t smem = kGramRows * c * sizeof(double);
-    const int nc = (c + 15) / 16;
-    switch (nc) {
-        case 1: k_gram_part<double, 1><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 2: k_gram_part<double, 2><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 3: k_gram_part<double, 3><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 4: k_gram_part<double, 4><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 5: k_gram_part<double, 5><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 6: k_gram_part<double, 6><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        case 7: k_gram_part<double, 7><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-        default: k_gram_part<double, 8><<<nblk, 256, smem, cx.s>>>(X, rows, c, chunk, cx.part.p, cond); break;
-    }
-    k_gram_reduce<<<(c * c + 31) / 32, 32 * kRedSlices, 0, cx.s>>>(cx.part.p, nblk, c, G, cond);
-    SVDB_CHECK_LAUNCH_N(2);
+    parts = n <= kCholParts ? h.blocks : 0;
+    tn_launch(h, X, c, c, X, c, c, rows, cx.part.p, parts ? nullptr : G, cond, cx.s);
+    return parts ? cx.part.p : G;
 }
 
+// Out (rows x cout, or cout x rows when trans) = X (rows x c) S (c x lds,
+// first cout columns); upper: S is upper triangular
 static void right_mul(const double* X, int64_t rows, int c, const double* S, int lds, int cout, double* Out,
-                      cudaStream_t s, const int* cond = nullptr) {
-    const size_t s_bytes = (size_t)c * cout * sizeof(double), tile = (size_t)kRmRows * c * sizeof(double);
-    if (s_bytes + tile > 220 * 1024 || cout > 128)
-        throw Error(SVDB_ERR_UNSUPPORTED, "dense factor wider than the shared-memory tile");
-    // one X tile buffer: at c = 60 that is 59 KB of shared memory and three
-    // blocks per SM instead of two with a second buffer, 908 against 956 us
-    // of k_right_mul per randomized solve (100k x 30k)
-    const int nbuf = 1;
-    const size_t smem = s_bytes + nbuf * tile;
-    const int64_t tiles = (rows + kRmRows - 1) / kRmRows;
-    auto go = [&](auto kern) {
-        if (smem > 48 * 1024)
-            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per_sm = 0;  // one wave of resident blocks, each looping over tiles
-        SVDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
-        const int blocks = (int)std::max<int64_t>(
-            1, std::min<int64_t>(tiles, (int64_t)device_props().sms * std::max(per_sm, 1)));
-        kern<<<blocks, 256, smem, s>>>(X, rows, c, S, lds, cout, Out, cond, nbuf);
-    };
-    if (cout <= 16) go(k_right_mul<double, double, 1>);
-    else if (cout <= 32) go(k_right_mul<double, double, 2>);
-    else if (cout <= 64) go(k_right_mul<double, double, 4>);
-    else go(k_right_mul<double, double, 8>);
-    SVDB_CHECK_LAUNCH();
+                      cudaStream_t s, const int* cond = nullptr, bool upper = false, bool trans = false) {
+    nn_launch<0>(NnArgs<double, double>{X, c, rows, c, S, lds, nullptr, cout, upper, 1.0, nullptr, 0, 0.0, nullptr, 0,
+                                        nullptr, Out, trans ? rows : cout, trans, nullptr, cond},
+                 device_props().sms, s);
 }
 
-static void chol_inv(RandCtx& cx, const double* G, int c, int64_t rows, double* R, const int* cond) {
-    const bool two = 2 * (size_t)c * c * sizeof(double) <= 200 * 1024;
-    const size_t smem = (two ? 2 : 1) * (size_t)c * c * sizeof(double);
-    // chol_inv_body also holds about 1 KB of static shared memory
+static void chol_inv(RandCtx& cx, const double* G, int parts, int c, int64_t rows, double* R, const int* cond) {
+    const size_t smem = chol_smem(c);
+    // chol_inv_body also holds some static shared memory
     if (smem > 40 * 1024)
         SVDB_CUDA(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // shifted CholeskyQR: shift = 11 (rows c + c (c + 1)) u ||X||_F^2, ||X||_F^2 = trace(G)
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
-    k_chol_inv<<<1, 1024, smem, cx.s>>>(G, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond, two);
+    k_chol_inv<<<1, 256, smem, cx.s>>>(G, parts, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond);
     SVDB_CHECK_LAUNCH();
 }
 
@@ -457,26 +276,23 @@ static void cholesky_qr(RandCtx& cx, double* X, int64_t rows, int c, double* Rou
     if ((int64_t)cx.T.n < rows * c) cx.T.alloc(rows * c, s);
     double* T = cx.T.p;
     SVDB_CUDA(cudaMemsetAsync(cx.shifted.p, 0, sizeof(int), s));
-    // pass 1: X -> T (its Gram on the tensor cores under SVDB_MIXED: only its R1
-    // has to be good enough for pass 2, which is FP64)
-    if (cx.tensor_gram && c <= 64) gram_tensor(cx, X, rows, c, cx.G.p, nullptr);
-    else gram(cx, X, rows, c, cx.G.p, nullptr);
-    chol_inv(cx, cx.G.p, c, rows, cx.R1.p, nullptr);
-    right_mul(X, rows, c, cx.Ri.p, c, c, T, s);
-    // pass 2: T -> X
-    gram(cx, T, rows, c, cx.G.p, nullptr);
-    chol_inv(cx, cx.G.p, c, rows, cx.R2.p, nullptr);
-    right_mul(T, rows, c, cx.Ri.p, c, c, X, s);
+    auto pass = [&](const double* in, double* out, double* R, const int* cond) {
+        int parts = 0;
+        const double* G = gram(cx, in, rows, c, cx.G.p, cond, parts);
+        chol_inv(cx, G, parts, c, rows, R, cond);
+        right_mul(in, rows, c, cx.Ri.p, c, c, out, s, cond, true);
+    };
+    pass(X, T, cx.R1.p, nullptr);
+    pass(T, X, cx.R2.p, nullptr);
     // pass 3 only after a shifted pass: X -> T -> X
     const int* cond = cx.shifted.p;
-    gram(cx, X, rows, c, cx.G.p, cond);
-    chol_inv(cx, cx.G.p, c, rows, cx.R3.p, cond);
-    right_mul(X, rows, c, cx.Ri.p, c, c, T, s, cond);
+    pass(X, T, cx.R3.p, cond);
     k_copy_cond<<<nb(rows * c, 256), 256, 0, s>>>(T, X, rows * c, cond);
     SVDB_CHECK_LAUNCH();
     if (Rout) {
-        k_small_gemm<<<1, 256, 0, s>>>(cx.R2.p, cx.R1.p, c, Rout, nullptr);
-        k_small_gemm<<<1, 256, 0, s>>>(cx.R3.p, Rout, c, cx.Rtmp.p, cond);
+        const int blocks = (c * c + 127) / 128;
+        k_small_gemm<<<blocks, 128, 0, s>>>(cx.R2.p, cx.R1.p, c, Rout, nullptr);
+        k_small_gemm<<<blocks, 128, 0, s>>>(cx.R3.p, Rout, c, cx.Rtmp.p, cond);
         k_copy_cond<<<1, 256, 0, s>>>(cx.Rtmp.p, Rout, (int64_t)c * c, cond);
         SVDB_CHECK_LAUNCH_N(3);
     }
@@ -510,9 +326,11 @@ void gram_device(const double* X, int64_t rows, int c, double* G, int precision,
     cx.s = s;
     if (precision == SVDB_MIXED) {
         if (c > 64) throw Error(SVDB_ERR_UNSUPPORTED, "gram: the tensor-core form takes at most 64 columns");
-        gram_tensor(cx, X, rows, c, G, nullptr);
+        gram_tensor(cx, X, rows, c, G);
     } else {
-        gram(cx, X, rows, c, G, nullptr);
+        const TnShape h = tn_shape(rows, c, c, true, device_props().sms);
+        cx.part.alloc((int64_t)h.blocks * c * c, s);
+        tn_launch(h, X, c, c, X, c, c, rows, cx.part.p, G, nullptr, s);
     }
     SVDB_CUDA(cudaStreamSynchronize(s));
     gram_tc_check();
@@ -541,7 +359,6 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
 
     RandCtx cx;
     cx.s = s;
-    cx.tensor_gram = mixed && !getenv_is("SVDB_GRAM", "fp64");
     const int cmax = l;
     for (DevBuf<double>* b : {&cx.G, &cx.R1, &cx.R2, &cx.R3, &cx.Ri, &cx.Rtmp}) b->alloc((size_t)cmax * cmax, s);
     cx.flags.alloc(1, s);
@@ -642,49 +459,47 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
     if (verbose) printf("SVD | Randomized | Transposed Matrix Multiplication %.3f ms\n", ms_since(t0));
 
     // SVD(B), B = Bt^T (c x n).  r = min(c, n).
+    // U = Q U_B (m x r) and Vt = V_B^T, of which the leading actual_rank are kept
     const int r = (int)std::min<int64_t>(c, n);
-    DevBuf<double> UB((size_t)c * r, s), sig(r, s), VtB((size_t)r * n, s);
-    {
-        DevBuf<double> Ur((size_t)r * r, s), Vr((size_t)r * r, s), R((size_t)r * r, s);
-        const size_t smem = ((size_t)r * (r + 1) + (size_t)(r + 1) * (r + 1) + (r + 1)) * sizeof(double);
-        if (smem > 220 * 1024) throw Error(SVDB_ERR_UNSUPPORTED, "randomized_svd: sample width above the Jacobi tile");
-        SVDB_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (n >= c) {
-            // B^T = Q_b R;  R = U_J S V_J^T  ->  B = V_J S (Q_b U_J)^T.  The one-sided
-            // Jacobi runs on R^T = V_J S U_J^T, whose columns (the rows of the QR
-            // factor) are graded, which takes fewer sweeps than R itself.
-            cholesky_qr(cx, Bt.p, n, c, R.p);
-            DevBuf<double> Rt((size_t)r * r, s);
-            transpose_dense<double>(R.p, Rt.p, r, r, s);
-            k_jacobi_svd<<<1, jacobi_threads(r, 1024), smem, s>>>(Rt.p, r, Vr.p, Ur.p, sig.p, jac_status.p);
-            // U_B = V_J (c x r); V_B = Q_b U_J (n x r)
-            SVDB_CUDA(cudaMemcpyAsync(UB.p, Vr.p, (size_t)r * r * 8, cudaMemcpyDeviceToDevice, s));
-            DevBuf<double> VB((size_t)n * r, s);
-            right_mul(Bt.p, n, c, Ur.p, r, r, VB.p, s);
-            transpose_dense<double>(VB.p, VtB.p, n, r, s);
-        } else {
-            // B (c x n) is tall: B = Q_b R (R: n x n), R = U_J S V_J^T -> B = (Q_b U_J) S V_J^T
-            DevBuf<double> B((size_t)c * n, s);
-            transpose_dense<double>(Bt.p, B.p, n, c, s);
-            cholesky_qr(cx, B.p, c, (int)n, R.p);
-            DevBuf<double> Rt((size_t)r * r, s);
-            transpose_dense<double>(R.p, Rt.p, r, r, s);
-            k_jacobi_svd<<<1, jacobi_threads(r, 1024), smem, s>>>(Rt.p, r, Vr.p, Ur.p, sig.p, jac_status.p);
-            right_mul(B.p, c, (int)n, Ur.p, r, r, UB.p, s);
-            transpose_dense<double>(Vr.p, VtB.p, r, r, s);
-        }
-        SVDB_CHECK_LAUNCH();
-    }
-    if (verbose) printf("SVD | Randomized | Running Singular Value Decomposition, took %.3f ms\n", ms_since(t0));
-    // U = Q U_B (m x r), truncated to actual_rank columns
     const int64_t actual = std::min<int64_t>((int64_t)target_rank, r);
     DevBuf<double> U(std::max<int64_t>(m * actual, 1), s), Vt(std::max<int64_t>(actual * n, 1), s),
         S(std::max<int64_t>(actual, 1), s);
-    if (actual > 0) {
-        right_mul(Y.p, m, c, UB.p, r, (int)actual, U.p, s);
-        SVDB_CUDA(cudaMemcpyAsync(Vt.p, VtB.p, actual * n * 8, cudaMemcpyDeviceToDevice, s));
-        SVDB_CUDA(cudaMemcpyAsync(S.p, sig.p, actual * 8, cudaMemcpyDeviceToDevice, s));
+    {
+        DevBuf<double> Ur((size_t)r * r, s), Vr((size_t)r * r, s), R((size_t)r * r, s), Rt((size_t)r * r, s), sig(r, s);
+        const size_t smem = ((size_t)r * (r + 1) + (size_t)(r + 1) * (r + 1) + (r + 1)) * sizeof(double);
+        if (smem > 220 * 1024) throw Error(SVDB_ERR_UNSUPPORTED, "randomized_svd: sample width above the Jacobi tile");
+        SVDB_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DevBuf<double> B;  // n < c: B = Bt^T (c x n) is the tall one
+        if (n < c) {
+            B.alloc((size_t)c * n, s);
+            transpose_dense<double>(Bt.p, B.p, n, c, s);
+        }
+        // tall = Q_b R;  R = U_J S V_J^T.  The one-sided Jacobi runs on
+        // R^T = V_J S U_J^T, whose columns (the rows of the QR factor) are
+        // graded, which takes fewer sweeps than R itself.
+        double* tall = n < c ? B.p : Bt.p;
+        const int64_t trows = n < c ? c : n;
+        cholesky_qr(cx, tall, trows, r, R.p);
+        transpose_dense<double>(R.p, Rt.p, r, r, s);
+        k_jacobi_svd<<<1, jacobi_threads(r, 1024), smem, s>>>(Rt.p, r, Vr.p, Ur.p, sig.p, jac_status.p);
+        SVDB_CHECK_LAUNCH();
+        if (actual > 0) {
+            if (n >= c) {
+                // B = Bt^T = V_J S (Q_b U_J)^T: U_B = V_J, V_B = Q_b U_J
+                right_mul(Y.p, m, c, Vr.p, r, (int)actual, U.p, s);
+                right_mul(tall, n, c, Ur.p, r, (int)actual, Vt.p, s, nullptr, false, true);
+            } else {
+                // B = (Q_b U_J) S V_J^T: U_B = Q_b U_J (c x r), V_B = V_J
+                DevBuf<double> UB((size_t)c * r, s), VrT((size_t)r * r, s);
+                right_mul(tall, c, r, Ur.p, r, r, UB.p, s);
+                right_mul(Y.p, m, c, UB.p, r, (int)actual, U.p, s);
+                transpose_dense<double>(Vr.p, VrT.p, r, r, s);
+                SVDB_CUDA(cudaMemcpyAsync(Vt.p, VrT.p, actual * n * 8, cudaMemcpyDeviceToDevice, s));
+            }
+            SVDB_CUDA(cudaMemcpyAsync(S.p, sig.p, actual * 8, cudaMemcpyDeviceToDevice, s));
+        }
     }
+    if (verbose) printf("SVD | Randomized | Running Singular Value Decomposition, took %.3f ms\n", ms_since(t0));
     SVDB_CUDA(cudaEventRecord(e1, s));
     int hflags = 0, hjac = 0;
     SVDB_CUDA(cudaMemcpyAsync(&hflags, cx.flags.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -701,9 +516,11 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
         cudaEventDestroy(ev.first);
         cudaEventDestroy(ev.second);
     }
-    spmm_tma_check();
-    spmm_panel_check();
-    gram_tc_check();
+    // the opt-in product kernels' wait flags (each look is a synchronous copy)
+    if (const char* e = getenv("SVDB_SPMM"); e && *e) {
+        spmm_tma_check();
+        spmm_panel_check();
+    }
     if (split) dense_split_check();
     if (verbose) printf("SVD | Randomized | Jacobi sweeps on R: %d%s\n", hjac >> 8, (hjac & 2) ? " (limit)" : "");
     if (hflags & 2) throw Error(SVDB_ERR_LAS2, "randomized_svd: CholeskyQR broke down even with a shift");

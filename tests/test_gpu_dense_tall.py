@@ -5,7 +5,10 @@ import pytest
 
 import matrices as M
 from gpu_util import upload
-from single_svdlib import adjoint
+import oracle as O
+import torch
+from single_svdlib import _abi, adjoint, randomized
+from single_svdlib._core import check
 from test_gpu_adjoint import at_pattern, dense_reference
 
 pytestmark = pytest.mark.gpu
@@ -27,3 +30,34 @@ def test_adjoint_widths(k):
     got = adjoint.svd_adjoint(upload("csr", A), U, S, V, gU, gs, gV)
     ref = at_pattern(A, D)
     assert np.abs(got - ref).max() <= 1e-8 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("c", [1, 7, 8, 9, 24, 25, 32, 33, 40, 60, 64, 65, 96, 100, 128])
+@pytest.mark.parametrize("rows", [1, 3, 64, 65, 1000, 20011])
+def test_gram(rows, c):
+    """X^T X: rows terms of one rounding each, u sum |x_a| |x_b|, and symmetric."""
+    x = torch.from_numpy(np.random.default_rng(rows + c).standard_normal((rows, c))).cuda()
+    g = torch.full((c, c), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    check(_abi.lib().svdb_gram_device(x.data_ptr(), rows, c, g.data_ptr(), 0, None))
+    torch.cuda.synchronize()
+    bound = (rows + 2) * 2.0 ** -53 * (x.abs().T @ x.abs())
+    assert bool(((g - x.T @ x).abs() <= 2 * bound).all())  # the reference rounds as often
+    assert bool((g == g.T).all())
+
+
+@pytest.mark.parametrize("l", [1, 2, 7, 8, 9, 15, 16, 17, 33, 40, 59, 64, 65, 100, 117])
+@pytest.mark.parametrize("shape", [(260, 200), (1500, 130), (120, 700)])
+def test_solve_widths(l, shape):
+    """CholeskyQR2 (panels of eight pivots, one tile row per panel), X R^-1 and
+    the back products at every width class against the checker on the same
+    Omega.  Singular values within 1e-10, the suite's bound for FP64."""
+    m, n = shape
+    A = M.uniform(m, n, 0.3, 40 + m, -1.0, 1.0)
+    om = M.omega(n, l, l)
+    g = randomized.randomized_svd(upload("csr", A), l, 0, 1, randomized.PowerIterationNormalizer.QR, False, 3, False,
+                                  omega=om)
+    r = O.randomized(A, l, 0, 1, "QR", omega=om)
+    np.testing.assert_allclose(g.s, r["s"], rtol=1e-10)
+    k = len(g.s)
+    assert np.abs(g.u.T @ g.u - np.eye(k)).max() < 1e-12 and np.abs(g.vt @ g.vt.T - np.eye(k)).max() < 1e-12
