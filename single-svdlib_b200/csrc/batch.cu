@@ -34,14 +34,13 @@
 
 #include "dense_small.cuh"
 #include "device_common.cuh"
+#include "lean.cuh"
 #include "ops.cuh"
 #include "svdb_internal.h"
 
 namespace svdb {
 
 constexpr int kBatchMaxL = 64;      // sample columns per subset
-constexpr int kGramChunks = 16;     // Gram partials per subset
-constexpr int kBTileRows = 32;
 
 // Per-subset dense matrices.  ROWS_M: subset b at p + b * m * cols, m rows;
 // otherwise at p + coff[b] * cols with coff[b+1] - coff[b] rows.
@@ -67,12 +66,12 @@ __global__ void k_b_o2m(const int32_t* __restrict__ m2o, const int64_t* __restri
 
 // Omega_b (nb x l): entries 0 .. nb*l of the seed's stream, as a single call draws it
 template <typename T>
-__global__ void k_b_omega(uint64_t seed, const int64_t* __restrict__ coff, int l, T* __restrict__ Om) {
+__global__ void k_b_omega(uint64_t seed, const int64_t* __restrict__ coff, int l, int ld, T* __restrict__ Om) {
     const int64_t b = blockIdx.y;
-    const int64_t base = coff[b] * l, tot = (coff[b + 1] - coff[b]) * l;
+    const int64_t base = coff[b] * ld, tot = (coff[b + 1] - coff[b]) * l;
     const uint64_t key = omega_key(seed);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x)
-        Om[base + i] = (T)omega_value(key, i);
+        Om[base + (ld == l ? i : i / l * ld + i % l)] = (T)omega_value(key, i);
 }
 
 // ------------------------------------------------------------ products ----
@@ -82,13 +81,13 @@ struct ChunkType {
 };
 
 // Y_b = A_b X_b for the subsets b = g*GS + t (t < GS) of group g; item
-// (g, r), group-major, one warp each.  X_b: nb x l at X + coff[b]*l; Y_b:
-// m x l at Y + b*m*l.  Lane owns dense columns lane*CPL .. +CPL.
+// (g, r), group-major, one warp each.  X_b: nb x l at X + coff[b]*ld; Y_b:
+// m x l at Y + b*m*ld, rows ld apart.  Lane owns dense columns lane*CPL .. +CPL.
 template <typename VT, typename XT, int GS, int CPL>
 __global__ void __launch_bounds__(256) k_b_spmm_rows(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                                      const VT* __restrict__ val, int64_t m,
                                                      const int32_t* __restrict__ o2m, int64_t n,
-                                                     const int64_t* __restrict__ coff, int64_t count, int l,
+                                                     const int64_t* __restrict__ coff, int64_t count, int l, int ld,
                                                      const XT* __restrict__ X, XT* __restrict__ Y) {
     using CT = typename ChunkType<XT>::type;
     const unsigned full = 0xffffffffu;
@@ -105,7 +104,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_rows(const int64_t* __restrict__
 #pragma unroll
         for (int t = 0; t < GS; ++t) {
             bb[t] = g * GS + t;
-            xb[t] = bb[t] < count ? X + coff[bb[t]] * l : X;
+            xb[t] = bb[t] < count ? X + coff[bb[t]] * ld : X;
         }
         double acc[GS][CPL];
 #pragma unroll
@@ -135,7 +134,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_rows(const int64_t* __restrict__
                 for (int t = 0; t < GS; ++t) {
                     const int32_t jq = __shfl_sync(full, jm[t], q);
                     if (jq >= 0) {
-                        const XT* xr = xb[t] + (int64_t)jq * l + c0;
+                        const XT* xr = xb[t] + (int64_t)jq * ld + c0;
 #pragma unroll
                         for (int u = 0; u < CPL; ++u)
                             if (c0 + u < l) ch[t][u] = fma(vq, (CT)__ldg(xr + u), ch[t][u]);
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_rows(const int64_t* __restrict__
 #pragma unroll
         for (int t = 0; t < GS; ++t) {
             if (bb[t] >= count) continue;
-            XT* yr = Y + (bb[t] * m + r) * l + c0;
+            XT* yr = Y + (bb[t] * m + r) * ld + c0;
 #pragma unroll
             for (int u = 0; u < CPL; ++u)
                 if (c0 + u < l) yr[u] = (XT)acc[t][u];
@@ -164,7 +163,7 @@ template <typename VT, typename XT, typename OT, int CPL>
 __global__ void __launch_bounds__(256) k_b_spmm_cols(const int64_t* __restrict__ cp, const int32_t* __restrict__ ri,
                                                      const VT* __restrict__ cv, int64_t m,
                                                      const int32_t* __restrict__ m2o, const int64_t* __restrict__ coff,
-                                                     int64_t count, int l, const XT* __restrict__ Y,
+                                                     int64_t count, int l, int ld, const XT* __restrict__ Y,
                                                      OT* __restrict__ Z) {
     using CT = typename ChunkType<XT>::type;
     const unsigned full = 0xffffffffu;
@@ -176,7 +175,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_cols(const int64_t* __restrict__
     int64_t b = 0;
     for (int64_t it = warp0; it < total; it += nw) {
         while (coff[b + 1] <= it) ++b;  // items rise, so b only moves forward
-        const XT* yb = Y + b * m * l;
+        const XT* yb = Y + b * m * ld;
         const int32_t c = m2o[it];
         const int64_t s = cp[c], e = cp[c + 1];
         double acc[CPL];
@@ -197,7 +196,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_cols(const int64_t* __restrict__
             for (int q = 0; q < cnt; ++q) {
                 const CT vq = __shfl_sync(full, vm, q);
                 const int32_t rq = __shfl_sync(full, rm, q);
-                const XT* yr = yb + (int64_t)rq * l + c0;
+                const XT* yr = yb + (int64_t)rq * ld + c0;
 #pragma unroll
                 for (int u = 0; u < CPL; ++u)
                     if (c0 + u < l) ch[u] = fma(vq, (CT)__ldg(yr + u), ch[u]);
@@ -205,7 +204,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_cols(const int64_t* __restrict__
 #pragma unroll
             for (int u = 0; u < CPL; ++u) acc[u] += (double)ch[u];
         }
-        OT* zr = Z + it * l + c0;
+        OT* zr = Z + it * ld + c0;
 #pragma unroll
         for (int u = 0; u < CPL; ++u)
             if (c0 + u < l) zr[u] = (OT)acc[u];
@@ -230,7 +229,7 @@ constexpr int kBLeanU = 8;  // gathers in flight per lane
 // (cnt == 32) needs no bounds tests.  X is the same for the whole warp and
 // the offsets are 32-bit (no 64-bit per-lane address arithmetic).
 template <int H>
-__device__ __forceinline__ void lean_chunk(const int2* __restrict__ E, int cnt, int g, bool active,
+__device__ __forceinline__ void lean_chunk32(const int2* __restrict__ E, int cnt, int g, bool active,
                                            const float* __restrict__ X, uint32_t c0, float (&c4)[4]) {
     constexpr int PER = 32 / H;
     if (cnt == 32) {
@@ -340,7 +339,7 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, 4)
             if (fill >= 32) {
                 __syncwarp();
                 float c4[4] = {0.f, 0.f, 0.f, 0.f};
-                lean_chunk<H>(E, 32, g, active, Xb, c0a, c4);
+                lean_chunk32<H>(E, 32, g, active, Xb, c0a, c4);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[j] += (double)c4[j];
                 __syncwarp();  // every lane has read E[0 .. 32)
@@ -354,7 +353,7 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, 4)
         if (fill > 0) {
             __syncwarp();
             float c4[4] = {0.f, 0.f, 0.f, 0.f};
-            lean_chunk<H>(E, fill, g, active, Xb, c0a, c4);
+            lean_chunk32<H>(E, fill, g, active, Xb, c0a, c4);
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] += (double)c4[j];
         }
@@ -410,7 +409,7 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, 4)
                 myv = __ldg(cv + k0 + 32 + lane);
             }
             float c4[4] = {0.f, 0.f, 0.f, 0.f};
-            lean_chunk<H>(E, cnt, g, active, Yb, c0a, c4);
+            lean_chunk32<H>(E, cnt, g, active, Yb, c0a, c4);
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] += (double)c4[j];
         }
@@ -428,74 +427,208 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, 4)
 }
 
 
-// --------------------------------------------------------- CholeskyQR2 ----
-// Gram partials: block (chunk, b) sums X_b^T X_b over its rows (32-row tiles
-// staged in shared memory; a 16 x 16 thread grid holds an NC x NC tile).
-template <typename T, int NC>
-__global__ void __launch_bounds__(256) k_b_gram_part(const T* __restrict__ X, SubLayout L,
-                                                     const int64_t* __restrict__ coff, int c,
-                                                     double* __restrict__ part, const int* __restrict__ cond) {
-    const int64_t b = blockIdx.y;
-    if (cond && cond[b] == 0) return;
-    extern __shared__ double xs[];  // kBTileRows x c
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int64_t rows = sub_rows(L, coff, b);
-    const T* xb = X + sub_row0(L, coff, b) * c;
-    const int64_t chunk = (rows + gridDim.x - 1) / gridDim.x;
-    const int64_t r0 = blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
-    double acc[NC][NC];
+// The FP64 forms of the two kernels above, for any l <= 64: the dense rows are
+// ld (even) doubles apart, and groups of GL lanes with NL vectors of two
+// columns each gather them (lean.cuh).  12 subsets of a 10,007 x 3,001 matrix,
+// l = 17: rows 149 us and columns 121 us per product, against 420 and 600 for
+// the warp-per-entry kernels (ncu, cold caches).
+template <int H, int NL>
+__global__ void __launch_bounds__(kBLeanWarps * 32, NL == 3 ? 2 : 3)
+    k_b_rows_lean64(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ val,
+                    int64_t m, const int32_t* __restrict__ o2m, int64_t n, const int64_t* __restrict__ coff,
+                    int64_t count, int l, int ld, const double* __restrict__ X, double* __restrict__ Y,
+                    unsigned long long* __restrict__ next) {
+    constexpr int GL = 32 / H, U = H == 8 ? 4 : NL == 1 ? 8 : 4;
+    using Slots = LeanSlots<double, H>;
+    // members waiting: the first 32 in slot order, the rest as they come
+    __shared__ __align__(16) uint32_t s_off[kBLeanWarps][64];
+    __shared__ __align__(16) double s_val[kBLeanWarps][H * Slots::VS + 32];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / GL, gl = lane % GL;
+    bool active[NL];
+    uint32_t col[NL];
 #pragma unroll
-    for (int i = 0; i < NC; ++i)
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * 2;
+        active[j] = c < l;
+        col[j] = active[j] ? (uint32_t)c : 0u;
+    }
+    uint32_t* const O = s_off[w];
+    double* const V = s_val[w];
+    const uint32_t* const og = O + g * Slots::PER;
+    const double* const vg = V + g * Slots::VS;
+    auto put = [&](int k, uint32_t off, double v) {
+        if (k < 32) {
+            O[Slots::off(k)] = off;
+            V[Slots::val(k)] = v;
+        } else {
+            O[k] = off;
+            V[H * Slots::VS + k - 32] = v;
+        }
+    };
+    const int64_t items = count * m;
+    for (int64_t it = lean_next(next, lane); it < items; it = lean_next(next, lane)) {
+        const int64_t b = it / m, r = it - b * m;
+        const double* Xb = X + coff[b] * ld;
+        const int32_t* om = o2m + b * n;
+        const int64_t s = __ldg(rp + r), e = __ldg(rp + r + 1);
+        double acc[NL][2];
 #pragma unroll
-        for (int j = 0; j < NC; ++j) acc[i][j] = 0.0;
-    for (int64_t rb = r0; rb < r1; rb += kBTileRows) {
-        const int nr = (int)min((int64_t)kBTileRows, r1 - rb);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * c; t += blockDim.x) xs[t] = (double)xb[rb * c + t];
-        __syncthreads();
-        for (int r = 0; r < nr; ++r) {
-            double xa[NC], xc[NC];
-#pragma unroll
-            for (int i = 0; i < NC; ++i) {
-                const int a = ty + 16 * i, bq = tx + 16 * i;
-                xa[i] = a < c ? xs[r * c + a] : 0.0;
-                xc[i] = bq < c ? xs[r * c + bq] : 0.0;
+        for (int j = 0; j < NL; ++j) acc[j][0] = acc[j][1] = 0.0;
+        int32_t jm = -1, nxc = 0;
+        double myv = 0.0, nxv = 0.0;
+        if (s + lane < e) { myv = __ldg(val + s + lane); jm = __ldg(om + __ldg(ci + s + lane)); }
+        if (s + 32 + lane < e) { nxc = __ldg(ci + s + 32 + lane); nxv = __ldg(val + s + 32 + lane); }
+        int fill = 0;
+        for (int64_t k0 = s; k0 < e; k0 += 32) {
+            const unsigned mask = __ballot_sync(full, jm >= 0);
+            if (jm >= 0) put(fill + __popc(mask & ((1u << lane) - 1u)), (uint32_t)jm * (uint32_t)ld, myv);
+            fill += __popc(mask);
+            jm = (k0 + 32 + lane < e) ? __ldg(om + nxc) : -1;
+            myv = nxv;
+            if (k0 + 64 + lane < e) {
+                nxc = __ldg(ci + k0 + 64 + lane);
+                nxv = __ldg(val + k0 + 64 + lane);
             }
-#pragma unroll
-            for (int i = 0; i < NC; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j) acc[i][j] = fma(xa[i], xc[j], acc[i][j]);
+            if (fill >= 32) {
+                __syncwarp();
+                lean_chunk<double, H, NL, U, false>(og, vg, 32, g, Xb, col, active, acc);
+                __syncwarp();  // every lane has read the first 32
+                if (lane < fill - 32) put(lane, O[32 + lane], V[H * Slots::VS + lane]);
+                fill -= 32;
+                __syncwarp();
+            }
         }
+        __syncwarp();
+        if (fill > 0) lean_chunk<double, H, NL, U, false>(og, vg, fill, g, Xb, col, active, acc);
+        __syncwarp();  // the buffer is free for the next item
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) acc[j][q] += __shfl_xor_sync(full, acc[j][q], o);
+        if (g != 0) continue;
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+            if (active[j])  // ld is even: the column past an odd l is padding
+                *reinterpret_cast<double2*>(Y + (b * m + r) * ld + col[j]) = make_double2(acc[j][0], acc[j][1]);
     }
-    double* out = part + (b * gridDim.x + blockIdx.x) * (int64_t)c * c;
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            const int a = ty + 16 * i, bq = tx + 16 * j;
-            if (a < c && bq < c) out[a * c + bq] = acc[i][j];
-        }
 }
 
-// G_b = sum of the subset's partials in chunk order
-__global__ void k_b_gram_reduce(const double* __restrict__ part, int nchunk, int c, double* __restrict__ G,
-                                const int* __restrict__ cond) {
+template <int H, int NL>
+__global__ void __launch_bounds__(kBLeanWarps * 32, NL == 3 ? 2 : 3)
+    k_b_cols_lean64(const int64_t* __restrict__ cp, const int32_t* __restrict__ ri, const double* __restrict__ cv,
+                    int64_t m, const int32_t* __restrict__ m2o, const int64_t* __restrict__ coff, int64_t count,
+                    int l, int ld, const double* __restrict__ Y, double* __restrict__ Z,
+                    unsigned long long* __restrict__ next) {
+    constexpr int GL = 32 / H, U = H == 8 ? 4 : NL == 1 ? 8 : 4;
+    using Slots = LeanSlots<double, H>;
+    __shared__ __align__(16) uint32_t s_off[kBLeanWarps][32];
+    __shared__ __align__(16) double s_val[kBLeanWarps][H * Slots::VS];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / GL, gl = lane % GL;
+    bool active[NL];
+    uint32_t col[NL];
+#pragma unroll
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * 2;
+        active[j] = c < l;
+        col[j] = active[j] ? (uint32_t)c : 0u;
+    }
+    uint32_t* const oput = s_off[w] + Slots::off(lane);
+    double* const vput = s_val[w] + Slots::val(lane);
+    const uint32_t* const og = s_off[w] + g * Slots::PER;
+    const double* const vg = s_val[w] + g * Slots::VS;
+    const int64_t total = coff[count];
+    int64_t b = 0;
+    for (int64_t it = lean_next(next, lane); it < total; it = lean_next(next, lane)) {
+        while (coff[b + 1] <= it) ++b;  // a warp's items rise, so b only moves forward
+        const double* Yb = Y + b * m * ld;
+        const int32_t c = m2o[it];
+        const int64_t s = __ldg(cp + c);
+        int64_t left = __ldg(cp + c + 1) - s;
+        const int32_t* rp = ri + s + lane;
+        const double* vp = cv + s + lane;
+        double acc[NL][2];
+#pragma unroll
+        for (int j = 0; j < NL; ++j) acc[j][0] = acc[j][1] = 0.0;
+        int32_t myr = 0;
+        double myv = 0.0;
+        if (lane < left) { myr = __ldg(rp); myv = __ldg(vp); }
+        for (; left > 0; left -= 32) {
+            __syncwarp();
+            *oput = (uint32_t)myr * (uint32_t)ld;
+            *vput = myv;
+            __syncwarp();
+            rp += 32;
+            vp += 32;
+            if (lane + 32 < left) { myr = __ldg(rp); myv = __ldg(vp); }
+            lean_chunk<double, H, NL, U, false>(og, vg, left < 32 ? (int)left : 32, g, Yb, col, active, acc);
+        }
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) acc[j][q] += __shfl_xor_sync(full, acc[j][q], o);
+        if (g != 0) continue;
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+            if (active[j])
+                *reinterpret_cast<double2*>(Z + it * ld + col[j]) = make_double2(acc[j][0], acc[j][1]);
+    }
+}
+
+// --------------------------------------------------------- CholeskyQR2 ----
+// Gram partials: block (chunk, b) sums X_b^T X_b over its rows on the FP64
+// matrix instruction (dense_tall.cuh), the tile blocks I <= J only.  16
+// subsets, l = 40, the 20,000-row and the about 2,250-row operands of a mixed
+// solve: 32 us on average, against 129 for register tiles staged through
+// shared memory.
+template <typename T, int NT>
+__global__ void __launch_bounds__(512, 1) k_b_gram_part(const T* __restrict__ X, SubLayout L,
+                                                        const int64_t* __restrict__ coff, int c, int ld, int nb, int rg,
+                                                        double* __restrict__ part, const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
-    const int cc = c * c;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < cc; p += gridDim.x * blockDim.x) {
-        double s0 = 0.0, s1 = 0.0;
-        int k = 0;
-        for (; k + 2 <= nchunk; k += 2) {
-            s0 += part[(b * nchunk + k) * cc + p];
-            s1 += part[(b * nchunk + k + 1) * cc + p];
-        }
-        if (k < nchunk) s0 += part[(b * nchunk + k) * cc + p];
-        G[b * cc + p] = s0 + s1;
+    extern __shared__ double bg_sm[];
+    const int64_t rows = sub_rows(L, coff, b), step = 4 * rg;
+    const int64_t chunk = ((rows + gridDim.x - 1) / gridDim.x + step - 1) / step * step;
+    const int64_t r0 = blockIdx.x * chunk;
+    const T* xb = X + sub_row0(L, coff, b) * ld;
+    tn_part_body<T, T, NT>(xb, ld, c, xb, ld, c, min(r0, rows), min(rows, r0 + chunk), nb, nb, true, rg,
+                           part + (b * gridDim.x + blockIdx.x) * (int64_t)c * c, bg_sm);
+}
+
+// G_b = sum of the subset's partials in chunk order (elements of tile blocks
+// below the diagonal are not read by the factorisation and stay undefined)
+__global__ void __launch_bounds__(256) k_b_gram_reduce(const double* __restrict__ part, int nchunk, int c,
+                                                       double* __restrict__ G, const int* __restrict__ cond) {
+    const int64_t b = blockIdx.y;
+    if (cond && cond[b] == 0) return;
+    __shared__ double sh[8][32];
+    const int cc = c * c, lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
+    double acc = 0.0;
+    if (p < cc) {
+        const int per = (nchunk + 7) / 8, k0 = sl * per, k1 = min(nchunk, k0 + per);
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) acc += part[(b * nchunk + k) * cc + p];
+    }
+    sh[sl][lane] = acc;
+    __syncthreads();
+    if (sl == 0 && p < cc) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t += sh[k][lane];
+        G[b * cc + p] = t;
     }
 }
 
-__global__ void __launch_bounds__(256) k_b_chol_inv(const double* __restrict__ G, int c, SubLayout L, const int64_t* __restrict__ coff,
+__global__ void __launch_bounds__(256) k_b_chol_inv(const double* __restrict__ G, int nparts, int c, SubLayout L, const int64_t* __restrict__ coff,
                              double* __restrict__ R, double* __restrict__ Ri, int* __restrict__ flags,
                              int* __restrict__ shifted, const int* __restrict__ cond) {
     const int64_t b = blockIdx.x;
@@ -504,49 +637,39 @@ __global__ void __launch_bounds__(256) k_b_chol_inv(const double* __restrict__ G
     const int64_t rows = sub_rows(L, coff, b);
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
     const int64_t cc = (int64_t)c * c;
-    chol_inv_body(G + b * cc, 0, c, shift_scale, R + b * cc, Ri + b * cc, flags + b, shifted + b, sm);
+    chol_inv_body(G + b * cc * max(nparts, 1), nparts, c, shift_scale, R + b * cc, Ri + b * cc, flags + b, shifted + b, sm);
 }
 
-// Out_b (rows x cout) = X_b (rows x c) S_b (c x lds, first cout columns),
-// S_b = S + b*c*lds.  X and Out may be the same array (each tile is staged
-// before it is written).  TRANS: Out_b is stored cout x rows.
-template <typename TI, typename TO, bool TRANS>
-__global__ void __launch_bounds__(256) k_b_right_mul(const TI* X, SubLayout LX, const int64_t* __restrict__ coff,
-                                                     int c, const double* __restrict__ S, int lds, int cout, TO* Out,
-                                                     const int* __restrict__ cond) {
+// Out_b (rows x cout) = X_b (rows x c) S_b (c x c, first cout columns) on the
+// FP64 matrix instruction (dense_tall.cuh).  X and Out may be the same array
+// (a warp has read its rows before it writes them).  trans: Out_b is stored
+// cout x rows.  The same solve's: 35 us on average, against 162 for a dot
+// product per thread.
+template <typename TI, typename TO, int NQ>
+__global__ void __launch_bounds__(32 * kNnWarps, 2) k_b_right_mul(const TI* X, SubLayout L,
+                                                                  const int64_t* __restrict__ coff, int c, int ldx,
+                                                                  const double* __restrict__ S, int cout, int upper,
+                                                                  TO* Out, int ldo, int trans,
+                                                                  const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
-    extern __shared__ double sm[];
-    double* ss = sm;                // c x cout
-    double* xs = sm + c * cout;     // kBTileRows x c
-    const double* sb = S + b * (int64_t)c * lds;
-    for (int t = threadIdx.x; t < c * cout; t += blockDim.x) ss[t] = sb[(t / cout) * lds + t % cout];
-    const int64_t rows = sub_rows(LX, coff, b), row0 = sub_row0(LX, coff, b);
-    const TI* xb = X + row0 * c;
-    TO* ob = Out + row0 * cout;
-    for (int64_t r0 = (int64_t)blockIdx.x * kBTileRows; r0 < rows; r0 += (int64_t)gridDim.x * kBTileRows) {
-        const int nr = (int)min((int64_t)kBTileRows, rows - r0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * c; t += blockDim.x) xs[t] = (double)xb[r0 * c + t];
-        __syncthreads();
-        for (int t = threadIdx.x; t < nr * cout; t += blockDim.x) {
-            const int rr = TRANS ? t % nr : t / cout, j = TRANS ? t / nr : t % cout;
-            const double* xr = xs + rr * c;
-            double s = 0.0;
-            for (int k = 0; k < c; ++k) s = fma(xr[k], ss[k * cout + j], s);
-            if (TRANS) ob[(int64_t)j * rows + r0 + rr] = (TO)s;
-            else ob[(r0 + rr) * cout + j] = (TO)s;
-        }
-    }
+    extern __shared__ double br_sm[];
+    const int64_t rows = sub_rows(L, coff, b), row0 = sub_row0(L, coff, b);
+    if ((int64_t)blockIdx.x * kNnWarps * 8 * kNnMT >= rows) return;
+    const NnArgs<TI, TO> A{X + row0 * ldx, ldx, rows, c, S + b * (int64_t)c * c, c, nullptr, cout, upper, 1.0, nullptr,
+                           0, 0.0, nullptr, 0, nullptr, Out + row0 * (trans ? cout : ldo), trans ? rows : ldo, trans,
+                           nullptr, nullptr};
+    nn_body<TI, TO, NQ, 0>(A, (int64_t)blockIdx.x * kNnWarps + (threadIdx.x >> 5), (int64_t)gridDim.x * kNnWarps, 0,
+                           br_sm);
 }
 
-// C_b = A_b B_b (c x c), one block per subset
+// C_b = A_b B_b (c x c), one thread per element
 __global__ void k_b_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int c,
                                double* __restrict__ C, const int* __restrict__ cond) {
-    const int64_t b = blockIdx.x;
+    const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
     const int64_t cc = (int64_t)c * c;
-    for (int t = threadIdx.x; t < c * c; t += blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < c * c; t += gridDim.x * blockDim.x) {
         const int i = t / c, j = t % c;
         double s = 0.0;
         for (int k = 0; k < c; ++k) s = fma(A[b * cc + i * c + k], B[b * cc + k * c + j], s);
@@ -563,23 +686,23 @@ __global__ void k_b_copy_cond(const double* __restrict__ src, double* __restrict
 
 // LU normaliser (mod.rs:239-293): column j of X_b scaled to unit norm unless its norm is <= 1e-10
 template <typename T>
-__global__ void k_b_colnorm(T* __restrict__ X, SubLayout L, const int64_t* __restrict__ coff, int c) {
+__global__ void k_b_colnorm(T* __restrict__ X, SubLayout L, const int64_t* __restrict__ coff, int ld) {
     __shared__ double sh[32];
     __shared__ double scale;
     const int j = blockIdx.x;
     const int64_t b = blockIdx.y;
     const int64_t rows = sub_rows(L, coff, b);
-    T* xb = X + sub_row0(L, coff, b) * c;
+    T* xb = X + sub_row0(L, coff, b) * ld;
     double acc = 0.0;
     for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) {
-        const double v = (double)xb[r * c + j];
+        const double v = (double)xb[r * ld + j];
         acc = fma(v, v, acc);
     }
     const double nrm = sqrt(block_sum(acc, sh));
     if (threadIdx.x == 0) scale = nrm > 1e-10 ? 1.0 / nrm : 1.0;
     __syncthreads();
     if (nrm > 1e-10)
-        for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) xb[r * c + j] = (T)((double)xb[r * c + j] * scale);
+        for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) xb[r * ld + j] = (T)((double)xb[r * ld + j] * scale);
 }
 
 __global__ void __launch_bounds__(512) k_b_jacobi(const double* __restrict__ R, int c, double* __restrict__ U,
@@ -609,6 +732,8 @@ struct svdb_batch {
     cudaStream_t s = nullptr;
     bool mixed = false, on_device = false, use_graph = true;
     int64_t m = 0, n = 0, count = 0, rank = 0, l = 0, q = 0, total_cols = 0;
+    int ld = 0;         // row stride of the dense operands: l, even at FP64 (16-byte rows)
+    int gram_parts = 1;  // Gram partials per subset
     int normalizer = 0;
     uint64_t seed = 0;
     int gs = 4, cpl = 2;
@@ -650,12 +775,23 @@ static T* dense_ptr(svdb_batch& B, DevBuf<float>& f, DevBuf<double>& d) {
     else return d.p;
 }
 
-// the lean kernels apply to SVDB_MIXED batches with l a multiple of 4
-// (16-byte rows), 32-bit offsets, and SVDB_BATCH_SPMM=warp not set
+// the lean kernels apply with 32-bit offsets, and at FP32 with l a multiple of
+// 4 (16-byte rows; other widths keep the warp kernels' FP32 summation order);
+// SVDB_BATCH_SPMM=warp turns them off
 static bool lean_batch(const svdb_batch& B, int64_t rows_per_item_operand) {
     const char* e = getenv("SVDB_BATCH_SPMM");
     if (e && std::string(e) == "warp") return false;
-    return B.mixed && B.l % 4 == 0 && B.l <= 64 && rows_per_item_operand * B.l < ((int64_t)1 << 31);
+    return (!B.mixed || B.l % 4 == 0) && B.l <= 64 && rows_per_item_operand * B.ld < ((int64_t)1 << 31);
+}
+
+// FP64 lane groups as narrow as the columns allow, as launch_lean (spmm.cu)
+template <typename F>
+static void lean64_width(int l, F&& f) {
+    if (l <= 8) f(std::integral_constant<int, 8>(), std::integral_constant<int, 1>());
+    else if (l <= 16) f(std::integral_constant<int, 4>(), std::integral_constant<int, 1>());
+    else if (l <= 32) f(std::integral_constant<int, 4>(), std::integral_constant<int, 2>());
+    else if (l <= 48) f(std::integral_constant<int, 4>(), std::integral_constant<int, 3>());
+    else f(std::integral_constant<int, 2>(), std::integral_constant<int, 2>());
 }
 
 // Y_b = A_b X_b with `gs` subsets per row item
@@ -680,16 +816,26 @@ static void rows_product(svdb_batch& B, const T* X, T* Y, int gs) {
                 dense_batch_rows(B.A, X, B.coff.p, B.o2m.p, B.count, (int)B.l, Y, B.dbh_r.p, B.dbl_r.p, B.s);
             return;
         }
+    } else {
+        if (lean_batch(B, B.n)) {
+            SVDB_CUDA(cudaMemsetAsync(B.next.p, 0, sizeof(unsigned long long), B.s));
+            lean64_width((int)B.l, [&](auto h, auto nl) {
+                k_b_rows_lean64<h.value, nl.value><<<grid_cap(nl.value == 3 ? 2 : 3), kBLeanWarps * 32, 0, B.s>>>(
+                    A.ptr.p, A.idx.p, A.val.p, B.m, B.o2m.p, B.n, B.coff.p, B.count, (int)B.l, B.ld, X, Y, B.next.p);
+            });
+            SVDB_CHECK_LAUNCH();
+            return;
+        }
     }
     const int blocks = grid_cap(6);
 #define SVDB_ROWS(GS)                                                                                             \
     case GS:                                                                                                      \
         if (B.mixed)                                                                                              \
             k_b_spmm_rows<float, T, GS, 2><<<blocks, 256, 0, B.s>>>(A.ptr.p, A.idx.p, A.val32.p, B.m, B.o2m.p,     \
-                                                                    B.n, B.coff.p, B.count, (int)B.l, X, Y);      \
+                                                                    B.n, B.coff.p, B.count, (int)B.l, B.ld, X, Y); \
         else                                                                                                      \
             k_b_spmm_rows<double, T, GS, 2><<<blocks, 256, 0, B.s>>>(A.ptr.p, A.idx.p, A.val.p, B.m, B.o2m.p,      \
-                                                                     B.n, B.coff.p, B.count, (int)B.l, X, Y);     \
+                                                                     B.n, B.coff.p, B.count, (int)B.l, B.ld, X, Y); \
         break;
     switch (gs) {
         SVDB_ROWS(1)
@@ -729,14 +875,24 @@ static void cols_product(svdb_batch& B, const T* Y, OT* Z) {
                                      B.dpart.p, B.s);
             return;
         }
+    } else {
+        if (lean_batch(B, B.m)) {
+            SVDB_CUDA(cudaMemsetAsync(B.next.p, 0, sizeof(unsigned long long), B.s));
+            lean64_width((int)B.l, [&](auto h, auto nl) {
+                k_b_cols_lean64<h.value, nl.value><<<grid_cap(nl.value == 3 ? 2 : 3), kBLeanWarps * 32, 0, B.s>>>(
+                    At.ptr.p, At.idx.p, At.val.p, B.m, B.m2o.p, B.coff.p, B.count, (int)B.l, B.ld, Y, Z, B.next.p);
+            });
+            SVDB_CHECK_LAUNCH();
+            return;
+        }
     }
     const int blocks = grid_cap(8);
     if (B.mixed)
         k_b_spmm_cols<float, T, OT, 2><<<blocks, 256, 0, B.s>>>(At.ptr.p, At.idx.p, At.val32.p, B.m, B.m2o.p,
-                                                                B.coff.p, B.count, (int)B.l, Y, Z);
+                                                                B.coff.p, B.count, (int)B.l, B.ld, Y, Z);
     else
         k_b_spmm_cols<double, T, OT, 2><<<blocks, 256, 0, B.s>>>(At.ptr.p, At.idx.p, At.val.p, B.m, B.m2o.p,
-                                                                 B.coff.p, B.count, (int)B.l, Y, Z);
+                                                                 B.coff.p, B.count, (int)B.l, B.ld, Y, Z);
     SVDB_CHECK_LAUNCH();
     if constexpr (std::is_same<T, float>::value) {
         if (B.dsplit)
@@ -745,50 +901,73 @@ static void cols_product(svdb_batch& B, const T* Y, OT* Z) {
     }
 }
 
+// Gram partials of every X_b, then their sums in B.G unless the factorisation
+// adds them itself (parts > 0: small ones)
+constexpr int64_t kBCholParts = 16384;
 template <typename T>
-static void gram(svdb_batch& B, const T* X, SubLayout L, const int* cond) {
+static const double* gram(svdb_batch& B, const T* X, SubLayout L, const int* cond, int& parts) {
     const int c = (int)B.l;
-    const size_t smem = (size_t)kBTileRows * c * sizeof(double);
-    dim3 grid(kGramChunks, (unsigned)B.count);
-    const int nc = (c + 15) / 16;
-    switch (nc) {
-        case 1: k_b_gram_part<T, 1><<<grid, 256, smem, B.s>>>(X, L, B.coff.p, c, B.part.p, cond); break;
-        case 2: k_b_gram_part<T, 2><<<grid, 256, smem, B.s>>>(X, L, B.coff.p, c, B.part.p, cond); break;
-        case 3: k_b_gram_part<T, 3><<<grid, 256, smem, B.s>>>(X, L, B.coff.p, c, B.part.p, cond); break;
-        default: k_b_gram_part<T, 4><<<grid, 256, smem, B.s>>>(X, L, B.coff.p, c, B.part.p, cond); break;
+    const TnShape h = tn_shape(1, c, c, true, 1);  // the tiles; the chunks are the kernel's own
+    const dim3 grid(B.gram_parts, (unsigned)B.count);
+    auto go = [&](auto kern) {
+        if (h.smem() > 48 * 1024)
+            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem()));
+        kern<<<grid, h.threads(), h.smem(), B.s>>>(X, L, B.coff.p, c, B.ld, h.nbp, h.rg, B.part.p, cond);
+    };
+    switch (h.nt) {
+        case 1: go(k_b_gram_part<T, 1>); break;
+        case 2: go(k_b_gram_part<T, 2>); break;
+        case 3: go(k_b_gram_part<T, 3>); break;
+        default: go(k_b_gram_part<T, 4>); break;
     }
-    k_b_gram_reduce<<<dim3((c * c + 127) / 128, (unsigned)B.count), 128, 0, B.s>>>(B.part.p, kGramChunks, c, B.G.p,
-                                                                                   cond);
-    SVDB_CHECK_LAUNCH_N(2);
+    SVDB_CHECK_LAUNCH();
+    parts = (int64_t)B.gram_parts * c * c <= kBCholParts ? B.gram_parts : 0;
+    if (parts) return B.part.p;
+    k_b_gram_reduce<<<dim3((c * c + 31) / 32, (unsigned)B.count), 256, 0, B.s>>>(B.part.p, B.gram_parts, c, B.G.p,
+                                                                                 cond);
+    SVDB_CHECK_LAUNCH();
+    return B.G.p;
 }
 
-template <typename TI, typename TO, bool TRANS>
-static void right_mul(svdb_batch& B, const TI* X, SubLayout L, const double* S, int lds, int cout, TO* Out,
-                      const int* cond) {
-    const int c = (int)B.l;
-    const size_t smem = ((size_t)c * cout + (size_t)kBTileRows * c) * sizeof(double);
-    if (smem > 48 * 1024)
-        SVDB_CUDA(cudaFuncSetAttribute(k_b_right_mul<TI, TO, TRANS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+template <typename TI, typename TO>
+static void right_mul(svdb_batch& B, const TI* X, SubLayout L, const double* S, bool upper, int cout, TO* Out, int ldo,
+                      bool trans, const int* cond) {
+    const int c = (int)B.l, nq = (cout + 7) / 8;
+    const size_t smem = nn_smem(c, nq);
     int64_t rows = L.by_coff ? 0 : L.m;
     if (L.by_coff)
         for (int64_t b = 0; b < B.count; ++b) rows = std::max(rows, B.coff_h[b + 1] - B.coff_h[b]);
-    // about 8 blocks per SM over all subsets
-    const int64_t per_subset = std::max<int64_t>(1, (int64_t)device_props().sms * 8 / B.count);
-    const unsigned tiles =
-        (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + kBTileRows - 1) / kBTileRows, per_subset));
-    k_b_right_mul<TI, TO, TRANS><<<dim3(tiles, (unsigned)B.count), 256, smem, B.s>>>(X, L, B.coff.p, c, S, lds, cout,
-                                                                                     Out, cond);
+    // about four blocks per SM over all subsets
+    const int64_t per_subset = std::max<int64_t>(1, (int64_t)device_props().sms * 4 / B.count);
+    const int64_t tile = 8 * kNnMT * kNnWarps;
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + tile - 1) / tile, per_subset)),
+                    (unsigned)B.count);
+    auto go = [&](auto kern) {
+        if (smem > 48 * 1024)
+            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<grid, 32 * kNnWarps, smem, B.s>>>(X, L, B.coff.p, c, B.ld, S, cout, (int)upper, Out, ldo, (int)trans,
+                                                 cond);
+    };
+    switch (nq) {
+        case 1: go(k_b_right_mul<TI, TO, 1>); break;
+        case 2: go(k_b_right_mul<TI, TO, 2>); break;
+        case 3: go(k_b_right_mul<TI, TO, 3>); break;
+        case 4: go(k_b_right_mul<TI, TO, 4>); break;
+        case 5: go(k_b_right_mul<TI, TO, 5>); break;
+        case 6: go(k_b_right_mul<TI, TO, 6>); break;
+        case 7: go(k_b_right_mul<TI, TO, 7>); break;
+        default: go(k_b_right_mul<TI, TO, 8>); break;
+    }
     SVDB_CHECK_LAUNCH();
 }
 
-static void chol(svdb_batch& B, SubLayout L, double* R, const int* cond) {
+static void chol(svdb_batch& B, SubLayout L, const double* G, int parts, double* R, const int* cond) {
     const int c = (int)B.l;
     const size_t smem = chol_smem(c);
     // chol_inv_body also holds some static shared memory
     if (smem > 40 * 1024)
         SVDB_CUDA(cudaFuncSetAttribute(k_b_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_b_chol_inv<<<(unsigned)B.count, 256, smem, B.s>>>(B.G.p, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,
+    k_b_chol_inv<<<(unsigned)B.count, 256, smem, B.s>>>(G, parts, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,
                                                          cond);
     SVDB_CHECK_LAUNCH();
 }
@@ -799,19 +978,20 @@ template <typename T>
 static void cholesky_qr(svdb_batch& B, T* X, SubLayout L, bool want_r) {
     const int c = (int)B.l;
     SVDB_CUDA(cudaMemsetAsync(B.shifted.p, 0, B.count * sizeof(int), B.s));
-    gram<T>(B, X, L, nullptr);
-    chol(B, L, B.R1.p, nullptr);
-    right_mul<T, T, false>(B, X, L, B.Ri.p, c, c, X, nullptr);
-    gram<T>(B, X, L, nullptr);
-    chol(B, L, B.R2.p, nullptr);
-    right_mul<T, T, false>(B, X, L, B.Ri.p, c, c, X, nullptr);
+    auto pass = [&](double* R, const int* cond) {
+        int parts = 0;
+        const double* G = gram<T>(B, X, L, cond, parts);
+        chol(B, L, G, parts, R, cond);
+        right_mul<T, T>(B, X, L, B.Ri.p, true, c, X, B.ld, false, cond);
+    };
+    pass(B.R1.p, nullptr);
+    pass(B.R2.p, nullptr);
     const int* cond = B.shifted.p;
-    gram<T>(B, X, L, cond);
-    chol(B, L, B.R3.p, cond);
-    right_mul<T, T, false>(B, X, L, B.Ri.p, c, c, X, cond);
+    pass(B.R3.p, cond);
     if (want_r) {
-        k_b_small_gemm<<<(unsigned)B.count, 256, 0, B.s>>>(B.R2.p, B.R1.p, c, B.Rout.p, nullptr);
-        k_b_small_gemm<<<(unsigned)B.count, 256, 0, B.s>>>(B.R3.p, B.Rout.p, c, B.Rtmp.p, cond);
+        const dim3 grid((c * c + 127) / 128, (unsigned)B.count);
+        k_b_small_gemm<<<grid, 128, 0, B.s>>>(B.R2.p, B.R1.p, c, B.Rout.p, nullptr);
+        k_b_small_gemm<<<grid, 128, 0, B.s>>>(B.R3.p, B.Rout.p, c, B.Rtmp.p, cond);
         k_b_copy_cond<<<dim3(1, (unsigned)B.count), 256, 0, B.s>>>(B.Rtmp.p, B.Rout.p, (int64_t)c * c, cond);
         SVDB_CHECK_LAUNCH_N(3);
     }
@@ -822,7 +1002,7 @@ static void normalize(svdb_batch& B, T* X, SubLayout L) {
     if (B.normalizer == SVDB_NORM_QR) {
         cholesky_qr<T>(B, X, L, false);
     } else if (B.normalizer == SVDB_NORM_LU) {
-        k_b_colnorm<T><<<dim3((unsigned)B.l, (unsigned)B.count), 256, 0, B.s>>>(X, L, B.coff.p, (int)B.l);
+        k_b_colnorm<T><<<dim3((unsigned)B.l, (unsigned)B.count), 256, 0, B.s>>>(X, L, B.coff.p, B.ld);
         SVDB_CHECK_LAUNCH();
     }
 }
@@ -837,7 +1017,7 @@ static void enqueue(svdb_batch& B) {
     const int c = (int)B.l;
     SVDB_CUDA(cudaMemsetAsync(B.flags.p, 0, B.count * sizeof(int), B.s));
     SVDB_CUDA(cudaMemsetAsync(B.jstat.p, 0, B.count * sizeof(int), B.s));
-    k_b_omega<T><<<dim3(64, (unsigned)B.count), 256, 0, B.s>>>(B.seed, B.coff.p, c, Om);
+    k_b_omega<T><<<dim3(64, (unsigned)B.count), 256, 0, B.s>>>(B.seed, B.coff.p, c, B.ld, Om);
     SVDB_CHECK_LAUNCH();
     rows_product<T>(B, Om, Y, B.gs);
     for (int64_t it = 0; it < B.q; ++it) {
@@ -855,8 +1035,8 @@ static void enqueue(svdb_batch& B) {
     k_b_jacobi<<<(unsigned)B.count, jacobi_threads(c, 512), smem, B.s>>>(B.Rout.p, c, B.Ur.p, B.Vr.p, B.sig.p, B.jstat.p);
     SVDB_CHECK_LAUNCH();
     // U_b = Q_b V_J[:, :rank] (m x rank);  V_b^T = (Q_Bt U_J[:, :rank])^T (rank x nb)
-    right_mul<T, double, false>(B, Y, LY, B.Vr.p, c, (int)B.rank, B.U.p, nullptr);
-    right_mul<double, double, true>(B, B.Bt.p, LZ, B.Ur.p, c, (int)B.rank, B.Vt.p, nullptr);
+    right_mul<T, double>(B, Y, LY, B.Vr.p, false, (int)B.rank, B.U.p, (int)B.rank, false, nullptr);
+    right_mul<double, double>(B, B.Bt.p, LZ, B.Ur.p, false, (int)B.rank, B.Vt.p, 0, true, nullptr);
 }
 
 static void enqueue_any(svdb_batch& B) {
@@ -883,6 +1063,7 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
     B->on_device = o.result_on_device != 0;
     B->use_graph = o.use_graph != 0;
     B->m = m; B->n = n; B->count = (int64_t)count; B->rank = (int64_t)target_rank; B->l = l; B->q = (int64_t)q;
+    B->ld = (int)(B->mixed ? l : (l + 1) / 2 * 2);
     B->normalizer = normalizer;
     B->seed = has_seed ? seed : 0;
     // with_columns per subset: ascending, duplicates dropped, bounds checked (masked.rs:48-55)
@@ -932,14 +1113,18 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
             B->dsplit = ds;
         }
     }
-    const int64_t tc = B->total_cols;
+    const int64_t tc = B->total_cols, ld = B->ld;
     if (B->mixed) {
-        B->Om32.alloc(tc * l, s); B->Y32.alloc(count * m * l, s); B->Z32.alloc(tc * l, s);
+        B->Om32.alloc(tc * ld, s); B->Y32.alloc(count * m * ld, s); B->Z32.alloc(tc * ld, s);
     } else {
-        B->Om64.alloc(tc * l, s); B->Y64.alloc(count * m * l, s); B->Z64.alloc(tc * l, s);
+        B->Om64.alloc(tc * ld, s); B->Y64.alloc(count * m * ld, s); B->Z64.alloc(tc * ld, s);
     }
-    B->Bt.alloc(tc * l, s);
-    B->part.alloc(count * kGramChunks * l * l, s);
+    B->Bt.alloc(tc * ld, s);
+    // one CTA per SM over all subsets (four waves of short ones took 59 us, one
+    // 54, in the mixed solve of 16 subsets of 20,000 x 6,000), none of them below 256 rows
+    B->gram_parts = (int)std::max<int64_t>(
+        1, std::min<int64_t>((int64_t)device_props().sms / (int64_t)count, (m + 255) / 256));
+    B->part.alloc(count * B->gram_parts * l * l, s);
     for (DevBuf<double>* p : {&B->G, &B->R1, &B->R2, &B->R3, &B->Ri, &B->Rout, &B->Rtmp, &B->Ur, &B->Vr})
         p->alloc(count * l * l, s);
     B->sig.alloc(count * l, s);
@@ -969,7 +1154,7 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
         auto it = g_tuned.find(key);
         if (it != g_tuned.end()) { gs = it->second; cached = true; }
     }
-    // the lean row kernel (SVDB_MIXED) takes one subset per item: nothing to tune
+    // the lean row kernels take one subset per item: nothing to tune
     if (!cached && lean_batch(*B, n)) {
         gs = 1;
         cached = true;
@@ -985,12 +1170,12 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
             float ms = 0.f;
             auto run = [&]() {
                 if (B->mixed) {
-                    k_b_omega<float><<<dim3(64, (unsigned)count), 256, 0, s>>>(B->seed, B->coff.p, (int)l, B->Om32.p);
+                    k_b_omega<float><<<dim3(64, (unsigned)count), 256, 0, s>>>(B->seed, B->coff.p, (int)l, B->ld, B->Om32.p);
                     SVDB_CHECK_LAUNCH();
                     SVDB_CUDA(cudaEventRecord(e0, s));
                     rows_product<float>(*B, B->Om32.p, B->Y32.p, cand);
                 } else {
-                    k_b_omega<double><<<dim3(64, (unsigned)count), 256, 0, s>>>(B->seed, B->coff.p, (int)l, B->Om64.p);
+                    k_b_omega<double><<<dim3(64, (unsigned)count), 256, 0, s>>>(B->seed, B->coff.p, (int)l, B->ld, B->Om64.p);
                     SVDB_CHECK_LAUNCH();
                     SVDB_CUDA(cudaEventRecord(e0, s));
                     rows_product<double>(*B, B->Om64.p, B->Y64.p, cand);

@@ -91,36 +91,49 @@ __device__ __forceinline__ void tn_part_body(const TX* __restrict__ X, int64_t l
     for (int i = 0; i < NT; ++i)
 #pragma unroll
         for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    double a[NT], b[NT];
-    auto load = [&](int64_t r, double (&fa)[NT], double (&fb)[NT]) {
-        const bool rok = r + kl < r1;
-        const TX* px = X + (r + kl) * ldx + ca;
-        const TY* py = Y + (r + kl) * ldy + cb;
+    // KS groups of four rows per step; the next step's loads are in flight during
+    // this one's products (NT = 4: the accumulators leave registers for one group)
+    constexpr int KS = NT <= 3 ? 2 : 1;
+    TX a[KS][NT];  // converted when used: a conversion beside its load would wait for it
+    TY b[KS][NT];
+    auto load = [&](int64_t r, TX (&fa)[KS][NT], TY (&fb)[KS][NT]) {
 #pragma unroll
-        for (int t = 0; t < NT; ++t) fa[t] = (rok && ca + 8 * t < p) ? (double)px[8 * t] : 0.0;
-        if (!diag) {
+        for (int k = 0; k < KS; ++k) {
+            const int64_t row = r + (int64_t)k * 4 * rg + kl;
+            const bool rok = row < r1;
+            const TX* px = X + row * ldx + ca;
+            const TY* py = Y + row * ldy + cb;
 #pragma unroll
-            for (int t = 0; t < NT; ++t) fb[t] = (rok && cb + 8 * t < q) ? (double)py[8 * t] : 0.0;
+            for (int t = 0; t < NT; ++t) fa[k][t] = (rok && ca + 8 * t < p) ? px[8 * t] : TX(0);
+            if (!diag) {
+#pragma unroll
+                for (int t = 0; t < NT; ++t) fb[k][t] = (rok && cb + 8 * t < q) ? py[8 * t] : TY(0);
+            }
         }
     };
     int64_t r = r0 + 4 * g;
     if (r < r1) load(r, a, b);
-    for (; r < r1; r += 4 * rg) {
-        double na[NT], nb[NT];
-        if (r + 4 * rg < r1) load(r + 4 * rg, na, nb);  // in flight during the products of this group
-        if (diag) {
+    for (; r < r1; r += (int64_t)KS * 4 * rg) {
+        TX na[KS][NT];
+        TY nb[KS][NT];
+        if (r + (int64_t)KS * 4 * rg < r1) load(r + (int64_t)KS * 4 * rg, na, nb);
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            double da[NT], db[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                da[t] = (double)a[k][t];
+                db[t] = diag ? da[t] : (double)b[k][t];
+            }
 #pragma unroll
             for (int i = 0; i < NT; ++i)
 #pragma unroll
-                for (int j = 0; j < NT; ++j) dmma(acc[i][j], a[i], a[j]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < NT; ++i)
-#pragma unroll
-                for (int j = 0; j < NT; ++j) dmma(acc[i][j], a[i], b[j]);
+                for (int j = 0; j < NT; ++j) dmma(acc[i][j], da[i], db[j]);
         }
 #pragma unroll
-        for (int t = 0; t < NT; ++t) { a[t] = na[t]; b[t] = nb[t]; }
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) { a[k][t] = na[k][t]; b[k][t] = nb[k][t]; }
     }
     constexpr int W = NT * 8;
     double* mine = sm + (size_t)warp * W * W;
@@ -271,6 +284,18 @@ __device__ __forceinline__ void nn_body(const NnArgs<TX, TO>& A, int64_t g0, int
         for (int n = 0; n < NQ; ++n) dacc[n][0] = dacc[n][1] = 0.0;
     }
     const int nk = p4 / 4;
+    TX a[kNnKU][kNnMT];
+    auto load = [&](int64_t grp, int k0, TX (&f)[kNnKU][kNnMT]) {
+#pragma unroll
+        for (int u = 0; u < kNnKU; ++u)
+#pragma unroll
+            for (int i = 0; i < kNnMT; ++i) {
+                const int64_t row = (grp * kNnMT + i) * 8 + il;
+                const int col = 4 * (k0 + u) + kl;
+                f[u][i] = (row < A.rows && col < A.p) ? A.X[row * A.ldx + col] : TX(0);
+            }
+    };
+    load(g0, 0, a);
     for (int64_t g = g0; g * (8 * kNnMT) < A.rows; g += gstep) {
         const int64_t row0 = g * (8 * kNnMT);
         double acc[kNnMT][NQ][2];
@@ -278,21 +303,10 @@ __device__ __forceinline__ void nn_body(const NnArgs<TX, TO>& A, int64_t g0, int
         for (int i = 0; i < kNnMT; ++i)
 #pragma unroll
             for (int n = 0; n < NQ; ++n) acc[i][n][0] = acc[i][n][1] = 0.0;
-        double a[kNnKU][kNnMT];
-        auto load = [&](int k0, double (&f)[kNnKU][kNnMT]) {
-#pragma unroll
-            for (int u = 0; u < kNnKU; ++u)
-#pragma unroll
-                for (int i = 0; i < kNnMT; ++i) {
-                    const int64_t row = row0 + 8 * i + il;
-                    const int col = 4 * (k0 + u) + kl;
-                    f[u][i] = (row < A.rows && col < A.p) ? (double)A.X[row * A.ldx + col] : 0.0;
-                }
-        };
-        load(0, a);
         for (int k0 = 0; k0 < nk; k0 += kNnKU) {
-            double na[kNnKU][kNnMT];
-            if (k0 + kNnKU < nk) load(k0 + kNnKU, na);
+            TX na[kNnKU][kNnMT];  // in flight meanwhile: this group's next k-steps, or the next group's first
+            if (k0 + kNnKU < nk) load(g, k0 + kNnKU, na);
+            else load(g + gstep, 0, na);
 #pragma unroll
             for (int u = 0; u < kNnKU; ++u) {
                 if (k0 + u >= nk) break;
@@ -303,7 +317,7 @@ __device__ __forceinline__ void nn_body(const NnArgs<TX, TO>& A, int64_t g0, int
                     if (n < nlow) continue;
                     const double bf = cr[8 * n];
 #pragma unroll
-                    for (int i = 0; i < kNnMT; ++i) dmma(acc[i][n], a[u][i], bf);
+                    for (int i = 0; i < kNnMT; ++i) dmma(acc[i][n], (double)a[u][i], bf);
                 }
             }
 #pragma unroll

@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "device_common.cuh"
+#include "lean.cuh"
 #include "ops.cuh"
 #include "svdb_internal.h"
 
@@ -77,11 +78,6 @@ __device__ __forceinline__ void store_cols(T* __restrict__ p, int ncols_here, co
 // used.  The (index, value) pairs of the next 32 entries are loaded while the
 // current ones are consumed.  With FP32 operands the products of one 32-entry
 // chunk are summed in FP32 and the chunk sum is added to an FP64 accumulator.
-template <typename T>
-struct AccOf { using type = double; };
-template <>
-struct AccOf<float> { using type = float; };
-
 template <typename VT, typename XT, typename OT, int CPL, int H, int U>
 __global__ void __launch_bounds__(256, sizeof(XT) == 4 ? 4 : 3) k_spmm_seg(const int32_t* __restrict__ ci, const VT* __restrict__ val,
                                                      const int32_t* __restrict__ seg_row,
@@ -194,23 +190,6 @@ __global__ void __launch_bounds__(256, sizeof(XT) == 4 ? 4 : 3) k_spmm_seg(const
 // CTA's warps starting together, which raised the L1 hits from 7 to 26 % and
 // gained 3 % on long rows but lost 10 % on A^T X.
 constexpr int kLeanWarps = 8;
-template <typename T>
-struct LeanVec;
-template <>
-struct alignas(16) LeanVec<float> { float v[4]; };
-template <>
-struct alignas(16) LeanVec<double> { double v[2]; };
-template <typename T>
-__device__ __forceinline__ void lean_values4(const T* p, T (&v)[4]) {  // four consecutive shared values
-    constexpr int VEC = 16 / (int)sizeof(T);
-#pragma unroll
-    for (int i = 0; i < 4 / VEC; ++i) {
-        const LeanVec<T> t = reinterpret_cast<const LeanVec<T>*>(p)[i];
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) v[i * VEC + e] = t.v[e];
-    }
-}
-
 template <typename T, typename OT, int H, int NL, int U, int MINB, bool BYTES>
 __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
     k_spmm_lean(const int32_t* __restrict__ ci, const T* __restrict__ val, const int32_t* __restrict__ seg_row,
@@ -220,11 +199,9 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
     using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
     constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int GL = 32 / H;   // lanes per group
-    constexpr int PER = 32 / H;  // entries of a chunk per group
-    constexpr int VS = PER + (sizeof(T) == 8 && H > 1 ? 2 : 0);  // a group's values, off the others' banks
-    static_assert(U % 4 == 0 && U <= PER, "batches of whole quads");
+    using Slots = LeanSlots<T, H>;
     __shared__ __align__(16) uint32_t s_off[kLeanWarps][32];
-    __shared__ __align__(16) T s_val[kLeanWarps][H * VS];
+    __shared__ __align__(16) T s_val[kLeanWarps][H * Slots::VS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int g = lane / GL, gl = lane % GL;
     bool active[NL];
@@ -236,17 +213,10 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
         col[j] = active[j] ? (uint32_t)c : 0u;
     }
     const uint32_t scale = BYTES ? ldx * (uint32_t)sizeof(T) : ldx;
-    uint32_t* const oput = s_off[w] + (lane % H) * PER + lane / H;
-    T* const vput = s_val[w] + (lane % H) * VS + lane / H;
-    const uint32_t* const og = s_off[w] + g * PER;
-    const T* const vg = s_val[w] + g * VS;
-    auto gather = [&](uint32_t off, int j) {
-        if constexpr (BYTES)
-            return *reinterpret_cast<const LeanVec<T>*>(reinterpret_cast<const char*>(X) +
-                                                        (off + col[j] * (uint32_t)sizeof(T)));
-        else
-            return *reinterpret_cast<const LeanVec<T>*>(X + (off + col[j]));
-    };
+    uint32_t* const oput = s_off[w] + Slots::off(lane);
+    T* const vput = s_val[w] + Slots::val(lane);
+    const uint32_t* const og = s_off[w] + g * Slots::PER;
+    const T* const vg = s_val[w] + g * Slots::VS;
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t sg = gwarp; sg < nseg; sg += nwarps) {
@@ -276,59 +246,7 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
             for (int j = 0; j < NL; ++j)
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
-            if (left >= 32) {
-#pragma unroll 1
-                for (int qb = 0; qb < PER; qb += U) {  // one batch live at a time
-                    LeanVec<T> xv[U][NL];
-                    T vv[U];
-#pragma unroll
-                    for (int q = 0; q < U; q += 4) {
-                        const uint4 o = *reinterpret_cast<const uint4*>(og + qb + q);
-                        T v4[4];
-                        lean_values4(vg + qb + q, v4);
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            vv[q + u] = v4[u];
-                            const uint32_t off = u == 0 ? o.x : u == 1 ? o.y : u == 2 ? o.z : o.w;
-#pragma unroll
-                            for (int j = 0; j < NL; ++j) {
-                                if (active[j]) xv[q + u][j] = gather(off, j);
-                                else xv[q + u][j] = LeanVec<T>{};
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-#pragma unroll
-                        for (int j = 0; j < NL; ++j)
-#pragma unroll
-                            for (int e = 0; e < VEC; ++e) cs[j][e] = fma((CT)vv[u], (CT)xv[u][j].v[e], cs[j][e]);
-                }
-            } else {
-                const int mine = (left - g + H - 1) / H;  // entries of this group
-#pragma unroll 1
-                for (int qb = 0; qb * H < left; qb += 4) {
-                    LeanVec<T> xv[4][NL];
-                    T vv[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const bool ok = qb + u < mine;
-                        vv[u] = ok ? vg[qb + u] : T(0);
-                        const uint32_t off = og[qb + u];
-#pragma unroll
-                        for (int j = 0; j < NL; ++j) {
-                            if (ok && active[j]) xv[u][j] = gather(off, j);
-                            else xv[u][j] = LeanVec<T>{};
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int j = 0; j < NL; ++j)
-#pragma unroll
-                            for (int e = 0; e < VEC; ++e) cs[j][e] = fma((CT)vv[u], (CT)xv[u][j].v[e], cs[j][e]);
-                }
-            }
+            lean_chunk<T, H, NL, U, BYTES>(og, vg, left, g, X, col, active, cs);
 #pragma unroll
             for (int j = 0; j < NL; ++j)
 #pragma unroll
