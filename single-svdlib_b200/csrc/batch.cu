@@ -584,18 +584,22 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, NL == 3 ? 2 : 3)
 
 // --------------------------------------------------------- CholeskyQR2 ----
 // Gram partials: block (chunk, b) sums X_b^T X_b over its rows on the FP64
-// matrix instruction (dense_tall.cuh), the tile blocks I <= J only.  16
-// subsets, l = 40, the 20,000-row and the about 2,250-row operands of a mixed
-// solve: 32 us on average, against 129 for register tiles staged through
-// shared memory.
+// matrix instruction (dense_tall.cuh), the tile blocks I <= J only.  At FP32
+// the chunks are sixteenths of the rows, each summed in row order by one warp
+// per tile block (rg = 1, small blocks, so that there are enough warps), and
+// the sixteen are added in one order whatever the batch: X R^-1 is rounded to
+// FP32, where a Gram that depended on the number of subsets in its last bit
+// would change a subset's results with its company.  16 subsets, l = 40, the
+// 20,000-row and the about 2,250-row operands of a mixed solve: 70 us on
+// average, against 129 for register tiles staged through shared memory.
 template <typename T, int NT>
-__global__ void __launch_bounds__(512, 1) k_b_gram_part(const T* __restrict__ X, SubLayout L,
+__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_b_gram_part(const T* __restrict__ X, SubLayout L,
                                                         const int64_t* __restrict__ coff, int c, int ld, int nb, int rg,
                                                         double* __restrict__ part, const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
     extern __shared__ double bg_sm[];
-    const int64_t rows = sub_rows(L, coff, b), step = 4 * rg;
+    const int64_t rows = sub_rows(L, coff, b), step = rg > 1 ? 4 * rg : 1;
     const int64_t chunk = ((rows + gridDim.x - 1) / gridDim.x + step - 1) / step * step;
     const int64_t r0 = blockIdx.x * chunk;
     const T* xb = X + sub_row0(L, coff, b) * ld;
@@ -605,6 +609,24 @@ __global__ void __launch_bounds__(512, 1) k_b_gram_part(const T* __restrict__ X,
 
 // G_b = sum of the subset's partials in chunk order (elements of tile blocks
 // below the diagonal are not read by the factorisation and stay undefined)
+constexpr int kGramChunks = 16;  // of a mixed batch
+__global__ void k_b_gram_reduce16(const double* __restrict__ part, int c, double* __restrict__ G,
+                                  const int* __restrict__ cond) {
+    const int64_t b = blockIdx.y;
+    if (cond && cond[b] == 0) return;
+    const int cc = c * c;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < cc; p += gridDim.x * blockDim.x) {
+        double v[kGramChunks], s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < kGramChunks; ++k) v[k] = part[(b * kGramChunks + k) * cc + p];
+#pragma unroll
+        for (int k = 0; k < kGramChunks; k += 2) {
+            s0 += v[k];
+            s1 += v[k + 1];
+        }
+        G[b * cc + p] = s0 + s1;
+    }
+}
 __global__ void __launch_bounds__(256) k_b_gram_reduce(const double* __restrict__ part, int nchunk, int c,
                                                        double* __restrict__ G, const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
@@ -628,7 +650,7 @@ __global__ void __launch_bounds__(256) k_b_gram_reduce(const double* __restrict_
     }
 }
 
-__global__ void __launch_bounds__(256) k_b_chol_inv(const double* __restrict__ G, int nparts, int c, SubLayout L, const int64_t* __restrict__ coff,
+__global__ void __launch_bounds__(384) k_b_chol_inv(const double* __restrict__ G, int nparts, int c, SubLayout L, const int64_t* __restrict__ coff,
                              double* __restrict__ R, double* __restrict__ Ri, int* __restrict__ flags,
                              int* __restrict__ shifted, const int* __restrict__ cond) {
     const int64_t b = blockIdx.x;
@@ -907,18 +929,33 @@ constexpr int64_t kBCholParts = 16384;
 template <typename T>
 static const double* gram(svdb_batch& B, const T* X, SubLayout L, const int* cond, int& parts) {
     const int c = (int)B.l;
-    const TnShape h = tn_shape(1, c, c, true, 1);  // the tiles; the chunks are the kernel's own
-    const dim3 grid(B.gram_parts, (unsigned)B.count);
+    constexpr bool f32 = std::is_same<T, float>::value;
+    TnShape h = tn_shape(1, c, c, true, 1);  // the tiles; the chunks are the kernel's own
+    if (f32) {  // 2 x 2 fragments per warp
+        h.nt = 2;
+        h.nbp = h.nbq = ((c + 7) / 8 + 1) / 2;
+        h.ntb = h.nbp * (h.nbp + 1) / 2;
+        h.rg = 1;
+    }
+    const dim3 grid(f32 ? kGramChunks : B.gram_parts, (unsigned)B.count);
     auto go = [&](auto kern) {
         if (h.smem() > 48 * 1024)
             SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem()));
         kern<<<grid, h.threads(), h.smem(), B.s>>>(X, L, B.coff.p, c, B.ld, h.nbp, h.rg, B.part.p, cond);
     };
-    switch (h.nt) {
-        case 1: go(k_b_gram_part<T, 1>); break;
-        case 2: go(k_b_gram_part<T, 2>); break;
-        case 3: go(k_b_gram_part<T, 3>); break;
-        default: go(k_b_gram_part<T, 4>); break;
+    if constexpr (f32) {
+        go(k_b_gram_part<float, 2>);
+        k_b_gram_reduce16<<<dim3((c * c + 127) / 128, (unsigned)B.count), 128, 0, B.s>>>(B.part.p, c, B.G.p, cond);
+        SVDB_CHECK_LAUNCH_N(2);
+        parts = 0;
+        return B.G.p;
+    } else {
+        switch (h.nt) {
+            case 1: go(k_b_gram_part<double, 1>); break;
+            case 2: go(k_b_gram_part<double, 2>); break;
+            case 3: go(k_b_gram_part<double, 3>); break;
+            default: go(k_b_gram_part<double, 4>); break;
+        }
     }
     SVDB_CHECK_LAUNCH();
     parts = (int64_t)B.gram_parts * c * c <= kBCholParts ? B.gram_parts : 0;
@@ -967,7 +1004,7 @@ static void chol(svdb_batch& B, SubLayout L, const double* G, int parts, double*
     // chol_inv_body also holds some static shared memory
     if (smem > 40 * 1024)
         SVDB_CUDA(cudaFuncSetAttribute(k_b_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_b_chol_inv<<<(unsigned)B.count, 256, smem, B.s>>>(G, parts, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,
+    k_b_chol_inv<<<(unsigned)B.count, 384, smem, B.s>>>(G, parts, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,
                                                          cond);
     SVDB_CHECK_LAUNCH();
 }
@@ -1124,7 +1161,7 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
     // 54, in the mixed solve of 16 subsets of 20,000 x 6,000), none of them below 256 rows
     B->gram_parts = (int)std::max<int64_t>(
         1, std::min<int64_t>((int64_t)device_props().sms / (int64_t)count, (m + 255) / 256));
-    B->part.alloc(count * B->gram_parts * l * l, s);
+    B->part.alloc(count * std::max(B->gram_parts, B->mixed ? kGramChunks : 1) * l * l, s);
     for (DevBuf<double>* p : {&B->G, &B->R1, &B->R2, &B->R3, &B->Ri, &B->Rout, &B->Rtmp, &B->Ur, &B->Vr})
         p->alloc(count * l * l, s);
     B->sig.alloc(count * l, s);

@@ -36,17 +36,27 @@ __device__ __forceinline__ double omega_value(uint64_t key, int64_t i) {
 //   - every warp that owns columns factors the 8 x 8 diagonal block in
 //     registers (redundantly: no broadcast, no barrier) and eliminates one
 //     column per thread;
-//   - the trailing tiles are updated with the FP64 matrix instruction.
-// What bounds it is the chain of c pivots (a reciprocal square root and two
-// multiply-adds each, about 90 cycles) and two barriers per eight of them.  The
-// form before it (a barrier and a division per pivot, then a forward
-// substitution per row of R^-1) took 70 us at c = 60, 36 at 40 and 15 at 20;
-// this one 22, 13 and 11 (ncu, cold caches).
+//   - the trailing tiles of G are updated by FMAs, those of R^-T by the FP64
+//     matrix instruction.
+// What bounds it is the chain of c pivots (a division, a multiplication and a
+// multiply-add each, about 135 cycles) and two barriers per eight of them.  A
+// barrier per pivot, then a forward substitution per row of R^-1, took 70 us
+// at c = 60, 36 at 40 and 15 at 20; this form, with twelve warps, 24, 15 and
+// 11 (ncu, cold caches; eight warps 29, 17 and 13: the FMA tiles' latency).
+//
+// Every element sees one fixed sequence of operations, whatever the panels:
+//   a_ij = fma(-(a_ki a_kj), 1 / a_kk, a_ij), k ascending, unscaled rows;
+//   R_kj = a_kj (1 / sqrt(a_kk)), R_kk = sqrt(a_kk);
+//   y_e = fma(-y_k, R_ke, y_e), k ascending, then y_e (1 / R_ee)   (R^-1 = y^T)
+// (m8n8k4.f64 is the same ascending chain of FMAs).  Mixed batches store
+// X R^-1 in FP32, so a factor that differed in its last FP64 bit would now and
+// then flip an FP32 rounding; this keeps their results reproducible.
 //
 // Layout: rows of 8 x 8 tiles, row tile I: tiles 0 .. I hold R^-T (I, 0 .. I)
-// (the identity before panel I), tiles I + 1 .. nt hold G / R (I, I .. nt - 1);
-// padded to whole tiles with the identity.  The factored diagonal tiles go to
-// their own buffer, since other warps may still be reading the unfactored one.
+// (the identity before panel I), tiles I + 1 .. nt hold G's unscaled rows
+// (I, I .. nt - 1); padded to whole tiles with the identity.  The factored
+// diagonal tiles go to a buffer of their own, since other warps may still be
+// reading the unfactored one.
 //
 // A pivot that is not positive and finite restarts the factorisation on
 // G + shift I with shift = shift_scale * trace(G) (shifted CholeskyQR); that
@@ -58,15 +68,17 @@ __device__ __forceinline__ double omega_value(uint64_t key, int64_t i) {
 __host__ __device__ inline int chol_ld(int c) { return ((c + 7) / 8 + 1) * 8 + 4; }  // = 4 or 12 mod 16: no conflicts
 __host__ __device__ inline size_t chol_smem(int c) {
     const int nt = (c + 7) / 8;
-    return ((size_t)nt * 8 * chol_ld(c) + (size_t)nt * 64) * sizeof(double);
+    return ((size_t)(nt + 1) * 8 * chol_ld(c) + (size_t)nt * (64 + 8)) * sizeof(double);
 }
 __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int nparts, int c, double shift_scale,
                                               double* __restrict__ R, double* __restrict__ Ri,
                                               int* __restrict__ flags, int* __restrict__ shifted, double* sm) {
     __shared__ int s_fail;
-    __shared__ double s_red[32];
+    __shared__ double s_inv[8], s_shift;
     const int nt = (c + 7) / 8, c8 = nt * 8, ld = chol_ld(c), cc = c * c;
-    double* const dg = sm + (size_t)c8 * ld;
+    double* const rp = sm + (size_t)c8 * ld;  // the panel's rows of R (8 x ld)
+    double* const dg = rp + 8 * ld;           // the factored diagonal tiles, unscaled
+    double* const rs = dg + nt * 64;          // 1 / sqrt of the pivots
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (blockDim.x < 160 || c > 128) {  // one thread per column of the widest row
         if (threadIdx.x == 0) atomicOr(flags, 2);
@@ -96,7 +108,7 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
         bool failed = false;
         for (int K = 0; K < nt; ++K) {
             if (warp * 32 < c8 + 8) {
-                double d[8][8], r[8];
+                double d[8][8], inv[8];
                 const double* blk = sm + 8 * K * ld + 8 * (K + 1);
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
@@ -106,33 +118,58 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     ok = ok && d[k][k] > 0.0 && isfinite(d[k][k]);
-                    r[k] = rsqrt(d[k][k]);
-#pragma unroll
-                    for (int i = k; i < 8; ++i) d[k][i] *= r[k];
+                    inv[k] = 1.0 / d[k][k];
 #pragma unroll
                     for (int i = k + 1; i < 8; ++i)
 #pragma unroll
-                        for (int j = i; j < 8; ++j) d[i][j] = fma(-d[k][i], d[k][j], d[i][j]);
+                        for (int j = i; j < 8; ++j) d[i][j] = fma(-(d[k][i] * d[k][j]), inv[k], d[i][j]);
                 }
                 if (!ok && lane == 0) s_fail = 1;
+                // 1 / sqrt and 1 / R_kk = 1 / (sqrt) of pivot k in lane k, read from there: once per
+                // warp, off the chain of the factorisation
+                double piv = d[0][0];
+#pragma unroll
+                for (int k = 1; k < 8; ++k)
+                    if (lane == k) piv = d[k][k];
+                const double rq = 1.0 / sqrt(piv);
+                if (warp == 0 && lane < 8) {
+                    s_inv[lane] = 1.0 / piv;
+                    rs[8 * K + lane] = rq;
+                }
                 const int j = threadIdx.x, tile = j >> 3;
+                double a[8];
                 if (j < c8 + 8) {
-                    double a[8];
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         a[k] = tile == K ? ((j & 7) == k ? 1.0 : 0.0) : sm[(8 * K + k) * ld + j];
+                    if (tile > K) {  // a column of G
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        a[k] *= r[k];
+                        for (int k = 0; k < 8; ++k)
 #pragma unroll
-                        for (int i = k + 1; i < 8; ++i) a[i] = fma(-d[k][i], a[k], a[i]);
+                            for (int i = k + 1; i < 8; ++i) a[i] = fma(-(d[k][i] * a[k]), inv[k], a[i]);
                     }
-                    if (tile == K + 1) {
+                }
+                double r[8];
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) dg[(8 * K + k) * 8 + (j & 7)] = (j & 7) < k ? 0.0 : a[k];
+                for (int k = 0; k < 8; ++k) r[k] = __shfl_sync(0xffffffffu, rq, k);
+                if (j < c8 + 8) {
+                    if (tile <= K) {  // a column of R^-T
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            a[k] *= r[k];
+#pragma unroll
+                            for (int i = k + 1; i < 8; ++i) a[i] = fma(-a[k], d[k][i] * r[k], a[i]);
+                            sm[(8 * K + k) * ld + j] = a[k];
+                        }
+                    } else if (tile == K + 1) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) dg[(8 * K + k) * 8 + (j & 7)] = a[k];
                     } else {
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) sm[(8 * K + k) * ld + j] = a[k];
+                        for (int k = 0; k < 8; ++k) {
+                            sm[(8 * K + k) * ld + j] = a[k];
+                            rp[k * ld + j] = a[k] * r[k];
+                        }
                     }
                 }
             }
@@ -143,28 +180,41 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
             }
             // row tiles I > K: tiles 0 .. K of R^-T and I .. nt - 1 of G
             const int kl = lane & 3, il = lane >> 2;
-            const double* pk = sm + (8 * K + kl) * ld + il;
-            for (int q = warp; q < (nt - 1 - K) * (nt + 1); q += nw) {
-                const int I = K + 1 + q / (nt + 1), t = q % (nt + 1);
+            for (int qq = warp; qq < (nt - 1 - K) * (nt + 1); qq += nw) {
+                const int I = K + 1 + qq / (nt + 1), t = qq % (nt + 1);
                 if (t > K && t <= I) continue;
                 double* cp = sm + (8 * I + il) * ld + 8 * t + 2 * kl;
                 double acc[2] = {cp[0], cp[1]};
-                dmma(acc, -pk[8 * (I + 1)], pk[8 * t]);
-                dmma(acc, -pk[4 * ld + 8 * (I + 1)], pk[4 * ld + 8 * t]);
+                if (t <= K) {
+                    const double* pa = rp + kl * ld + 8 * (I + 1) + il;
+                    const double* pb = sm + (8 * K + kl) * ld + 8 * t + il;
+                    dmma(acc, -pa[0], pb[0]);
+                    dmma(acc, -pa[4 * ld], pb[4 * ld]);
+                } else {
+                    const double* pa = sm + 8 * K * ld + 8 * (I + 1) + il;
+                    const double* pb = sm + 8 * K * ld + 8 * t + 2 * kl;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const double x = pa[k * ld];
+                        acc[0] = fma(-(x * pb[k * ld]), s_inv[k], acc[0]);
+                        acc[1] = fma(-(x * pb[k * ld + 1]), s_inv[k], acc[1]);
+                    }
+                }
                 cp[0] = acc[0];
                 cp[1] = acc[1];
             }
             __syncthreads();
         }
         if (!failed || attempt == 1) break;
-        double tr = 0.0;
-        for (int i = threadIdx.x; i < c; i += blockDim.x) tr += g_at(i, i);
-        shift = shift_scale * block_sum(tr, s_red);  // also orders this attempt's reads before the next one's writes
-        if (!(shift > 0.0)) shift = 1e-300;
         if (threadIdx.x == 0) {
+            double tr = 0.0;
+            for (int i = 0; i < c; ++i) tr += g_at(i, i);
+            s_shift = shift_scale * tr > 0.0 ? shift_scale * tr : 1e-300;
             atomicOr(flags, 1);
             *shifted = 1;
         }
+        __syncthreads();  // also orders this attempt's reads before the next one's writes
+        shift = s_shift;
     }
     if (s_fail) {
         if (threadIdx.x == 0) atomicOr(flags, 2);
@@ -173,7 +223,8 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
     }
     for (int i = warp; i < c; i += nw)
         for (int j = lane; j < c; j += 32) {
-            R[i * c + j] = (j >> 3) == (i >> 3) ? dg[i * 8 + (j & 7)] : j > i ? sm[i * ld + 8 + j] : 0.0;
+            const double v = (j >> 3) == (i >> 3) ? dg[i * 8 + (j & 7)] : sm[i * ld + 8 + j];
+            R[i * c + j] = j > i ? v * rs[i] : j == i ? sqrt(v) : 0.0;
             Ri[i * c + j] = j >= i ? sm[j * ld + i] : 0.0;
         }
 }

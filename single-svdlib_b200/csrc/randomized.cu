@@ -44,7 +44,7 @@ __global__ void k_omega(uint64_t seed, int64_t total, T* __restrict__ out) {
 // ------------------------------------------------------ small dense ops ----
 // Every kernel of a CholeskyQR pass takes `cond`: when it points to 0 the
 // kernel returns at once (the conditional third pass of shifted CholeskyQR).
-__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int nparts, int c, double shift_scale,
+__global__ void __launch_bounds__(384) k_chol_inv(const double* __restrict__ G, int nparts, int c, double shift_scale,
                                                   double* __restrict__ R, double* __restrict__ Ri,
                                                   int* __restrict__ flags, int* __restrict__ shifted,
                                                   const int* __restrict__ cond) {
@@ -263,7 +263,7 @@ static void chol_inv(RandCtx& cx, const double* G, int parts, int c, int64_t row
         SVDB_CUDA(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // shifted CholeskyQR: shift = 11 (rows c + c (c + 1)) u ||X||_F^2, ||X||_F^2 = trace(G)
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
-    k_chol_inv<<<1, 256, smem, cx.s>>>(G, parts, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond);
+    k_chol_inv<<<1, 384, smem, cx.s>>>(G, parts, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond);
     SVDB_CHECK_LAUNCH();
 }
 
