@@ -9,6 +9,8 @@ constructed and keep a device handle for their lifetime.
 from __future__ import annotations
 
 import ctypes as C
+import threading
+import weakref
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -133,20 +135,56 @@ class SvdRec:
         return (self.u * self.s) @ self.vt
 
 
+# Result buffers of 64 KB and more are page-locked memory that the library
+# reuses (csrc/hostmem.cu).  An array takes its buffer over and hands it back
+# when the last view of it dies: copying 86 MB of results into fresh pages took
+# about 20 ms beside 4 ms of solving.  At most _LENT_MAX bytes are out at a
+# time (page-locked memory is scarce, and a caller that keeps every result
+# would have each call page-lock anew); past that, and for small results, the
+# values are copied and the buffer is released at once.
+_LENT_MIN, _LENT_MAX = 64 << 10, 512 << 20
+_lent = 0
+_lent_mu = threading.RLock()  # a finaliser may run inside the locked region
+
+
+def _give_back(addr, nbytes):
+    global _lent
+    r = _abi.svdb_rec()
+    r.u = C.cast(addr, C.POINTER(C.c_double))
+    _abi.lib().svdb_rec_free(C.byref(r))
+    with _lent_mu:
+        _lent -= nbytes
+
+
+def _take(r, name, count, shape, dtype):
+    """Array of the record's host buffer `name`; a lent buffer leaves the record."""
+    global _lent
+    if count == 0:
+        return np.zeros(shape, dtype=dtype)
+    ptr = getattr(r, name)
+    nbytes = count * np.dtype(dtype).itemsize
+    with _lent_mu:
+        lend = nbytes >= _LENT_MIN and _lent + nbytes <= _LENT_MAX
+        if lend:
+            _lent += nbytes
+    if not lend:
+        return np.ctypeslib.as_array(ptr, (count,)).copy().reshape(shape)
+    addr = C.cast(ptr, C.c_void_p).value
+    buf = (ptr._type_ * count).from_address(addr)
+    weakref.finalize(buf, _give_back, addr, nbytes).atexit = False  # the process's end frees it anyway
+    setattr(r, name, None)
+    return np.frombuffer(buf, dtype=dtype).reshape(shape)
+
+
 def rec_from_c(r) -> SvdRec:
     """SvdRec from an svdb_rec (T = f64) or an svdb_rec_f32 (T = f32, float32 arrays)."""
     d = int(r.d)
     ur, uc, vr, vc = int(r.u_rows), int(r.u_cols), int(r.vt_rows), int(r.vt_cols)
     dtype = np.float32 if isinstance(r, _abi.svdb_rec_f32) else np.float64
 
-    def arr(ptr, count, shape):
-        if count == 0:
-            return np.zeros(shape, dtype=dtype)
-        return np.ctypeslib.as_array(ptr, (count,)).copy().reshape(shape)
-
-    u = arr(r.u, ur * uc, (ur, uc))
-    s = arr(r.s, d, (d,))
-    vt = arr(r.vt, vr * vc, (vr, vc))
+    u = _take(r, "u", ur * uc, (ur, uc), dtype)
+    s = _take(r, "s", d, (d,), dtype)
+    vt = _take(r, "vt", vr * vc, (vr, vc), dtype)
     dg = r.diagnostics
     diag = Diagnostics(int(dg.non_zero), int(dg.dimensions), int(dg.iterations), bool(dg.transposed),
                        int(dg.lanczos_steps), int(dg.ritz_values_stabilized), int(dg.significant_values),
