@@ -939,8 +939,7 @@ static const double* gram(svdb_batch& B, const T* X, SubLayout L, const int* con
     }
     const dim3 grid(f32 ? kGramChunks : B.gram_parts, (unsigned)B.count);
     auto go = [&](auto kern) {
-        if (h.smem() > 48 * 1024)
-            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem()));
+        allow_smem(kern, tn_smem_max(h.nt));
         kern<<<grid, h.threads(), h.smem(), B.s>>>(X, L, B.coff.p, c, B.ld, h.nbp, h.rg, B.part.p, cond);
     };
     if constexpr (f32) {
@@ -980,8 +979,7 @@ static void right_mul(svdb_batch& B, const TI* X, SubLayout L, const double* S, 
     const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + tile - 1) / tile, per_subset)),
                     (unsigned)B.count);
     auto go = [&](auto kern) {
-        if (smem > 48 * 1024)
-            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_smem(kern, nn_smem(kBatchMaxL, nq));
         kern<<<grid, 32 * kNnWarps, smem, B.s>>>(X, L, B.coff.p, c, B.ld, S, cout, (int)upper, Out, ldo, (int)trans,
                                                  cond);
     };
@@ -1001,9 +999,7 @@ static void right_mul(svdb_batch& B, const TI* X, SubLayout L, const double* S, 
 static void chol(svdb_batch& B, SubLayout L, const double* G, int parts, double* R, const int* cond) {
     const int c = (int)B.l;
     const size_t smem = chol_smem(c);
-    // chol_inv_body also holds some static shared memory
-    if (smem > 40 * 1024)
-        SVDB_CUDA(cudaFuncSetAttribute(k_b_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_b_chol_inv, chol_smem(kBatchMaxL));
     k_b_chol_inv<<<(unsigned)B.count, 384, smem, B.s>>>(G, parts, c, L, B.coff.p, R, B.Ri.p, B.flags.p, B.shifted.p,
                                                          cond);
     SVDB_CHECK_LAUNCH();

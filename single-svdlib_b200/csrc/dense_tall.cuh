@@ -43,6 +43,7 @@ struct TnShape {
     int threads() const { return 32 * ntb * rg; }
     size_t smem() const { return (size_t)ntb * rg * nt * nt * 64 * sizeof(double); }
 };
+inline size_t tn_smem_max(int nt) { return (size_t)16 * nt * nt * 64 * sizeof(double); }  // sixteen warps
 // `ctas` CTAs at most.  One CTA of up to 16 warps per SM: 148 partials to add
 // instead of the 296 of two smaller CTAs.
 inline TnShape tn_shape(int64_t rows, int p, int q, bool sym, int ctas) {
@@ -206,11 +207,9 @@ static __global__ void __launch_bounds__(32 * kTnSlices) k_tn_reduce(const doubl
 template <typename TX, typename TY>
 inline void tn_launch(const TnShape& h, const TX* X, int64_t ldx, int p, const TY* Y, int64_t ldy, int q, int64_t rows,
                       double* part, double* C, const int* cond, cudaStream_t s) {
-    const size_t smem = h.smem();
     auto go = [&](auto kern) {
-        if (smem > 48 * 1024)
-            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<h.blocks, h.threads(), smem, s>>>(X, ldx, p, Y, ldy, q, rows, h.chunk, h.nbp, h.nbq, (int)h.sym, h.rg,
+        allow_smem(kern, tn_smem_max(h.nt));
+        kern<<<h.blocks, h.threads(), h.smem(), s>>>(X, ldx, p, Y, ldy, q, rows, h.chunk, h.nbp, h.nbq, (int)h.sym, h.rg,
                                                  part, cond);
     };
     switch (h.nt) {
@@ -407,8 +406,7 @@ inline void nn_launch(const NnArgs<TX, TO>& A, int sms, cudaStream_t s) {
     if (DOT) smem = std::max(smem, (size_t)kNnWarps * nq * 8 * sizeof(double));
     const dim3 grid(nn_blocks(A.rows, sms), ny);
     auto go = [&](auto kern) {
-        if (smem > 48 * 1024)
-            SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_smem(kern, nn_smem(128, nq));
         kern<<<grid, 32 * kNnWarps, smem, s>>>(A);
     };
     switch (nq) {

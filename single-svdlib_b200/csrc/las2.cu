@@ -244,6 +244,7 @@ class Las2Run {
     int eta_sel_ = 0;
     int64_t npurge_ = 0;
     int lz_blocks_ = 0, lz_cluster_ = 0;
+    LzResident lz_res_{};     // cluster launches with the operands in shared memory (res.on)
     bool lz_sliced_ = false;  // grid launches use both operands' column-sliced copies
     std::vector<double> alf_h_, bet_h_, ritz_, bnd_, w5_;
     // rotations of lanso's last Ritz analysis when it ran imtqlb (SVDLIBC)
@@ -434,6 +435,11 @@ int64_t Las2Run::lanczos_step(int64_t first, int64_t last, int64_t& ll, bool& en
         a.first = j; a.last = last; a.resume = resume ? 1 : 0;
         a.eps1 = EPS * std::sqrt((double)n_);
         a.sqrt_eps = std::sqrt(EPS);
+        a.res = lz_res_;
+        if (lz_res_.on) {  // alpha, beta and eta of this launch beside the operands, where they fit
+            a.res.coef = (int)std::min<int64_t>(last + 2, 1 << 20);
+            if (lz_res_layout(a.res, fp32_ ? 4 : 8).bytes > lanczos_resident_smem()) a.res.coef = 0;
+        }
         launch_lanczos_block(a, lz_blocks_, 512, lz_cluster_, s_, lz_sliced_);
         GridBarrier hb;
         SVDB_CUDA(cudaMemcpyAsync(&hs, st_.p, sizeof hs, cudaMemcpyDeviceToHost, s_));
@@ -702,6 +708,29 @@ void Las2Run::run(int64_t dimensions, int64_t iterations, double endl, double en
                 if (lanczos_cluster_ok(c, 512)) { lz_cluster_ = c; break; }
         }
         if (lz_cluster_) lz_blocks_ = lz_cluster_;
+        // Both operands in the cluster's shared memory where they fit: one
+        // element of every vector per thread (n <= 16 x 512), 16-bit column
+        // indices, and each CTA's slices beside the gathered vector
+        // (SVDB_LZ_CLUSTER=2 keeps the operands in global memory).
+        lz_res_.on = 0;
+        if (lz_cluster_ == kLzResCluster && !(env && atoi(env) == 2) && n_ > 0 && n_ <= kLzResCluster * 512 &&
+            op1_->nmajor <= 65535 && op1_->plan.slice16_nnz + op2_->plan.slice16_nnz < 65536) {
+            LzResident r{};
+            const DevCompressed* ops[2] = {op1_, op2_};
+            for (int k = 0; k < 2; ++k) {
+                r.rows_c[k] = (int)slice16_rows(ops[k]->nmajor);
+                r.max_nnz[k] = (int)ops[k]->plan.slice16_nnz;
+                r.g[k] = 2;  // lanes per row: about six entries each, eight in flight
+                while (r.g[k] < 32 && 6.5 * r.g[k] < ops[k]->avg_per_major()) r.g[k] *= 2;
+            }
+            r.n = (int)n_;
+            r.m = (int)op1_->nmajor;
+            const size_t smem = lz_res_layout(r, fp32_ ? 4 : 8).bytes;
+            if (lanczos_resident_ok(smem, 512)) {
+                r.on = 1;
+                lz_res_ = r;
+            }
+        }
     }
     // Large operators in grid mode: x slices in shared memory for both
     // products (spmv_sliced.cu), one block per SM (SVDB_SPMV=gather keeps the

@@ -258,9 +258,7 @@ static void right_mul(const double* X, int64_t rows, int c, const double* S, int
 
 static void chol_inv(RandCtx& cx, const double* G, int parts, int c, int64_t rows, double* R, const int* cond) {
     const size_t smem = chol_smem(c);
-    // chol_inv_body also holds some static shared memory
-    if (smem > 40 * 1024)
-        SVDB_CUDA(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_chol_inv, chol_smem(128));
     // shifted CholeskyQR: shift = 11 (rows c + c (c + 1)) u ||X||_F^2, ||X||_F^2 = trace(G)
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
     k_chol_inv<<<1, 384, smem, cx.s>>>(G, parts, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond);

@@ -337,6 +337,13 @@ __global__ void k_seg_fill(const int64_t* __restrict__ rp, const int64_t* __rest
     }
 }
 
+// counts[2] = the most entries in one of 16 equal row ranges
+__global__ void k_slice16(const int64_t* __restrict__ rp, int64_t rows, unsigned long long* __restrict__ counts) {
+    const int64_t per = slice16_rows(rows);
+    const int64_t r0 = min(rows, threadIdx.x * per), r1 = min(rows, r0 + per);
+    if (threadIdx.x < 16) atomicMax(counts + 2, (unsigned long long)(rp[r1] - rp[r0]));
+}
+
 __global__ void k_bin_flags(const int64_t* __restrict__ rp, int64_t rows, int64_t lo, int64_t hi,
                             uint8_t* __restrict__ flag, int32_t* __restrict__ ids) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
@@ -377,16 +384,21 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.seg_end.alloc(std::max<int64_t>(nseg, 1), s);
     p.multi_rows.alloc(std::max<int64_t>(rows, 1), s);
     p.long_rows.alloc(std::max<int64_t>(m.nnz / kSegNnz, 1), s);
-    DevBuf<unsigned long long> nm(2, s);
-    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, 2 * sizeof(unsigned long long), s));
+    DevBuf<unsigned long long> nm(3, s);
+    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, 3 * sizeof(unsigned long long), s));
     k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, seg, p.seg_row.p, p.seg_beg.p,
                                                    p.seg_end.p, p.multi_rows.p, p.long_rows.p, nm.p);
     SVDB_CHECK_LAUNCH();
-    unsigned long long hm[2] = {0, 0};
+    if (m.nnz < ((int64_t)1 << 20)) {
+        k_slice16<<<1, 32, 0, s>>>(m.ptr.p, rows, nm.p);
+        SVDB_CHECK_LAUNCH();
+    }
+    unsigned long long hm[3] = {0, 0, 0};
     SVDB_CUDA(cudaMemcpyAsync(hm, nm.p, sizeof(hm), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
     p.nmulti = (int64_t)hm[0];
     p.nlong = (int64_t)hm[1];
+    p.slice16_nnz = (int64_t)hm[2];
 
     // SpMV bins: a stable partition of the rows by length
     p.bin_rows.alloc(std::max<int64_t>(rows, 1), s);

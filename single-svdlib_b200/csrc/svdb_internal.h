@@ -42,6 +42,15 @@ void discount_launches(uint64_t n);  // launches recorded into a graph, counted 
     } while (0)
 #define SVDB_CHECK_LAUNCH() SVDB_CHECK_LAUNCH_N(1)
 
+// Allows `bytes` of dynamic shared memory for launches of `kern`.  Call it with
+// the most any launch of that kernel takes, not with this launch's: the setting
+// belongs to the kernel, and another thread's smaller one must not come between.
+template <typename F>
+inline void allow_smem(F kern, size_t bytes) {
+    if (bytes > 40 * 1024)  // below the default 48 KB with the kernels' static shared memory
+        SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // --------------------------------------------------------- device memory ----
 // Owning device buffer, stream-ordered (cudaMallocAsync pool).
 template <typename T>
@@ -89,6 +98,8 @@ constexpr int64_t kSegNnz = 2048;
 // kSpmvBinLen[b] entries (and more than kSpmvBinLen[b-1]), ascending, taken
 // by groups of (2 << b) lanes; rows of more than kSegNnz entries are
 // long_rows, one block each.
+// Rows of one of the 16 equal ranges slice16_nnz is counted over (even).
+__host__ __device__ inline int64_t slice16_rows(int64_t rows) { return ((rows + 15) / 16 + 1) / 2 * 2; }
 constexpr int kSpmvBins = 5;
 constexpr int64_t kSpmvBinLen[kSpmvBins] = {8, 16, 32, 64, kSegNnz};
 struct SpmvBins {
@@ -98,6 +109,7 @@ struct SpmvBins {
 };
 struct SegPlan {
     int64_t nseg = 0, nmulti = 0, nlong = 0;
+    int64_t slice16_nnz = 0;  // most entries in one of 16 equal row ranges (structures below 2^20 nonzeros)
     DevBuf<int32_t> bin_rows;
     SpmvBins bins{};
     DevBuf<int64_t> seg_first;
