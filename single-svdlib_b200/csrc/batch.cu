@@ -727,13 +727,13 @@ __global__ void k_b_colnorm(T* __restrict__ X, SubLayout L, const int64_t* __res
         for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) xb[r * ld + j] = (T)((double)xb[r * ld + j] * scale);
 }
 
-__global__ void __launch_bounds__(512) k_b_jacobi(const double* __restrict__ R, int c, double* __restrict__ U,
+__global__ void __launch_bounds__(256) k_b_jacobi(const double* __restrict__ R, int c, double* __restrict__ U,
                                                   double* __restrict__ V, double* __restrict__ sig,
                                                   int* __restrict__ status) {
     extern __shared__ double sm[];
     const int64_t b = blockIdx.x;
     const int64_t cc = (int64_t)c * c;
-    jacobi_svd_body(R + b * cc, c, U + b * cc, V + b * cc, sig + b * c, status + b, sm);
+    jacobi_svd_body<false>(R + b * cc, false, c, U + b * cc, V + b * cc, sig + b * c, status + b, sm);
 }
 
 // ------------------------------------------------------------ the batch ----
@@ -1062,10 +1062,9 @@ static void enqueue(svdb_batch& B) {
     cholesky_qr<T>(B, Y, LY, false);   // Q = qr(y).q()
     cols_product<T, double>(B, Y, B.Bt.p);  // B^T = A^T Q (FP64)
     cholesky_qr<double>(B, B.Bt.p, LZ, true);
-    const size_t smem = ((size_t)c * (c + 1) + (size_t)(c + 1) * (c + 1) + (c + 1)) * sizeof(double);
-    if (smem > 40 * 1024)  // jacobi_svd_body keeps a little static shared memory too
-        SVDB_CUDA(cudaFuncSetAttribute(k_b_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_b_jacobi<<<(unsigned)B.count, jacobi_threads(c, 512), smem, B.s>>>(B.Rout.p, c, B.Ur.p, B.Vr.p, B.sig.p, B.jstat.p);
+    allow_smem(k_b_jacobi, jacobi_smem(kBatchMaxL));
+    k_b_jacobi<<<(unsigned)B.count, jacobi_threads(c), jacobi_smem(c), B.s>>>(B.Rout.p, c, B.Ur.p, B.Vr.p, B.sig.p,
+                                                                              B.jstat.p);
     SVDB_CHECK_LAUNCH();
     // U_b = Q_b V_J[:, :rank] (m x rank);  V_b^T = (Q_Bt U_J[:, :rank])^T (rank x nb)
     right_mul<T, double>(B, Y, LY, B.Vr.p, false, (int)B.rank, B.U.p, (int)B.rank, false, nullptr);

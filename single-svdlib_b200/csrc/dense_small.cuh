@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "dense_tall.cuh"
 #include "device_common.cuh"
@@ -229,106 +230,150 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
         }
 }
 
-// Lanes per column pair in jacobi_svd_body (about eight elements of a column
-// per lane), and the block size that gives every pair of the padded columns
-// its lanes, capped at `cap` threads.
-__host__ __device__ inline int jacobi_group(int c) { return c <= 64 ? 8 : (c <= 128 ? 16 : 32); }
-__host__ __device__ inline int jacobi_threads(int c, int cap) {
+// Lanes per column pair in jacobi_svd_body (at most four 16-byte vectors of a
+// column per lane), and the block size that gives every pair of the padded
+// columns its lanes.  c <= 128.
+__host__ __device__ inline int jacobi_group(int c) { return c <= 32 ? 4 : (c <= 64 ? 8 : 16); }
+__host__ __device__ inline int jacobi_threads(int c) {
     const int cp = c + (c & 1);
     const int t = ((cp / 2) * jacobi_group(c) + 31) / 32 * 32;
-    return t < 32 ? 32 : (t > cap ? cap : t);
+    return t < 32 ? 32 : t;
+}
+__host__ __device__ inline size_t jacobi_smem(int c) {
+    const size_t cp = c + (c & 1);
+    return (2 * cp * cp + cp) * sizeof(double) + cp * sizeof(int);
 }
 
-// One-sided Jacobi SVD of R (c x c, row-major) in one block: W = R V with
-// orthogonal columns, sigma_j = |W_j|, U_j = W_j / sigma_j.  Round-robin pair
-// ordering, jacobi_group(c) lanes per pair.  Outputs sorted by descending sigma:
-// U (c x c), V (c x c), sig (c).  *status = sweeps << 8, | 2 if the sweep limit is reached.
-// sm: (c * cp + cp * cp + cp) doubles, cp = c rounded up to even.  Any
-// block size that is a multiple of 32.
-__device__ __forceinline__ void jacobi_svd_body(const double* __restrict__ R, int c, double* __restrict__ U,
-                                                double* __restrict__ V, double* __restrict__ sig,
-                                                int* __restrict__ status, double* sm) {
-    // W (c x cp) | Vs (c x cp) | norms (cp) ; column-major
-    const int cp = c + (c & 1);     // even number of columns (zero padding column)
-    double* W = sm;
-    double* Vs = sm + (size_t)c * cp;
-    double* nr = Vs + (size_t)cp * cp;
-    __shared__ int s_rot;
-    for (int t = threadIdx.x; t < c * cp; t += blockDim.x) {
-        const int i = t % c, j = t / c;
-        W[j * c + i] = (j < c) ? R[i * c + j] : 0.0;
+// One round: every pair of columns (p, q) of the round-robin is made
+// orthogonal.  G lanes per pair, E double2 of each column per lane, all held
+// in registers between the sums and the update, and the columns of Vs read
+// while the rotation is computed.  Returns whether this thread's pair rotated.
+template <int G, int E>
+__device__ __forceinline__ bool jacobi_round(double* W, double* Vs, int cp, int round, double tol2) {
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const int pr = (int)threadIdx.x / G, half = cp / 2, ring = cp - 1;
+    // round-robin: position 0 fixed, the others rotate
+    int p = pr - 1 + round, q = cp - 2 - pr + round;
+    p = pr == 0 ? 0 : 1 + (p >= ring ? p - ring : p);
+    q = 1 + (q >= ring ? q - ring : q);
+    const bool valid = pr < half;
+    if (p > q) { const int t = p; p = q; q = t; }
+    if (!valid) p = q = 0;
+    double2* wp = reinterpret_cast<double2*>(W + p * cp) + sub;
+    double2* wq = reinterpret_cast<double2*>(W + q * cp) + sub;
+    double2* vp = reinterpret_cast<double2*>(Vs + p * cp) + sub;
+    double2* vq = reinterpret_cast<double2*>(Vs + q * cp) + sub;
+    constexpr bool AHEAD = G < 16;  // registers: wide blocks (c > 64) read Vs after the rotation
+    double2 x[E], y[E], vx[AHEAD ? E : 1], vy[AHEAD ? E : 1];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const bool in = valid && sub + G * e < half;
+        x[e] = in ? wp[G * e] : make_double2(0.0, 0.0);
+        y[e] = in ? wq[G * e] : make_double2(0.0, 0.0);
     }
-    for (int t = threadIdx.x; t < cp * cp; t += blockDim.x) Vs[t] = ((t % cp) == (t / cp)) ? 1.0 : 0.0;
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool in = valid && sub + G * e < half;
+            vx[e] = in ? vp[G * e] : make_double2(0.0, 0.0);
+            vy[e] = in ? vq[G * e] : make_double2(0.0, 0.0);
+        }
+    }
+    double al = 0, be = 0, ga = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        al = fma(x[e].y, x[e].y, fma(x[e].x, x[e].x, al));
+        be = fma(y[e].y, y[e].y, fma(y[e].x, y[e].x, be));
+        ga = fma(x[e].y, y[e].y, fma(x[e].x, y[e].x, ga));
+    }
+#pragma unroll
+    for (int o = G >> 1; o > 0; o >>= 1) {
+        al += __shfl_xor_sync(0xffffffffu, al, o);
+        be += __shfl_xor_sync(0xffffffffu, be, o);
+        ga += __shfl_xor_sync(0xffffffffu, ga, o);
+    }
+    // |ga| > tol sqrt(al be), compared in squares.  The rotation of the
+    // usual zeta = (be - al) / (2 ga), t = sign(zeta) / (|zeta| +
+    // sqrt(1 + zeta^2)), cs = 1 / sqrt(1 + t^2), with numerator and
+    // denominator of t scaled by |2 ga|: one sqrt, one division, one
+    // reciprocal square root on the dependent path.
+    if (!(valid && ga != 0.0 && ga * ga > tol2 * (al * be))) return false;
+    const double d = be - al, g2 = 2.0 * ga;
+    const bool pos = (d >= 0.0) == (ga > 0.0) || d == 0.0;  // sign(zeta) >= 0
+    const double t = (pos ? fabs(g2) : -fabs(g2)) / (fabs(d) + sqrt(fma(d, d, g2 * g2)));
+    const double cs = rsqrt(fma(t, t, 1.0)), sn = cs * t;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        if (sub + G * e >= half) continue;
+        wp[G * e] = make_double2(cs * x[e].x - sn * y[e].x, cs * x[e].y - sn * y[e].y);
+        wq[G * e] = make_double2(sn * x[e].x + cs * y[e].x, sn * x[e].y + cs * y[e].y);
+        const double2 a = AHEAD ? vx[AHEAD ? e : 0] : vp[G * e], b = AHEAD ? vy[AHEAD ? e : 0] : vq[G * e];
+        vp[G * e] = make_double2(cs * a.x - sn * b.x, cs * a.y - sn * b.y);
+        vq[G * e] = make_double2(sn * a.x + cs * b.x, sn * a.y + cs * b.y);
+    }
+    return true;
+}
+
+// One-sided Jacobi SVD of R (c x c, row-major; its transpose when `trans`) in
+// one block: W = R V with orthogonal columns, sigma_j = |W_j|, U_j = W_j /
+// sigma_j.  Round-robin pair ordering.  Outputs sorted by descending sigma: U
+// (c x c), V (c x c), sig (c).  *status = sweeps << 8, | 2 if the sweep limit
+// is reached.  sm: jacobi_smem(c) bytes; jacobi_threads(c) threads; c <= 64, or
+// 65 to 128 when WIDE.
+// A round is a chain (reads, three sums over the pair's lanes, square root,
+// division and reciprocal square root, update, barrier) and, at c = 60, 115 KB
+// through shared memory.  With every element read again for the update, 8-byte
+// accesses and Vs read after the rotation one solve took 750 us at c = 60, 388
+// at 40 and 136 at 20; this form 417, 228 and 79.
+template <bool WIDE>
+__device__ __forceinline__ void jacobi_svd_body(const double* __restrict__ R, bool trans, int c,
+                                                double* __restrict__ U, double* __restrict__ V,
+                                                double* __restrict__ sig, int* __restrict__ status, double* sm) {
+    // W (cp x cp) | Vs (cp x cp) | norms (cp) | ranks (cp) ; column-major, an
+    // odd c padded with a zero row and column
+    const int cp = c + (c & 1);
+    double* W = sm;
+    double* Vs = sm + (size_t)cp * cp;
+    double* nr = Vs + (size_t)cp * cp;
+    int* rank = reinterpret_cast<int*>(nr + cp);
+    for (int t = threadIdx.x; t < cp * cp; t += blockDim.x) {
+        const int j = t / cp, i = t - j * cp;
+        W[t] = (i < c && j < c) ? (trans ? R[j * c + i] : R[i * c + j]) : 0.0;
+        Vs[t] = i == j ? 1.0 : 0.0;
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int half = cp / 2;
-    // G lanes per column pair, 32 / G pairs per warp: the pair's scalar work
-    // (three sums, the rotation's sqrt, division and rsqrt) is issued once
-    // per warp for 32 / G pairs.  Pairs are walked warp by warp so that the
-    // shuffles see the whole warp.
-    const int G = jacobi_group(c), gpw = 32 / G, sub = lane & (G - 1), gw = lane / G;
-    const double tol = 2.220446049250313e-16 * (double)(c > 4 ? c : 4);
-    int sweep = 0;
-    for (; sweep < 60; ++sweep) {
-        if (threadIdx.x == 0) s_rot = 0;
-        __syncthreads();
-        for (int round = 0; round < cp - 1; ++round) {
-            for (int base = warp * gpw; base < half; base += nwarps * gpw) {
-                const int pr = base + gw;
-                const bool valid = pr < half;
-                // round-robin: position 0 fixed, others rotate
-                auto at = [&](int pos) { return pos == 0 ? 0 : 1 + (pos - 1 + round) % (cp - 1); };
-                int p = 0, q = 0;
-                if (valid) {
-                    p = at(pr);
-                    q = at(cp - 1 - pr);
-                    if (p > q) { int t = p; p = q; q = t; }
-                }
-                double al = 0, be = 0, ga = 0;
-                if (valid)
-                    for (int i = sub; i < c; i += G) {
-                        const double x = W[p * c + i], y = W[q * c + i];
-                        al = fma(x, x, al);
-                        be = fma(y, y, be);
-                        ga = fma(x, y, ga);
-                    }
-                for (int o = G >> 1; o > 0; o >>= 1) {
-                    al += __shfl_xor_sync(0xffffffffu, al, o);
-                    be += __shfl_xor_sync(0xffffffffu, be, o);
-                    ga += __shfl_xor_sync(0xffffffffu, ga, o);
-                }
-                // |ga| > tol sqrt(al be), compared in squares.  The rotation of the
-                // usual zeta = (be - al) / (2 ga), t = sign(zeta) / (|zeta| +
-                // sqrt(1 + zeta^2)), cs = 1 / sqrt(1 + t^2), with numerator and
-                // denominator of t scaled by |2 ga|: one sqrt, one division, one
-                // reciprocal square root on the dependent path.
-                if (valid && ga != 0.0 && ga * ga > (tol * tol) * (al * be)) {
-                    const double d = be - al, g2 = 2.0 * ga;
-                    const bool pos = (d >= 0.0) == (ga > 0.0) || d == 0.0;  // sign(zeta) >= 0
-                    const double t = (pos ? fabs(g2) : -fabs(g2)) / (fabs(d) + sqrt(fma(d, d, g2 * g2)));
-                    const double cs = rsqrt(fma(t, t, 1.0)), sn = cs * t;
-                    for (int i = sub; i < c; i += G) {
-                        const double x = W[p * c + i], y = W[q * c + i];
-                        W[p * c + i] = cs * x - sn * y;
-                        W[q * c + i] = sn * x + cs * y;
-                    }
-                    for (int i = sub; i < cp; i += G) {
-                        const double x = Vs[p * cp + i], y = Vs[q * cp + i];
-                        Vs[p * cp + i] = cs * x - sn * y;
-                        Vs[q * cp + i] = sn * x + cs * y;
-                    }
-                    if (sub == 0) s_rot = 1;
-                }
+    const double tol = 2.220446049250313e-16 * (double)(c > 4 ? c : 4), tol2 = tol * tol;
+    auto sweeps = [&](auto g, auto e) {
+        int sweep = 0;
+        for (; sweep < 60; ++sweep) {
+            int rot = 0;
+            for (int round = 0; round < cp - 1; ++round) {
+                rot |= jacobi_round<decltype(g)::value, decltype(e)::value>(W, Vs, cp, round, tol2);
+                __syncthreads();
             }
-            __syncthreads();
+            if (!__syncthreads_or(rot)) break;
         }
-        if (!s_rot) break;
-        __syncthreads();
+        return sweep;
+    };
+    int sweep;
+    using std::integral_constant;
+#define SVDB_JACOBI(G, E) sweep = sweeps(integral_constant<int, G>(), integral_constant<int, E>())
+    if constexpr (WIDE) {
+        if (c <= 96) SVDB_JACOBI(16, 3);
+        else SVDB_JACOBI(16, 4);
+    } else {
+        if (c <= 16) SVDB_JACOBI(4, 2);
+        else if (c <= 24) SVDB_JACOBI(4, 3);
+        else if (c <= 32) SVDB_JACOBI(4, 4);
+        else if (c <= 48) SVDB_JACOBI(8, 3);
+        else SVDB_JACOBI(8, 4);
     }
+#undef SVDB_JACOBI
     if (threadIdx.x == 0) *status = (sweep << 8) | (sweep == 60 ? 2 : 0);  // sweeps, limit flag
     for (int j = warp; j < cp; j += nwarps) {
         double s = 0.0;
-        for (int i = lane; i < c; i += 32) s = fma(W[j * c + i], W[j * c + i], s);
+        for (int i = lane; i < c; i += 32) s = fma(W[j * cp + i], W[j * cp + i], s);
         s = warp_sum(s);
         if (lane == 0) nr[j] = sqrt(s);
     }
@@ -338,11 +383,14 @@ __device__ __forceinline__ void jacobi_svd_body(const double* __restrict__ R, in
         int pos = 0;
         for (int k = 0; k < c; ++k)
             if (nr[k] > nr[j] || (nr[k] == nr[j] && k < j)) ++pos;
+        rank[j] = pos;
         sig[pos] = nr[j];
-        for (int i = 0; i < c; ++i) {
-            U[i * c + pos] = nr[j] > 0.0 ? W[j * c + i] / nr[j] : (i == pos ? 1.0 : 0.0);
-            V[i * c + pos] = Vs[j * cp + i];
-        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < c * c; t += blockDim.x) {
+        const int j = t / c, i = t - j * c, pos = rank[j];
+        U[i * c + pos] = nr[j] > 0.0 ? W[j * cp + i] / nr[j] : (i == pos ? 1.0 : 0.0);
+        V[i * c + pos] = Vs[j * cp + i];
     }
 }
 

@@ -90,11 +90,18 @@ __global__ void k_colnorm(T* __restrict__ X, int64_t rows, int c) {
 }
 
 // One-sided Jacobi SVD of the c x c R in one block (jacobi_svd_body).
-__global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ R, int c, double* __restrict__ U,
-                                                     double* __restrict__ V, double* __restrict__ sig,
-                                                     int* __restrict__ status) {
+__global__ void __launch_bounds__(960) k_jacobi_svd(const double* __restrict__ R, int trans, int c,
+                                                     double* __restrict__ U, double* __restrict__ V,
+                                                     double* __restrict__ sig, int* __restrict__ status) {
     extern __shared__ double sm[];
-    jacobi_svd_body(R, c, U, V, sig, status, sm);
+    jacobi_svd_body<true>(R, trans != 0, c, U, V, sig, status, sm);
+}
+// c <= 64: the widths of most solves, with the registers of smaller blocks
+__global__ void __launch_bounds__(256) k_jacobi_svd64(const double* __restrict__ R, int trans, int c,
+                                                      double* __restrict__ U, double* __restrict__ V,
+                                                      double* __restrict__ sig, int* __restrict__ status) {
+    extern __shared__ double sm[];
+    jacobi_svd_body<false>(R, trans != 0, c, U, V, sig, status, sm);
 }
 
 __global__ void k_to_float(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
@@ -463,10 +470,8 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
     DevBuf<double> U(std::max<int64_t>(m * actual, 1), s), Vt(std::max<int64_t>(actual * n, 1), s),
         S(std::max<int64_t>(actual, 1), s);
     {
-        DevBuf<double> Ur((size_t)r * r, s), Vr((size_t)r * r, s), R((size_t)r * r, s), Rt((size_t)r * r, s), sig(r, s);
-        const size_t smem = ((size_t)r * (r + 1) + (size_t)(r + 1) * (r + 1) + (r + 1)) * sizeof(double);
-        if (smem > 220 * 1024) throw Error(SVDB_ERR_UNSUPPORTED, "randomized_svd: sample width above the Jacobi tile");
-        SVDB_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DevBuf<double> Ur((size_t)r * r, s), Vr((size_t)r * r, s), R((size_t)r * r, s), sig(r, s);
+        if (r > 117) throw Error(SVDB_ERR_UNSUPPORTED, "randomized_svd: sample width above the Jacobi tile");
         DevBuf<double> B;  // n < c: B = Bt^T (c x n) is the tall one
         if (n < c) {
             B.alloc((size_t)c * n, s);
@@ -478,8 +483,13 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
         double* tall = n < c ? B.p : Bt.p;
         const int64_t trows = n < c ? c : n;
         cholesky_qr(cx, tall, trows, r, R.p);
-        transpose_dense<double>(R.p, Rt.p, r, r, s);
-        k_jacobi_svd<<<1, jacobi_threads(r, 1024), smem, s>>>(Rt.p, r, Vr.p, Ur.p, sig.p, jac_status.p);
+        if (r <= 64) {
+            allow_smem(k_jacobi_svd64, jacobi_smem(64));
+            k_jacobi_svd64<<<1, jacobi_threads(r), jacobi_smem(r), s>>>(R.p, 1, r, Vr.p, Ur.p, sig.p, jac_status.p);
+        } else {
+            allow_smem(k_jacobi_svd, jacobi_smem(117));
+            k_jacobi_svd<<<1, jacobi_threads(r), jacobi_smem(r), s>>>(R.p, 1, r, Vr.p, Ur.p, sig.p, jac_status.p);
+        }
         SVDB_CHECK_LAUNCH();
         if (actual > 0) {
             if (n >= c) {
