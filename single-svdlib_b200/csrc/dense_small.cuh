@@ -65,7 +65,10 @@ __device__ __forceinline__ double omega_value(uint64_t key, int64_t i) {
 // breakdown sets bit 2 and leaves R = R^-1 = I.
 // G: c x c, or with nparts > 0 the sum of nparts such matrices, in order (only
 // the tiles on and above the diagonal are read).  c <= 128; blockDim.x a
-// multiple of 32, at least 160.  sm: chol_smem(c) bytes.
+// multiple of 32, at least 160.  sm: chol_smem(c) bytes.  loose (may be null) is
+// set when an entry of G is more than 0.1 from the identity's, or on a shift: an
+// X with a G closer than that has kappa below 2, so X R^-1 is orthonormal to
+// rounding.
 __host__ __device__ inline int chol_ld(int c) { return ((c + 7) / 8 + 1) * 8 + 4; }  // = 4 or 12 mod 16: no conflicts
 __host__ __device__ inline size_t chol_smem(int c) {
     const int nt = (c + 7) / 8;
@@ -73,7 +76,8 @@ __host__ __device__ inline size_t chol_smem(int c) {
 }
 __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int nparts, int c, double shift_scale,
                                               double* __restrict__ R, double* __restrict__ Ri,
-                                              int* __restrict__ flags, int* __restrict__ shifted, double* sm) {
+                                              int* __restrict__ flags, int* __restrict__ shifted, double* sm,
+                                              int* __restrict__ loose = nullptr) {
     __shared__ int s_fail;
     __shared__ double s_inv[8], s_shift;
     const int nt = (c + 7) / 8, c8 = nt * 8, ld = chol_ld(c), cc = c * c;
@@ -100,7 +104,11 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
             for (int j = lane; j < i8; j += 32) sm[i * ld + j] = 0.0;
             for (int j = i8 + lane; j < c8; j += 32) {
                 double v = i == j ? 1.0 : 0.0;
-                if (i < c && j < c) v = g_at(i, j) + (i == j ? shift : 0.0);
+                if (i < c && j < c) {
+                    const double g = g_at(i, j);
+                    if (loose && !(fabs(g - v) <= 0.1)) *loose = 1;
+                    v = g + (i == j ? shift : 0.0);
+                }
                 sm[i * ld + 8 + j] = v;
             }
         }
@@ -213,6 +221,7 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
             s_shift = shift_scale * tr > 0.0 ? shift_scale * tr : 1e-300;
             atomicOr(flags, 1);
             *shifted = 1;
+            if (loose) *loose = 1;
         }
         __syncthreads();  // also orders this attempt's reads before the next one's writes
         shift = s_shift;

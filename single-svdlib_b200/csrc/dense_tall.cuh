@@ -46,7 +46,7 @@ struct TnShape {
 inline size_t tn_smem_max(int nt) { return (size_t)16 * nt * nt * 64 * sizeof(double); }  // sixteen warps
 // `ctas` CTAs at most.  One CTA of up to 16 warps per SM: 148 partials to add
 // instead of the 296 of two smaller CTAs.
-inline TnShape tn_shape(int64_t rows, int p, int q, bool sym, int ctas) {
+__host__ __device__ inline TnShape tn_shape(int64_t rows, int p, int q, bool sym, int ctas) {
     TnShape h;
     h.sym = sym;
     const int tiles = (std::max(p, q) + 7) / 8;
@@ -258,7 +258,7 @@ struct NnArgs {
 };
 
 constexpr int kNnWarps = 8, kNnMT = 2, kNnKU = 4;
-inline size_t nn_smem(int p, int nq) { return (size_t)((p + 3) / 4 * 4) * (nq * 8 + 4) * sizeof(double); }
+__host__ __device__ inline size_t nn_smem(int p, int nq) { return (size_t)((p + 3) / 4 * 4) * (nq * 8 + 4) * sizeof(double); }
 
 // the warps of the calling CTA walk row groups g0, g0 + gstep, ... (16 rows each)
 template <typename TX, typename TO, int NQ, int DOT>

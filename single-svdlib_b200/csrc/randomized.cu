@@ -14,6 +14,8 @@
 // SVDB_MIXED runs the sparse products on FP32 matrix values and an FP32 copy
 // of the dense operand (half the gathered bytes) with FP64 sums; the Gram
 // products, Cholesky, both CholeskyQR passes and the small SVD stay FP64.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -27,6 +29,8 @@
 #include "svdb_internal.h"
 
 namespace svdb {
+
+namespace cg = cooperative_groups;
 
 static int nb(int64_t work, int threads, int per_sm = 16) {
     int64_t b = (work + threads - 1) / threads;
@@ -47,10 +51,113 @@ __global__ void k_omega(uint64_t seed, int64_t total, T* __restrict__ out) {
 __global__ void __launch_bounds__(384) k_chol_inv(const double* __restrict__ G, int nparts, int c, double shift_scale,
                                                   double* __restrict__ R, double* __restrict__ Ri,
                                                   int* __restrict__ flags, int* __restrict__ shifted,
-                                                  const int* __restrict__ cond) {
+                                                  const int* __restrict__ cond, int* __restrict__ loose) {
     if (cond && *cond == 0) return;
     extern __shared__ double sm[];
-    chol_inv_body(G, nparts, c, shift_scale, R, Ri, flags, shifted, sm);
+    chol_inv_body(G, nparts, c, shift_scale, R, Ri, flags, shifted, sm, loose);
+}
+
+// CholeskyQR2 of X (rows x c, in place), the third pass included when a shift
+// was used, in one cluster of kQrCluster CTAs that each own a range of rows:
+// Gram partials in shared memory, summed a slice per CTA and handed round;
+// every CTA factors the same G (no hand-over), and multiplies its own rows.
+// One launch instead of ten to thirteen (four per pass, the third pass's
+// returning at once): for few rows the launches and their gaps were most of the
+// time (1,000 x 20: 40 us per factorisation against 55 and ten gaps; 5,600 x 40:
+// 92 us against 105).
+// Rout (may be null) = R_last ... R_first; Rw: 3 c x c of workspace.
+constexpr int kQrCluster = 16, kQrThreads = 384;
+struct QrLayout {
+    size_t part, red, G, chol, Ri, bytes;  // doubles; red, chol and the nn factor share one region
+};
+__host__ __device__ inline QrLayout qr_layout(int c) {
+    const TnShape h = tn_shape(1, c, c, true, 1);
+    const size_t red = (size_t)(kQrThreads / 32) * h.nt * h.nt * 64;
+    const size_t region = std::max(std::max(red, chol_smem(c) / 8), nn_smem(c, (c + 7) / 8) / 8);
+    QrLayout L;
+    L.part = 0;
+    L.G = (size_t)c * c;
+    L.Ri = L.G + (size_t)c * c;
+    L.red = L.Ri + (size_t)c * c;
+    L.chol = L.red;
+    L.bytes = (L.red + region) * 8;
+    return L;
+}
+template <int NT, int NQ>
+__device__ __forceinline__ void qr_pass(double* X, int64_t rows, int c, int nb, int rg, double shift_scale, double* R,
+                                        int* flags, int* shifted, int* loose, double* sm, const QrLayout& L) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), cc = c * c;
+    tn_part_body<double, double, NT>(X, c, c, X, c, c, 0, rows, nb, nb, true, rg, sm + L.part, sm + L.red);
+    cl.sync();  // every CTA's partial is there
+    // a slice of G per CTA, written into all of them (tile blocks I <= J; the
+    // others are never read)
+    const int per = (cc + kQrCluster - 1) / kQrCluster;
+    const int w = NT * 8;
+    for (int e = rank * per + (int)threadIdx.x; e < min(cc, (rank + 1) * per); e += blockDim.x) {
+        if ((e / c) / w > (e % c) / w) continue;
+        double v[kQrCluster], t = 0.0;
+#pragma unroll
+        for (int b = 0; b < kQrCluster; ++b) v[b] = *cl.map_shared_rank(sm + L.part + e, b);
+#pragma unroll
+        for (int b = 0; b < kQrCluster; ++b) t += v[b];
+#pragma unroll
+        for (int b = 0; b < kQrCluster; ++b) *cl.map_shared_rank(sm + L.G + e, b) = t;
+    }
+    cl.sync();
+    // flags and R: one CTA's stores are enough (the others' go where nobody looks)
+    chol_inv_body(sm + L.G, 0, c, shift_scale, rank == 0 ? R : sm + L.part, sm + L.Ri, flags, shifted, sm + L.chol,
+                  loose);
+    __syncthreads();
+    const NnArgs<double, double> A{X, c, rows, c, sm + L.Ri, c, nullptr, c, 1, 1.0, nullptr, 0, 0.0, nullptr, 0,
+                                   nullptr, X, c, 0, nullptr, nullptr};
+    nn_body<double, double, NQ, 0>(A, threadIdx.x >> 5, blockDim.x >> 5, 0, sm + L.red);
+    __syncthreads();
+}
+template <int NT, int NQ>
+__global__ void __launch_bounds__(kQrThreads, 1) k_cholqr_cluster(double* X, int64_t rows, int c, int nb, int rg,
+                                                                  double shift_scale, double* Rw, double* Rout,
+                                                                  int* flags, const int* cond, int* loose) {
+    if (cond && *cond == 0) return;  // the same for every CTA
+    extern __shared__ double qr_sm[];
+    __shared__ int s_shifted, s_loose;
+    cg::cluster_group cl = cg::this_cluster();
+    const QrLayout L = qr_layout(c);
+    const int rank = (int)cl.block_rank(), cc = c * c;
+    const int64_t per = (rows + kQrCluster - 1) / kQrCluster;
+    const int64_t r0 = min(rows, rank * per), mine = min(rows, r0 + per) - r0;
+    if (threadIdx.x == 0) s_shifted = s_loose = 0;
+    __syncthreads();
+    X += r0 * c;
+    int passes = 2;
+    for (int p = 0; p < passes; ++p) {
+        qr_pass<NT, NQ>(X, mine, c, nb, rg, shift_scale, Rw + p * cc, flags, &s_shifted, p == 1 ? &s_loose : nullptr,
+                        qr_sm, L);
+        if (p == 1 && s_shifted) passes = 3;  // every CTA factored the same matrices
+    }
+    if (rank == 0) {
+        if (threadIdx.x == 0 && loose && (s_loose || s_shifted)) *loose = 1;
+        if (Rout) {  // R_last ... R_first, this CTA's own stores
+            double* acc = qr_sm + L.part;
+            double* tmp = qr_sm + L.G;
+            for (int t = threadIdx.x; t < cc; t += blockDim.x) acc[t] = Rw[t];
+            __syncthreads();
+            for (int p = 1; p < passes; ++p) {
+                for (int t = threadIdx.x; t < cc; t += blockDim.x) {
+                    const int i = t / c, j = t - i * c;
+                    double v = 0.0;
+                    for (int k = i; k <= j; ++k) v = fma(Rw[(int64_t)p * cc + i * c + k], acc[k * c + j], v);
+                    tmp[t] = v;
+                }
+                __syncthreads();
+                double* o = acc;
+                acc = tmp;
+                tmp = o;
+            }
+            for (int t = threadIdx.x; t < cc; t += blockDim.x) Rout[t] = acc[t];
+        }
+    }
+    cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // C (c x c) = A (c x c) B (c x c), one thread per element
@@ -148,7 +255,7 @@ __global__ void k_major_means(const int64_t* __restrict__ ptr, const double* __r
 // every eighth row of the chunk, its lanes the columns, four rows in flight;
 // the warps' partials are added in warp order, the chunks' by k_tn_reduce.
 // 256-row chunks with one row in flight and one thread per column over all
-// chunks took 18 + 12 us per product of 30,011 x 40; this form DISPLACE.
+// chunks took 18 + 12 us per product of 30,011 x 40; this form 6 + 6.
 constexpr int kCsCols = 128;
 template <int NC>
 __global__ void __launch_bounds__(256) k_wcolsum_part(const double* __restrict__ X, int64_t rows, int64_t ld, int c,
@@ -224,8 +331,8 @@ void center_product(const double* X, int64_t xrows, int c, const double* mu, dou
 // ------------------------------------------------------ host helpers ----
 struct RandCtx {
     cudaStream_t s;
-    DevBuf<double> part, G, R1, R2, R3, Ri, Rtmp, T;
-    DevBuf<int> flags, shifted;
+    DevBuf<double> part, G, R1, Ri, Rtmp, T;  // R1: the passes' three factors
+    DevBuf<int> flags, shifted, loose;
     int64_t part_cap = 0;
 };
 
@@ -268,41 +375,108 @@ static void right_mul(const double* X, int64_t rows, int c, const double* S, int
                  device_props().sms, s);
 }
 
-static void chol_inv(RandCtx& cx, const double* G, int parts, int c, int64_t rows, double* R, const int* cond) {
+// shifted CholeskyQR: shift = 11 (rows c + c (c + 1)) u ||X||_F^2, ||X||_F^2 = trace(G)
+static double qr_shift(int64_t rows, int c) {
+    return 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
+}
+
+static void chol_inv(RandCtx& cx, const double* G, int parts, int c, int64_t rows, double* R, const int* cond,
+                     int* loose) {
     const size_t smem = chol_smem(c);
     allow_smem(k_chol_inv, chol_smem(128));
-    // shifted CholeskyQR: shift = 11 (rows c + c (c + 1)) u ||X||_F^2, ||X||_F^2 = trace(G)
-    const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
-    k_chol_inv<<<1, 384, smem, cx.s>>>(G, parts, c, shift_scale, R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond);
+    k_chol_inv<<<1, 384, smem, cx.s>>>(G, parts, c, qr_shift(rows, c), R, cx.Ri.p, cx.flags.p, cx.shifted.p, cond,
+                                       loose);
     SVDB_CHECK_LAUNCH();
+}
+
+// The one-cluster form: c <= 64 (one column block, in place), a device that can
+// hold the cluster, and few enough rows for its 16 SMs.  Whole solves (q = 2)
+// with it and without: 4,000 x 60 1.33 / 1.48 ms, 8,000 x 60 1.58 / 1.56; 8,000 x
+// 40 1.02 / 1.07, 16,000 x 40 1.36 / 1.17; 16,000 x 20 0.75 / 0.82.
+constexpr int64_t kQrClusterSize = 320 << 10;  // rows x columns
+template <int NT, int NQ>
+static bool cholqr_cluster_as(RandCtx& cx, double* X, int64_t rows, int c, double* Rout, const int* cond, int* loose) {
+    auto kern = k_cholqr_cluster<NT, NQ>;
+    const TnShape h = tn_shape(1, c, c, true, 1);
+    const size_t most = qr_layout(NQ * 8).bytes;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kQrCluster);
+    cfg.blockDim = dim3(kQrThreads / (32 * h.ntb) * h.ntb * 32);
+    cfg.dynamicSmemBytes = most;
+    cfg.stream = cx.s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kQrCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    // whether this device holds the kernel's widest cluster: asked once per
+    // thread and device, like device_props()
+    static thread_local int asked_dev = -1;
+    static thread_local bool holds = false;
+    int dev = 0;
+    SVDB_CUDA(cudaGetDevice(&dev));
+    if (dev != asked_dev) {
+        int n = 0;
+        holds = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
+        if (!holds) cudaGetLastError();
+        asked_dev = dev;
+    }
+    if (!holds) return false;
+    cfg.dynamicSmemBytes = qr_layout(c).bytes;
+    SVDB_CUDA(cudaLaunchKernelEx(&cfg, kern, X, rows, c, h.nbp, (int)cfg.blockDim.x / (32 * h.ntb), qr_shift(rows, c),
+                                 cx.R1.p, Rout, cx.flags.p, cond, loose));
+    SVDB_CHECK_LAUNCH();
+    return true;
+}
+static bool cholqr_cluster(RandCtx& cx, double* X, int64_t rows, int c, double* Rout, const int* cond, int* loose) {
+    if (rows * c > kQrClusterSize || c > 64) return false;
+    switch ((c + 7) / 8) {
+        case 1: return cholqr_cluster_as<1, 1>(cx, X, rows, c, Rout, cond, loose);
+        case 2: return cholqr_cluster_as<2, 2>(cx, X, rows, c, Rout, cond, loose);
+        case 3: return cholqr_cluster_as<3, 3>(cx, X, rows, c, Rout, cond, loose);
+        case 4: return cholqr_cluster_as<4, 4>(cx, X, rows, c, Rout, cond, loose);
+        case 5: return cholqr_cluster_as<3, 5>(cx, X, rows, c, Rout, cond, loose);
+        case 6: return cholqr_cluster_as<3, 6>(cx, X, rows, c, Rout, cond, loose);
+        case 7: return cholqr_cluster_as<4, 7>(cx, X, rows, c, Rout, cond, loose);
+        default: return cholqr_cluster_as<4, 8>(cx, X, rows, c, Rout, cond, loose);
+    }
 }
 
 // Thin Q of X (rows x c, rows >= c) in place; Rout (c x c) = R_last ... R_first
 // when requested.  CholeskyQR2; a pass whose Cholesky broke down is redone with
 // a shift and a third pass follows.  Nothing here waits for the device: the
-// third pass's kernels read the device flag and return when it is 0.
-static void cholesky_qr(RandCtx& cx, double* X, int64_t rows, int c, double* Rout) {
+// third pass's kernels read the device flag and return when it is 0.  only_if
+// (a device flag, may be null): nothing happens when it is 0.  loose: see
+// chol_inv_body, for the second pass's Gram.
+static void cholesky_qr(RandCtx& cx, double* X, int64_t rows, int c, double* Rout, const int* only_if = nullptr,
+                        int* loose = nullptr) {
     cudaStream_t s = cx.s;
+    if (cholqr_cluster(cx, X, rows, c, Rout, only_if, loose)) return;
     if ((int64_t)cx.T.n < rows * c) cx.T.alloc(rows * c, s);
     double* T = cx.T.p;
     SVDB_CUDA(cudaMemsetAsync(cx.shifted.p, 0, sizeof(int), s));
-    auto pass = [&](const double* in, double* out, double* R, const int* cond) {
+    double* R[3] = {cx.R1.p, cx.R1.p + (int64_t)c * c, cx.R1.p + 2 * (int64_t)c * c};
+    auto pass = [&](const double* in, double* out, double* Rp, const int* cond, int* ls) {
         int parts = 0;
         const double* G = gram(cx, in, rows, c, cx.G.p, cond, parts);
-        chol_inv(cx, G, parts, c, rows, R, cond);
+        chol_inv(cx, G, parts, c, rows, Rp, cond, ls);
         right_mul(in, rows, c, cx.Ri.p, c, c, out, s, cond, true);
     };
-    pass(X, T, cx.R1.p, nullptr);
-    pass(T, X, cx.R2.p, nullptr);
+    pass(X, T, R[0], only_if, nullptr);
+    pass(T, X, R[1], only_if, loose);
     // pass 3 only after a shifted pass: X -> T -> X
     const int* cond = cx.shifted.p;
-    pass(X, T, cx.R3.p, cond);
+    pass(X, T, R[2], cond, nullptr);
     k_copy_cond<<<nb(rows * c, 256), 256, 0, s>>>(T, X, rows * c, cond);
     SVDB_CHECK_LAUNCH();
     if (Rout) {
         const int blocks = (c * c + 127) / 128;
-        k_small_gemm<<<blocks, 128, 0, s>>>(cx.R2.p, cx.R1.p, c, Rout, nullptr);
-        k_small_gemm<<<blocks, 128, 0, s>>>(cx.R3.p, Rout, c, cx.Rtmp.p, cond);
+        k_small_gemm<<<blocks, 128, 0, s>>>(R[1], R[0], c, Rout, nullptr);
+        k_small_gemm<<<blocks, 128, 0, s>>>(R[2], Rout, c, cx.Rtmp.p, cond);
         k_copy_cond<<<1, 256, 0, s>>>(cx.Rtmp.p, Rout, (int64_t)c * c, cond);
         SVDB_CHECK_LAUNCH_N(3);
     }
@@ -310,9 +484,10 @@ static void cholesky_qr(RandCtx& cx, double* X, int64_t rows, int c, double* Rou
 
 // qr(X).q() for X (rows x c): returns the column count of Q; X is replaced by
 // Q (rows x k, k = min(rows, c)) stored with row stride k.
-static int thin_q(RandCtx& cx, DevBuf<double>& X, int64_t rows, int c) {
+static int thin_q(RandCtx& cx, DevBuf<double>& X, int64_t rows, int c, const int* only_if = nullptr,
+                  int* loose = nullptr) {
     if (rows >= c) {
-        cholesky_qr(cx, X.p, rows, c, nullptr);
+        cholesky_qr(cx, X.p, rows, c, nullptr, only_if, loose);
         return c;
     }
     // wide: Q spans R^rows; take the leading rows x rows block's Q
@@ -320,7 +495,7 @@ static int thin_q(RandCtx& cx, DevBuf<double>& X, int64_t rows, int c) {
     DevBuf<double> Xk((int64_t)rows * k, cx.s);
     k_take_cols<<<nb(rows * k, 256), 256, 0, cx.s>>>(X.p, rows, c, k, Xk.p);
     SVDB_CHECK_LAUNCH();
-    cholesky_qr(cx, Xk.p, rows, k, nullptr);
+    cholesky_qr(cx, Xk.p, rows, k, nullptr, nullptr, loose);
     X = std::move(Xk);
     return k;
 }
@@ -370,9 +545,11 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
     RandCtx cx;
     cx.s = s;
     const int cmax = l;
-    for (DevBuf<double>* b : {&cx.G, &cx.R1, &cx.R2, &cx.R3, &cx.Ri, &cx.Rtmp}) b->alloc((size_t)cmax * cmax, s);
+    for (DevBuf<double>* b : {&cx.G, &cx.Ri, &cx.Rtmp}) b->alloc((size_t)cmax * cmax, s);
+    cx.R1.alloc((size_t)3 * cmax * cmax, s);
     cx.flags.alloc(1, s);
     cx.shifted.alloc(1, s);
+    cx.loose.alloc(1, s);
     DevBuf<int> jac_status(1, s);
     SVDB_CUDA(cudaMemsetAsync(cx.flags.p, 0, sizeof(int), s));
     SVDB_CUDA(cudaMemsetAsync(jac_status.p, 0, sizeof(int), s));
@@ -418,8 +595,8 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
         SVDB_CUDA(cudaEventRecord(b, s));
         spmm_events.emplace_back(a, b);
     };
-    auto normalize = [&](DevBuf<double>& X, int64_t rows, int c) -> int {
-        if (normalizer == SVDB_NORM_QR) return thin_q(cx, X, rows, c);
+    auto normalize = [&](DevBuf<double>& X, int64_t rows, int c, int* loose) -> int {
+        if (normalizer == SVDB_NORM_QR) return thin_q(cx, X, rows, c, nullptr, loose);
         if (normalizer == SVDB_NORM_LU) {
             k_colnorm<double><<<c, 256, 0, s>>>(X.p, rows, c);
             SVDB_CHECK_LAUNCH();
@@ -451,17 +628,21 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
         DevBuf<double> Z(std::max<int64_t>(n * c, 1), s);
         spmm(Acsc, Y.p, c, Z.p);
         center(Y.p, m, c, Z.p, n, false);
-        c = normalize(Z, n, c);
+        c = normalize(Z, n, c, nullptr);
         DevBuf<double> Y2(std::max<int64_t>(m * c, 1), s);
         spmm(Acsr, Z.p, c, Y2.p);
         center(Z.p, n, c, Y2.p, m, true);
         Y = std::move(Y2);
-        c = normalize(Y, m, c);
+        SVDB_CUDA(cudaMemsetAsync(cx.loose.p, 0, sizeof(int), s));
+        c = normalize(Y, m, c, cx.loose.p);
         if (verbose)
             printf("SVD | Randomized | Power Iteration Normalization Backward-Step %.3f ms\n", ms_since(t0));
     }
     if (verbose) printf("SVD | Randomized | Running QR-Normalization after Power-Iterations %.3f ms\n", ms_since(t0));
-    c = thin_q(cx, Y, m, c);  // Q = qr(y).q()
+    // Q = qr(y).q().  After a QR-normalised iteration y is its own Q unless that
+    // factorisation was a difficult one (cx.loose): nothing to do otherwise.
+    const bool q_done = normalizer == SVDB_NORM_QR && n_power_iters > 0 && m >= c;
+    c = thin_q(cx, Y, m, c, q_done ? cx.loose.p : nullptr);
     // B^T = A^T Q (n x c)
     DevBuf<double> Bt(std::max<int64_t>(n * c, 1), s);
     spmm(Acsc, Y.p, c, Bt.p);

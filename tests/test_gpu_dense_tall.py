@@ -61,3 +61,27 @@ def test_solve_widths(l, shape):
     np.testing.assert_allclose(g.s, r["s"], rtol=1e-10)
     k = len(g.s)
     assert np.abs(g.u.T @ g.u - np.eye(k)).max() < 1e-12 and np.abs(g.vt @ g.vt.T - np.eye(k)).max() < 1e-12
+
+
+@pytest.mark.parametrize("q", [0, 1, 3])
+@pytest.mark.parametrize("m", [900, 6000])
+@pytest.mark.parametrize("kind", ["deficient", "graded"])
+def test_difficult_factorisations(kind, m, q):
+    """Shifted passes and nearly dependent columns, in the one-cluster form
+    (900 x 64) and the launch-per-step one (6,000 x 64), with the factorisation
+    after the last power iteration skipped only where it may be: the leading
+    singular values against numpy's, and orthonormal leading vectors.  A has 30
+    singular values, equal-sized or spread over 1e-9: with 64 sample columns its
+    range is captured to rounding, u ||A|| sqrt(n) = 2e-15 ||A||, 1e-12 asked."""
+    n, k = 200, 30
+    rng = np.random.default_rng(m + q)
+    U, _ = np.linalg.qr(rng.standard_normal((m, k)))
+    V, _ = np.linalg.qr(rng.standard_normal((n, k)))
+    s = np.linspace(5.0, 3.0, k) if kind == "deficient" else 10.0 ** np.linspace(0, -9, k)
+    A = M.dense((U * s) @ V.T)
+    g = randomized.randomized_svd(upload("csr", A), 40, 24, q, randomized.PowerIterationNormalizer.QR, False, 3)
+    ref = np.linalg.svd(M.to_scipy(A).toarray(), compute_uv=False)
+    assert np.abs(g.s[:k] - ref[:k]).max() <= 1e-12 * ref[0]
+    lead = k if kind == "deficient" else 20  # those above 1e-6: the others' directions are rounding at 1e-9
+    u, vt = g.u[:, :lead], g.vt[:lead]
+    assert np.abs(u.T @ u - np.eye(lead)).max() < 1e-10 and np.abs(vt @ vt.T - np.eye(lead)).max() < 1e-10
