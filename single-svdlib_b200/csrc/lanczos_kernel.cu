@@ -26,7 +26,7 @@ constexpr int kClSlots = 16 * (kThreads / 32);  // cluster sums: blocks x warps
 __device__ __forceinline__ bool cmp_eq(double a, double b) { return fabs(b - a) < kEps; }
 
 // Row-gather SpMV over the rows of `op`: rows of more than kSegNnz entries
-// (op.long_rows) one block each, the others through the length bins
+// (the first of op.bins.rows) one block each, the others through the length bins
 // (spmv_binned, spmv.cuh).  SCALE: x is read as x * rinv (the dscal
 // of w3 folded in).  EPI: y = acc + (-rnm) * w2, and returns this thread's
 // share of dot(y, w3).  Only the matrix arrays are read through the
@@ -55,14 +55,14 @@ __device__ __forceinline__ double spmv_rows(const LzOperand& op, const double* x
         else sliced_rows<double, SCALE>(op.sl, op.sv, x, rinv, dyn, finish);
         return dotacc;
     }
-    for (int64_t i = blockIdx.x; i < op.nlong; i += gridDim.x) {
-        const int64_t r = __ldg(op.long_rows + i);
+    spmv_deal(blockIdx.x, gridDim.x, op.bins.off[0], [&](int64_t i) {  // uniform over the block
+        const int64_t r = __ldg(op.bins.rows + i);
         const int64_t s = __ldg(op.rp + r), e = __ldg(op.rp + r + 1);
         double acc = FP32 ? row_dot(op.ci, op.vf, s, e, (int)threadIdx.x, (int)blockDim.x, xl)
                           : row_dot(op.ci, op.v, s, e, (int)threadIdx.x, (int)blockDim.x, xl);
         acc = block_sum(acc, sh);
         if (threadIdx.x == 0) finish(r, acc);
-    }
+    });
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     if (FP32) spmv_binned(op.rp, op.ci, op.vf, op.bins, gwarp, nwarps, xl, finish);

@@ -28,9 +28,7 @@ struct LzOperand {
     const double* v;
     const float* vf;  // FP32 values (mixed precision) or null
     int64_t rows;
-    const int32_t* long_rows;  // rows of more than kSegNnz entries, one block each
-    int64_t nlong;
-    SpmvBins bins;             // the other rows, by length
+    SpmvBins bins;             // all rows, longest first
     // the column-sliced copy (sliced launches only, spmv.cuh): its values
     SlicedOp sl;
     const double* sv;

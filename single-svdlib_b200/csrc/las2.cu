@@ -412,9 +412,9 @@ int64_t Las2Run::lanczos_step(int64_t first, int64_t last, int64_t& ll, bool& en
         LzArgs a;
         std::memset(&a, 0, sizeof a);
         a.op1 = {op1_->ptr.p, op1_->idx.p, op1_->val.p, fp32_ ? op1_->val32.p : nullptr, op1_->nmajor,
-                 op1_->plan.long_rows.p, op1_->plan.nlong, op1_->plan.bins, SlicedOp{}, nullptr, nullptr};
+                 op1_->plan.bins, SlicedOp{}, nullptr, nullptr};
         a.op2 = {op2_->ptr.p, op2_->idx.p, op2_->val.p, fp32_ ? op2_->val32.p : nullptr, op2_->nmajor,
-                 op2_->plan.long_rows.p, op2_->plan.nlong, op2_->plan.bins, SlicedOp{}, nullptr, nullptr};
+                 op2_->plan.bins, SlicedOp{}, nullptr, nullptr};
         if (lz_sliced_) {
             a.op1.sl = sliced_view(*op1_);
             a.op1.sv = op1_->sliced.sval.p;

@@ -30,19 +30,30 @@ int group_for(double avg) {
 // kSegNnz entries (one block per row, the plan's long rows), then its warps
 // take the other rows through the length bins.  The grid is one wave of
 // resident blocks, so the two parts overlap and no partial wave trails.
+// Bound by the latency of the (index, x) chains, so by how many the warps keep
+// in flight.  A x and A^T x of a 200,000 x 40,000 operator with Zipf row
+// lengths (38 M, FP64 values) and A x in FP32 values: 244, 148 and 220 us with
+// the rows dealt in row order; dealt by length 157, 130 and 152 without a
+// bound on the blocks, 131, 124 and 111 compiled for five blocks an SM (48
+// registers in both types), 139, 133 and 117 for four, 161, 154 and 129 for
+// eight (spills).  Uniform 100,000 x 20,000 (20 M): 78 and 82 -> 60 and 73 us.
+// The last two arguments are unused and bring the arguments to 160 bytes.  A
+// small product is bound by the host's launches, and their cost went with the
+// arguments' size: 3.7-3.8 us per call at 160 and 224 bytes, 4.05 at 152,
+// 4.3-4.6 at 144, 176 and 192.
 template <typename VT>
-__global__ void __launch_bounds__(256) k_spmv(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
+__global__ void __launch_bounds__(256, 5) k_spmv(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                               const VT* __restrict__ v, const __grid_constant__ SpmvBins bins,
-                                              const int32_t* __restrict__ long_rows, int64_t nlong,
-                                              const double* __restrict__ x, double* __restrict__ y) {
+                                              const double* __restrict__ x, double* __restrict__ y, int64_t,
+                                              int64_t) {
     __shared__ double sh[32];
     auto xl = [&](int32_t c) { return __ldg(x + c); };
-    for (int64_t i = blockIdx.x; i < nlong; i += gridDim.x) {
-        const int64_t r = long_rows[i];
+    spmv_deal(blockIdx.x, gridDim.x, bins.off[0], [&](int64_t i) {
+        const int64_t r = __ldg(bins.rows + i);
         const double acc = row_dot(ci, v, rp[r], rp[r + 1], (int)threadIdx.x, (int)blockDim.x, xl);
         const double tot = block_sum(acc, sh);
         if (threadIdx.x == 0) y[r] = tot;
-    }
+    });
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     spmv_binned(rp, ci, v, bins, gwarp, nwarps, xl, [&](int64_t r, double acc) { y[r] = acc; });
@@ -76,15 +87,15 @@ void spmv(const DevCompressed& m, bool fp32, const double* x, double* y, cudaStr
     if (m.nmajor == 0) return;
     const bool f = fp32 && m.val32.p;
     if (allow_sliced && !sliced_off() && spmv_sliced(m, f, x, y, s)) return;
-    const int64_t work = std::max<int64_t>(m.plan.bins.items[kSpmvBins] / 8, m.plan.nlong);
+    // an item for every warp: a warp's second item lengthened a 5000 x 2000 product, whose chain of
+    // loads is all its time, from 2.7 to 3.6 us
+    const int64_t work = std::max<int64_t>((m.plan.bins.items[kSpmvBins] + 7) / 8, m.plan.nlong);
     if (f) {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<float>()));
-        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, m.plan.long_rows.p,
-                                             m.plan.nlong, x, y);
+        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, x, y, 0, 0);
     } else {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<double>()));
-        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, m.plan.long_rows.p,
-                                              m.plan.nlong, x, y);
+        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, x, y, 0, 0);
     }
     SVDB_CHECK_LAUNCH();
 }

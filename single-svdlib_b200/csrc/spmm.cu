@@ -321,7 +321,7 @@ __global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_
 __global__ void k_seg_fill(const int64_t* __restrict__ rp, const int64_t* __restrict__ first, int64_t rows,
                            int64_t seg, int32_t* __restrict__ seg_row, int64_t* __restrict__ seg_beg,
                            int64_t* __restrict__ seg_end, int32_t* __restrict__ multi_rows,
-                           int32_t* __restrict__ long_rows, unsigned long long* __restrict__ counts) {
+                           unsigned long long* __restrict__ counts) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t f = first[r], f1 = first[r + 1], e = rp[r + 1];
         const bool multi = f1 - f > 1;
@@ -331,26 +331,45 @@ __global__ void k_seg_fill(const int64_t* __restrict__ rp, const int64_t* __rest
             seg_beg[s] = a;
             seg_end[s] = (a + seg < e) ? a + seg : e;
         }
-        // the lists' order is irrelevant to the sums
+        // the list's order is irrelevant to the sums
         if (multi) multi_rows[atomicAdd(counts, 1ull)] = (int32_t)r;
-        if (e - rp[r] > kSegNnz) long_rows[atomicAdd(counts + 1, 1ull)] = (int32_t)r;
     }
 }
 
-// counts[2] = the most entries in one of 16 equal row ranges
+// counts[1] = the most entries in one of 16 equal row ranges
 __global__ void k_slice16(const int64_t* __restrict__ rp, int64_t rows, unsigned long long* __restrict__ counts) {
     const int64_t per = slice16_rows(rows);
     const int64_t r0 = min(rows, threadIdx.x * per), r1 = min(rows, r0 + per);
-    if (threadIdx.x < 16) atomicMax(counts + 2, (unsigned long long)(rp[r1] - rp[r0]));
+    if (threadIdx.x < 16) atomicMax(counts + 1, (unsigned long long)(rp[r1] - rp[r0]));
 }
 
-__global__ void k_bin_flags(const int64_t* __restrict__ rp, int64_t rows, int64_t lo, int64_t hi,
-                            uint8_t* __restrict__ flag, int32_t* __restrict__ ids) {
+// Sort key of a row's SpMV class, longest first, and counts[2 ..]: the rows
+// of more than kSegNnz entries, then those of each bin.  Above 64 entries a
+// class is a quarter octave of the length (by octaves A x of the Zipf operator
+// in k_spmv's comment took 136 us, against 130); below, one bin, so that rows
+// next to each other in memory, which share cache lines, stay together.
+constexpr int kSpmvKeyBits = 7;
+__global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, uint8_t* __restrict__ key,
+                            int32_t* __restrict__ ids, unsigned long long* __restrict__ counts) {
+    __shared__ unsigned int sc[kSpmvBins + 1];
+    if (threadIdx.x <= kSpmvBins) sc[threadIdx.x] = 0;
+    __syncthreads();
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t len = rp[r + 1] - rp[r];
-        flag[r] = (len > lo && len <= hi) ? 1 : 0;
+        int c = 0;  // 0: one block, c: bin c - 1
+        while (c < kSpmvBins && len <= spmv_bin_len(c)) ++c;
+        if (c < 2) {
+            const int e = min(63 - __clzll(len), 31);
+            key[r] = (uint8_t)(127 - 4 * e - (int)((len >> (e - 2)) & 3));
+        } else {
+            key[r] = (uint8_t)(104 + c);  // 65 entries: 103
+        }
         ids[r] = (int32_t)r;
+        atomicAdd(sc + c, 1u);
     }
+    __syncthreads();
+    if (threadIdx.x <= kSpmvBins && sc[threadIdx.x])
+        atomicAdd(counts + 2 + threadIdx.x, (unsigned long long)sc[threadIdx.x]);
 }
 
 static int nblk(int64_t work, int threads, int per_sm) {
@@ -383,43 +402,37 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.seg_beg.alloc(std::max<int64_t>(nseg, 1), s);
     p.seg_end.alloc(std::max<int64_t>(nseg, 1), s);
     p.multi_rows.alloc(std::max<int64_t>(rows, 1), s);
-    p.long_rows.alloc(std::max<int64_t>(m.nnz / kSegNnz, 1), s);
-    DevBuf<unsigned long long> nm(3, s);
-    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, 3 * sizeof(unsigned long long), s));
+    constexpr int kCounts = 3 + kSpmvBins;
+    DevBuf<unsigned long long> nm(kCounts, s);
+    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, kCounts * sizeof(unsigned long long), s));
     k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, seg, p.seg_row.p, p.seg_beg.p,
-                                                   p.seg_end.p, p.multi_rows.p, p.long_rows.p, nm.p);
+                                                   p.seg_end.p, p.multi_rows.p, nm.p);
     SVDB_CHECK_LAUNCH();
     if (m.nnz < ((int64_t)1 << 20)) {
         k_slice16<<<1, 32, 0, s>>>(m.ptr.p, rows, nm.p);
         SVDB_CHECK_LAUNCH();
     }
-    unsigned long long hm[3] = {0, 0, 0};
+    // SpMV order: the rows' length classes, longest first, by one stable sort
+    p.bin_rows.alloc(rows, s);
+    DevBuf<uint8_t> key(rows, s), skey(rows, s);
+    DevBuf<int32_t> ids(rows, s);
+    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, key.p, ids.p, nm.p);
+    SVDB_CHECK_LAUNCH();
+    size_t tb2 = 0;
+    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb2, key.p, skey.p, ids.p, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
+    DevBuf<uint8_t> tmp2(std::max<size_t>(tb2, 1), s);
+    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(tmp2.p, tb2, key.p, skey.p, ids.p, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
+    unsigned long long hm[kCounts];
     SVDB_CUDA(cudaMemcpyAsync(hm, nm.p, sizeof(hm), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
     p.nmulti = (int64_t)hm[0];
-    p.nlong = (int64_t)hm[1];
-    p.slice16_nnz = (int64_t)hm[2];
-
-    // SpMV bins: a stable partition of the rows by length
-    p.bin_rows.alloc(std::max<int64_t>(rows, 1), s);
-    DevBuf<uint8_t> flag(rows, s);
-    DevBuf<int32_t> ids(rows, s);
-    DevBuf<int64_t> nsel(1, s);
-    size_t tb2 = 0;
-    SVDB_CUDA(cub::DeviceSelect::Flagged(nullptr, tb2, ids.p, flag.p, p.bin_rows.p, nsel.p, rows, s));
-    DevBuf<uint8_t> tmp2(std::max<size_t>(tb2, 1), s);
-    int64_t off = 0, items = 0;
+    p.slice16_nnz = (int64_t)hm[1];
+    p.nlong = (int64_t)hm[2];
+    int64_t off = p.nlong, items = 0;
     for (int b = 0; b < kSpmvBins; ++b) {
-        const int64_t lo = b ? kSpmvBinLen[b - 1] : -1, hi = kSpmvBinLen[b];
-        k_bin_flags<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, lo, hi, flag.p, ids.p);
-        SVDB_CHECK_LAUNCH();
-        SVDB_CUDA(cub::DeviceSelect::Flagged(tmp2.p, tb2, ids.p, flag.p, p.bin_rows.p + off, nsel.p, rows, s));
-        int64_t cnt = 0;
-        SVDB_CUDA(cudaMemcpyAsync(&cnt, nsel.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
-        SVDB_CUDA(cudaStreamSynchronize(s));
+        const int64_t cnt = (int64_t)hm[3 + b], rpw = (int64_t)1 << b;
         p.bins.off[b] = off;
         p.bins.items[b] = items;
-        const int64_t rpw = 32 / (2 << b);
         off += cnt;
         items += (cnt + rpw - 1) / rpw;
     }

@@ -94,18 +94,19 @@ struct DevBuf {
 // seg_row[s], stored as -(row + 1) when the row has several segments; those
 // rows are listed in multi_rows and merged by a second, ordered pass.
 constexpr int64_t kSegNnz = 2048;
-// SpMV row bins: bin b (< kSpmvBins) holds the rows of at most
-// kSpmvBinLen[b] entries (and more than kSpmvBinLen[b-1]), ascending, taken
-// by groups of (2 << b) lanes; rows of more than kSegNnz entries are
-// long_rows, one block each.
 // Rows of one of the 16 equal ranges slice16_nnz is counted over (even).
 __host__ __device__ inline int64_t slice16_rows(int64_t rows) { return ((rows + 15) / 16 + 1) / 2 * 2; }
+// SpMV row order: all rows, longest class first (a quarter octave of the length
+// above 64 entries, one bin below), ascending inside a class.  The first nlong
+// have more than kSegNnz entries and are taken by one block each.  Bin b
+// (< kSpmvBins) holds the rows of at most spmv_bin_len(b) entries (and more
+// than the next bin's), taken by groups of 32 >> b lanes.
 constexpr int kSpmvBins = 5;
-constexpr int64_t kSpmvBinLen[kSpmvBins] = {8, 16, 32, 64, kSegNnz};
+__host__ __device__ constexpr int64_t spmv_bin_len(int b) { return b ? 128 >> b : kSegNnz; }
 struct SpmvBins {
     const int32_t* rows;             // bin_rows
-    int64_t off[kSpmvBins + 1];      // bin b: rows[off[b] .. off[b+1])
-    int64_t items[kSpmvBins + 1];    // warp items before bin b (32 / (2 << b) rows per item)
+    int64_t off[kSpmvBins + 1];      // bin b: rows[off[b] .. off[b+1]); off[0] = nlong
+    int64_t items[kSpmvBins + 1];    // warp items before bin b (1 << b rows per item)
 };
 struct SegPlan {
     int64_t nseg = 0, nmulti = 0, nlong = 0;
@@ -115,7 +116,7 @@ struct SegPlan {
     DevBuf<int64_t> seg_first;
     DevBuf<int32_t> seg_row;
     DevBuf<int64_t> seg_beg, seg_end;
-    DevBuf<int32_t> multi_rows, long_rows;
+    DevBuf<int32_t> multi_rows;
 };
 
 // Panel plan of the FP32 SpMM (spmm_panel.cu), built on first use.  Rows
