@@ -386,14 +386,34 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
         p.nseg = p.nmulti = p.nlong = 0;
         return;
     }
-    DevBuf<int64_t> cnt(rows + 1, s);
     const int64_t seg = seg_len_for(m.nnz);
-    k_seg_count<<<nblk(rows + 1, 256, 16), 256, 0, s>>>(m.ptr.p, rows, seg, cnt.p);
+    p.multi_rows.alloc(rows, s);
+    p.bin_rows.alloc(rows, s);
+    // One scratch allocation for all temporaries: an allocation takes 10-25 us
+    // where the pool's free blocks belong to other streams.
+    constexpr int kCounts = 3 + kSpmvBins;
+    size_t tb = 0, tb2 = 0;
+    SVDB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int64_t*)nullptr, p.seg_first.p, rows + 1, s));
+    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb2, (uint8_t*)nullptr, (uint8_t*)nullptr, (int32_t*)nullptr,
+                                              p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
+    size_t bytes = 0;
+    auto piece = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t o_cnt = piece((rows + 1) * sizeof(int64_t)), o_nm = piece(kCounts * sizeof(unsigned long long)),
+                 o_key = piece(rows), o_skey = piece(rows), o_ids = piece(rows * sizeof(int32_t)),
+                 o_cub = piece(std::max(tb, tb2));
+    DevBuf<uint8_t> scratch(bytes, s);
+    int64_t* cnt = reinterpret_cast<int64_t*>(scratch.p + o_cnt);
+    unsigned long long* nm = reinterpret_cast<unsigned long long*>(scratch.p + o_nm);
+    uint8_t *key = scratch.p + o_key, *skey = scratch.p + o_skey, *cub_tmp = scratch.p + o_cub;
+    int32_t* ids = reinterpret_cast<int32_t*>(scratch.p + o_ids);
+
+    k_seg_count<<<nblk(rows + 1, 256, 16), 256, 0, s>>>(m.ptr.p, rows, seg, cnt);
     SVDB_CHECK_LAUNCH();
-    size_t tb = 0;
-    SVDB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.p, p.seg_first.p, rows + 1, s));
-    DevBuf<uint8_t> tmp(std::max<size_t>(tb, 1), s);
-    SVDB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt.p, p.seg_first.p, rows + 1, s));
+    SVDB_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, tb, cnt, p.seg_first.p, rows + 1, s));
     int64_t nseg = 0;
     SVDB_CUDA(cudaMemcpyAsync(&nseg, p.seg_first.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
@@ -401,29 +421,20 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.seg_row.alloc(std::max<int64_t>(nseg, 1), s);
     p.seg_beg.alloc(std::max<int64_t>(nseg, 1), s);
     p.seg_end.alloc(std::max<int64_t>(nseg, 1), s);
-    p.multi_rows.alloc(std::max<int64_t>(rows, 1), s);
-    constexpr int kCounts = 3 + kSpmvBins;
-    DevBuf<unsigned long long> nm(kCounts, s);
-    SVDB_CUDA(cudaMemsetAsync(nm.p, 0, kCounts * sizeof(unsigned long long), s));
+    SVDB_CUDA(cudaMemsetAsync(nm, 0, kCounts * sizeof(unsigned long long), s));
     k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, seg, p.seg_row.p, p.seg_beg.p,
-                                                   p.seg_end.p, p.multi_rows.p, nm.p);
+                                                   p.seg_end.p, p.multi_rows.p, nm);
     SVDB_CHECK_LAUNCH();
     if (m.nnz < ((int64_t)1 << 20)) {
-        k_slice16<<<1, 32, 0, s>>>(m.ptr.p, rows, nm.p);
+        k_slice16<<<1, 32, 0, s>>>(m.ptr.p, rows, nm);
         SVDB_CHECK_LAUNCH();
     }
     // SpMV order: the rows' length classes, longest first, by one stable sort
-    p.bin_rows.alloc(rows, s);
-    DevBuf<uint8_t> key(rows, s), skey(rows, s);
-    DevBuf<int32_t> ids(rows, s);
-    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, key.p, ids.p, nm.p);
+    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, key, ids, nm);
     SVDB_CHECK_LAUNCH();
-    size_t tb2 = 0;
-    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb2, key.p, skey.p, ids.p, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
-    DevBuf<uint8_t> tmp2(std::max<size_t>(tb2, 1), s);
-    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(tmp2.p, tb2, key.p, skey.p, ids.p, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
+    SVDB_CUDA(cub::DeviceRadixSort::SortPairs(cub_tmp, tb2, key, skey, ids, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
     unsigned long long hm[kCounts];
-    SVDB_CUDA(cudaMemcpyAsync(hm, nm.p, sizeof(hm), cudaMemcpyDeviceToHost, s));
+    SVDB_CUDA(cudaMemcpyAsync(hm, nm, sizeof(hm), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
     p.nmulti = (int64_t)hm[0];
     p.slice16_nnz = (int64_t)hm[1];
