@@ -1219,7 +1219,7 @@ def main():
             "sigma_rel_err_vs_oracle": sig_oracle,
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                          "traffic": profiled_traffic("spmm_f32_randomized_100kx30k.md"), "kernel": dominant,
-                         "kernel_name": "k_spmm_f32", "peak_source": peak_kind, "l2_row_gathers": gather,
+                         "kernel_name": "k_spmm_lean<float>", "peak_source": peak_kind, "l2_row_gathers": gather,
                          "spmm_csr_AZ": {"ms": ms_ax, "gbs": gbs_ax, "bytes": bytes_ax},
                          "spmm_csc_AtY": {"ms": ms_atx, "gbs": gbs_atx, "bytes": bytes_atx}},
             "cpu_baseline": cpu,

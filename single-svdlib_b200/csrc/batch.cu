@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) k_b_spmm_cols(const int64_t* __restrict__
 
 // ------------------------------------------------- lean batch products ----
 // The products of an SVDB_MIXED batch (FP32 values and dense operands, l a
-// multiple of 4 up to 64) with the instruction stream of k_spmm_f32: a
+// multiple of 4 up to 64) with the instruction stream of k_spmm_lean: a
 // chunk's 32 entries are loaded by the warp one chunk ahead, the entries
 // that count are staged once in a per-warp shared buffer as (row offset,
 // value) and read back by broadcast, lane groups of 32 / H lanes take every
