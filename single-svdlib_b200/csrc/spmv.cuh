@@ -50,7 +50,7 @@ __device__ __forceinline__ double row_dot(const int32_t* __restrict__ ci, const 
 // nonzeros) left SMs busy for 286,000 to 478,000 of 490,000 cycles: A x 244 us,
 // against 157 in this order (131 as k_spmv is compiled).  Two rounds at most go
 // forwards: the second one's items then fall to the blocks that started first
-// (20,000 x 5,000, 30 a row, 1.2 rounds: 4.3 us, backwards 5.2).
+// (20,000 x 5,000, 30 a row, 1.2 rounds: 4.4 us, backwards 5.2).
 template <typename F>
 __device__ __forceinline__ void spmv_deal(int64_t w, int64_t n, int64_t total, F f) {
     int64_t step = total > 2 * n ? 2 * (n - w) - 1 : n;
