@@ -334,6 +334,15 @@ int svdb_dense_split_info(const svdb_matrix* a, uint64_t* dense_cols, uint64_t* 
 
 /* Number of kernels this library has launched in the process so far. */
 uint64_t svdb_kernel_launches(void);
+/* How the calling thread's last LAS2 run launched its Lanczos blocks. */
+enum svdb_lanczos_form_t {
+    SVDB_LZ_NONE = 0,     /* none has run */
+    SVDB_LZ_GRID = 1,     /* cooperative grid */
+    SVDB_LZ_SLICED = 2,   /* cooperative grid, column-sliced operands */
+    SVDB_LZ_CLUSTER = 3,  /* one thread-block cluster, operands in global memory */
+    SVDB_LZ_RESIDENT = 4  /* one cluster, operands in its shared memory */
+};
+int svdb_lanczos_form(void);
 
 /* ---- LAS2 (src/lanczos/mod.rs) ---- */
 

@@ -17,6 +17,7 @@ void masked_maps(const svdb_matrix*, int64_t*, int64_t*);
 void destroy(svdb_matrix*);
 void las2(const svdb_matrix*, uint64_t, uint64_t, const double[2], double, uint32_t, bool, const svdb_options&,
           svdb_rec*, bool);
+int lanczos_form();
 int las2_plan(uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t*, uint64_t*, int32_t*, int32_t*);
 void randomized(const svdb_matrix*, uint64_t, uint64_t, uint64_t, int, int, int, uint64_t, int,
                 const svdb_options&, svdb_rec*, bool);
@@ -294,6 +295,7 @@ int svdb_multiply_with_dense_device(const svdb_matrix* a, const void* d_dense, u
 }
 
 uint64_t svdb_kernel_launches(void) { return g_launches.load(); }
+int svdb_lanczos_form(void) { return lanczos_form(); }
 
 int svdb_sliced_spmv_info(const svdb_matrix* a, int transposed, int32_t* nslices, int32_t* nranges) {
     return guarded([&] {

@@ -794,12 +794,11 @@ bool lanczos_cluster_ok(int cluster, int threads) {
 // (the kernels' static shared memory is below 8 KB)
 size_t lanczos_resident_smem() { return device_props().smem_optin > 8192 ? device_props().smem_optin - 8192 : 0; }
 
-bool lanczos_resident_ok(size_t smem, int threads) {
-    if (smem > lanczos_resident_smem()) return false;
+bool lanczos_resident_ok(int threads) {
+    const size_t smem = lanczos_resident_smem();  // what a launch may grow to with its coefficients
     auto fits = [&](auto kern) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lanczos_resident_smem()) !=
-                cudaSuccess) {
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }

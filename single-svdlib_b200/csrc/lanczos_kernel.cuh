@@ -35,34 +35,6 @@ struct LzOperand {
     const float* svf;
 };
 
-// Cluster launches on small operators keep both matrices in the CTAs' shared
-// memory: CTA c owns rows [c rows_c, (c + 1) rows_c) of each operand, with
-// 16-bit column indices, at most max_nnz entries; g lanes take a row.
-constexpr int kLzResCluster = 16;
-struct LzResident {
-    int on;
-    int rows_c[2], max_nnz[2], g[2];
-    int n, m;  // doubles of the two gathered vectors' copies (w3, temp)
-    int coef;  // doubles of each of alpha, beta and the two eta in block 0 (0: they stay in global memory)
-};
-// offsets (bytes) of the shared arrays; `bytes` in all
-struct LzResLayout {
-    size_t xa, xb, y, coef, rp[2], v[2], ci[2], bytes;
-};
-__host__ __device__ inline LzResLayout lz_res_layout(const LzResident& r, int value_bytes) {
-    LzResLayout L;
-    size_t o = 0;
-    L.xa = o; o += (size_t)(r.n + 1) / 2 * 16;
-    L.xb = o; o += (size_t)(r.m + 1) / 2 * 16;
-    L.coef = o; o += (size_t)r.coef * 32;
-    L.y = o; o += (size_t)(r.rows_c[0] > r.rows_c[1] ? r.rows_c[0] : r.rows_c[1]) * 8;
-    for (int k = 0; k < 2; ++k) { L.v[k] = o; o += ((size_t)r.max_nnz[k] * value_bytes + 7) / 8 * 8; }
-    for (int k = 0; k < 2; ++k) { L.rp[k] = o; o += (size_t)(r.rows_c[k] + 2) / 2 * 8; }
-    for (int k = 0; k < 2; ++k) { L.ci[k] = o; o += ((size_t)r.max_nnz[k] * 2 + 7) / 8 * 8; }
-    L.bytes = o;
-    return L;
-}
-
 struct LzArgs {
     LzOperand op1;     // temp = op1 x  (rows: internal nrows)
     LzOperand op2;     // y = op2 temp  (rows: n)
@@ -99,8 +71,8 @@ bool sliced_prepare(const DevCompressed& m, bool fp32, cudaStream_t s);
 SlicedOp sliced_view(const DevCompressed& m);
 int lanczos_max_blocks(int threads);
 bool lanczos_cluster_ok(int cluster, int threads);
-// Whether a resident cluster launch (a.res) with `smem` bytes of shared memory per CTA can run.
-bool lanczos_resident_ok(size_t smem, int threads);
+// Whether resident cluster launches (a.res) of up to lanczos_resident_smem() bytes a CTA can run.
+bool lanczos_resident_ok(int threads);
 size_t lanczos_resident_smem();  // most dynamic shared memory of such a CTA
 
 }  // namespace svdb

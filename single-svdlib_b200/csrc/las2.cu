@@ -51,7 +51,9 @@ static void insert_sort(size_t n, double* a1, double* a2) {
 // cluster of 2 * kLzCluster blocks where the device allows it, else of
 // kLzCluster (the portable size).
 constexpr int kLzCluster = 8;
-constexpr int64_t kLzClusterNnz = 1 << 20;
+
+static thread_local int g_lanczos_form = SVDB_LZ_NONE;  // of this thread's last run
+int lanczos_form() { return g_lanczos_form; }
 
 struct Mode {
     bool legacy = false;
@@ -708,29 +710,15 @@ void Las2Run::run(int64_t dimensions, int64_t iterations, double endl, double en
                 if (lanczos_cluster_ok(c, 512)) { lz_cluster_ = c; break; }
         }
         if (lz_cluster_) lz_blocks_ = lz_cluster_;
-        // Both operands in the cluster's shared memory where they fit: one
-        // element of every vector per thread (n <= 16 x 512), 16-bit column
-        // indices, and each CTA's slices beside the gathered vector
+        // Both operands in the cluster's shared memory where they fit
         // (SVDB_LZ_CLUSTER=2 keeps the operands in global memory).
         lz_res_.on = 0;
-        if (lz_cluster_ == kLzResCluster && !(env && atoi(env) == 2) && n_ > 0 && n_ <= kLzResCluster * 512 &&
-            op1_->nmajor <= 65535 && op1_->plan.slice16_nnz + op2_->plan.slice16_nnz < 65536) {
-            LzResident r{};
-            const DevCompressed* ops[2] = {op1_, op2_};
-            for (int k = 0; k < 2; ++k) {
-                r.rows_c[k] = (int)slice16_rows(ops[k]->nmajor);
-                r.max_nnz[k] = (int)ops[k]->plan.slice16_nnz;
-                r.g[k] = 2;  // lanes per row: about six entries each, eight in flight
-                while (r.g[k] < 32 && 6.5 * r.g[k] < ops[k]->avg_per_major()) r.g[k] *= 2;
-            }
-            r.n = (int)n_;
-            r.m = (int)op1_->nmajor;
-            const size_t smem = lz_res_layout(r, fp32_ ? 4 : 8).bytes;
-            if (lanczos_resident_ok(smem, 512)) {
-                r.on = 1;
-                lz_res_ = r;
-            }
-        }
+        const LzResOperand ops[2] = {{op1_->nmajor, op1_->nnz, op1_->plan.slice16_nnz},
+                                     {op2_->nmajor, op2_->nnz, op2_->plan.slice16_nnz}};
+        LzResident r{};
+        if (lz_cluster_ == kLzResCluster && !(env && atoi(env) == 2) &&
+            lz_resident_plan(ops, n_, 512, fp32_ ? 4 : 8, lanczos_resident_smem(), r) && lanczos_resident_ok(512))
+            lz_res_ = r;
     }
     // Large operators in grid mode: x slices in shared memory for both
     // products (spmv_sliced.cu), one block per SM (SVDB_SPMV=gather keeps the
@@ -746,6 +734,10 @@ void Las2Run::run(int64_t dimensions, int64_t iterations, double endl, double en
             }
         }
     }
+    g_lanczos_form = lz_res_.on    ? SVDB_LZ_RESIDENT
+                     : lz_cluster_ ? SVDB_LZ_CLUSTER
+                     : lz_sliced_  ? SVDB_LZ_SLICED
+                                   : SVDB_LZ_GRID;
     const int64_t nsplit_max = (n_ + 2047) / 2048;
     part_cap_ = std::max<int64_t>({2 * (int64_t)lz_blocks_, 2 * cap * nsplit_max, 2 * cap});
     part_.alloc(part_cap_, s_);

@@ -425,7 +425,8 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     k_seg_fill<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, p.seg_first.p, rows, seg, p.seg_row.p, p.seg_beg.p,
                                                    p.seg_end.p, p.multi_rows.p, nm);
     SVDB_CHECK_LAUNCH();
-    if (m.nnz < ((int64_t)1 << 20)) {
+    const bool slices = slice16_counted(m.nnz);
+    if (slices) {
         k_slice16<<<1, 32, 0, s>>>(m.ptr.p, rows, nm);
         SVDB_CHECK_LAUNCH();
     }
@@ -437,7 +438,7 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     SVDB_CUDA(cudaMemcpyAsync(hm, nm, sizeof(hm), cudaMemcpyDeviceToHost, s));
     SVDB_CUDA(cudaStreamSynchronize(s));
     p.nmulti = (int64_t)hm[0];
-    p.slice16_nnz = (int64_t)hm[1];
+    p.slice16_nnz = slices ? (int64_t)hm[1] : kSlice16Unknown;
     p.nlong = (int64_t)hm[2];
     int64_t off = p.nlong, items = 0;
     for (int b = 0; b < kSpmvBins; ++b) {

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/svdb200.h"
+#include "lz_resident.h"
 
 namespace svdb {
 
@@ -94,8 +95,6 @@ struct DevBuf {
 // seg_row[s], stored as -(row + 1) when the row has several segments; those
 // rows are listed in multi_rows and merged by a second, ordered pass.
 constexpr int64_t kSegNnz = 2048;
-// Rows of one of the 16 equal ranges slice16_nnz is counted over (even).
-__host__ __device__ inline int64_t slice16_rows(int64_t rows) { return ((rows + 15) / 16 + 1) / 2 * 2; }
 // SpMV row order: all rows, longest class first (a quarter octave of the length
 // above 64 entries, one bin below), ascending inside a class.  The first nlong
 // have more than kSegNnz entries and are taken by one block each.  Bin b
@@ -110,7 +109,7 @@ struct SpmvBins {
 };
 struct SegPlan {
     int64_t nseg = 0, nmulti = 0, nlong = 0;
-    int64_t slice16_nnz = 0;  // most entries in one of 16 equal row ranges (structures below 2^20 nonzeros)
+    int64_t slice16_nnz = kSlice16Unknown;  // most entries in one of 16 equal row ranges (lz_resident.h)
     DevBuf<int32_t> bin_rows;
     SpmvBins bins{};
     DevBuf<int64_t> seg_first;

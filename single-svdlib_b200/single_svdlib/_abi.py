@@ -116,6 +116,7 @@ SIGNATURES = {
     "svdb_release_cached_memory": (C.c_int, []),
     "svdb_gram_device": (C.c_int, [vp, u64, u64, vp, C.c_int, vp]),
     "svdb_kernel_launches": (u64, []),
+    "svdb_lanczos_form": (C.c_int, []),
     "svdb_wait_selftest": (C.c_int, [C.c_int, u64]),
     "svdb_dense_split_info": (C.c_int, [vp, P(u64), P(u64)]),
     "svdb_sliced_spmv_info": (C.c_int, [vp, C.c_int, P(i32), P(i32)]),

@@ -73,7 +73,7 @@ def las2_traced(a, dimensions=0, iterations=0, end_interval=(-1.0e-30, 1.0e-30),
                 algorithm="lanczos", precision="f64"):
     """Run LAS2 and return its internals with the result:
     {"rec": SvdRec or None, "error": SvdLibError or None, "alf", "bet", "ritz", "bnd", "steps",
-     "purges", "sparsity_branch", "lanczos_blocks"}."""
+     "purges", "sparsity_branch", "lanczos_blocks", "lanczos_form"}."""
     a = as_smat(a)
     cap = min(a.nrows(), a.ncols()) + 4
     bufs = {k: np.zeros(cap) for k in ("alf", "bet", "ritz", "bnd")}
@@ -93,5 +93,6 @@ def las2_traced(a, dimensions=0, iterations=0, end_interval=(-1.0e-30, 1.0e-30),
     out.update({"alf": bufs["alf"][: st + 1].copy(), "bet": bufs["bet"][: st + 2].copy(),
                 "ritz": bufs["ritz"][: st + 1].copy(), "bnd": bufs["bnd"][: st + 1].copy(), "steps": st,
                 "purges": int(tr.purges), "sparsity_branch": int(tr.sparsity_branch),
-                "lanczos_blocks": int(tr.lanczos_blocks)})
+                "lanczos_blocks": int(tr.lanczos_blocks),
+                "lanczos_form": ("none", "grid", "sliced", "cluster", "resident")[_abi.lib().svdb_lanczos_form()]})
     return out
