@@ -290,7 +290,8 @@ __global__ void __launch_bounds__(kThreads, (CL || SL) ? 1 : 2) k_lanczos_block(
             l_etaA = c + 2 * a.res.coef;
             l_etaB = c + 3 * a.res.coef;
         }
-        __syncthreads();
+        // the copies above, and every CTA has started: the first step stores into all of them
+        cg::this_cluster().sync();
     }
     auto put_back = [&] {
         if constexpr (RES) {
