@@ -9,6 +9,7 @@
 
 #include "dense_tall.cuh"
 #include "device_common.cuh"
+#include "qr_loose.h"
 
 namespace svdb {
 
@@ -66,9 +67,7 @@ __device__ __forceinline__ double omega_value(uint64_t key, int64_t i) {
 // G: c x c, or with nparts > 0 the sum of nparts such matrices, in order (only
 // the tiles on and above the diagonal are read).  c <= 128; blockDim.x a
 // multiple of 32, at least 160.  sm: chol_smem(c) bytes.  loose (may be null) is
-// set when an entry of G is more than 0.1 from the identity's, or on a shift: an
-// X with a G closer than that has kappa below 2, so X R^-1 is orthonormal to
-// rounding.
+// set when ||G - I||_F > 0.5 (qr_loose.h), or on a shift.
 __host__ __device__ inline int chol_ld(int c) { return ((c + 7) / 8 + 1) * 8 + 4; }  // = 4 or 12 mod 16: no conflicts
 __host__ __device__ inline size_t chol_smem(int c) {
     const int nt = (c + 7) / 8;
@@ -79,7 +78,7 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
                                               int* __restrict__ flags, int* __restrict__ shifted, double* sm,
                                               int* __restrict__ loose = nullptr) {
     __shared__ int s_fail;
-    __shared__ double s_inv[8], s_shift;
+    __shared__ double s_inv[8], s_shift, s_dev[32];
     const int nt = (c + 7) / 8, c8 = nt * 8, ld = chol_ld(c), cc = c * c;
     double* const rp = sm + (size_t)c8 * ld;  // the panel's rows of R (8 x ld)
     double* const dg = rp + 8 * ld;           // the factored diagonal tiles, unscaled
@@ -99,6 +98,7 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
     };
     double shift = 0.0;
     for (int attempt = 0;; ++attempt) {
+        double dev = 0.0;  // this thread's share of ||G - I||_F^2
         for (int i = warp; i < c8; i += nw) {
             const int i8 = i & ~7;
             for (int j = lane; j < i8; j += 32) sm[i * ld + j] = 0.0;
@@ -106,14 +106,23 @@ __device__ __forceinline__ void chol_inv_body(const double* __restrict__ G, int 
                 double v = i == j ? 1.0 : 0.0;
                 if (i < c && j < c) {
                     const double g = g_at(i, j);
-                    if (loose && !(fabs(g - v) <= 0.1)) *loose = 1;
+                    dev += loose_term(g, i, j);
                     v = g + (i == j ? shift : 0.0);
                 }
                 sm[i * ld + 8 + j] = v;
             }
         }
+        if (loose && attempt == 0) {
+            dev = warp_sum(dev);
+            if (lane == 0) s_dev[warp] = dev;
+        }
         if (threadIdx.x == 0) s_fail = 0;
         __syncthreads();
+        if (loose && attempt == 0 && threadIdx.x == 0) {
+            double t = 0.0;
+            for (int w = 0; w < nw; ++w) t += s_dev[w];
+            if (is_loose(t)) *loose = 1;
+        }
         bool failed = false;
         for (int K = 0; K < nt; ++K) {
             if (warp * 32 < c8 + 8) {
