@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_b_gram_part(con
                                                         double* __restrict__ part, const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
-    extern __shared__ double bg_sm[];
+    extern __shared__ __align__(16) double bg_sm[];
     const int64_t rows = sub_rows(L, coff, b), step = rg > 1 ? 4 * rg : 1;
     const int64_t chunk = ((rows + gridDim.x - 1) / gridDim.x + step - 1) / step * step;
     const int64_t r0 = blockIdx.x * chunk;
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(384) k_b_chol_inv(const double* __restrict__ G
                              int* __restrict__ shifted, const int* __restrict__ cond) {
     const int64_t b = blockIdx.x;
     if (cond && cond[b] == 0) return;
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     const int64_t rows = sub_rows(L, coff, b);
     const double shift_scale = 11.0 * ((double)rows * c + (double)c * (c + 1)) * 1.1102230246251565e-16;
     const int64_t cc = (int64_t)c * c;
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(32 * kNnWarps, 2) k_b_right_mul(const TI* X, S
                                                                   const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
     if (cond && cond[b] == 0) return;
-    extern __shared__ double br_sm[];
+    extern __shared__ __align__(16) double br_sm[];
     const int64_t rows = sub_rows(L, coff, b), row0 = sub_row0(L, coff, b);
     if ((int64_t)blockIdx.x * kNnWarps * 8 * kNnMT >= rows) return;
     const NnArgs<TI, TO> A{X + row0 * ldx, ldx, rows, c, S + b * (int64_t)c * c, c, nullptr, cout, upper, 1.0, nullptr,
@@ -730,7 +730,7 @@ __global__ void k_b_colnorm(T* __restrict__ X, SubLayout L, const int64_t* __res
 __global__ void __launch_bounds__(256) k_b_jacobi(const double* __restrict__ R, int c, double* __restrict__ U,
                                                   double* __restrict__ V, double* __restrict__ sig,
                                                   int* __restrict__ status) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     const int64_t b = blockIdx.x;
     const int64_t cc = (int64_t)c * c;
     jacobi_svd_body<false>(R + b * cc, false, c, U + b * cc, V + b * cc, sig + b * c, status + b, sm);

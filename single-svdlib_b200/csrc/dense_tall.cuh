@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(512, 1) k_tn_part(const TX* __restrict__ X, in
                                                     int64_t chunk, int nbp, int nbq, int sym, int rg,
                                                     double* __restrict__ part, const int* __restrict__ cond) {
     if (cond && *cond == 0) return;
-    extern __shared__ double tn_sm[];
+    extern __shared__ __align__(16) double tn_sm[];
     const int64_t r0 = blockIdx.x * chunk;
     tn_part_body<TX, TY, NT>(X, ldx, p, Y, ldy, q, r0, std::min<int64_t>(rows, r0 + chunk), nbp, nbq, sym != 0, rg,
                              part + (int64_t)blockIdx.x * p * q, tn_sm);
@@ -385,7 +385,7 @@ __device__ __forceinline__ void nn_body(const NnArgs<TX, TO>& A, int64_t g0, int
 template <typename TX, typename TO, int NQ, int DOT>
 __global__ void __launch_bounds__(32 * kNnWarps, 2) k_nn(const __grid_constant__ NnArgs<TX, TO> A) {
     if (A.cond && *A.cond == 0) return;
-    extern __shared__ double nn_sm[];
+    extern __shared__ __align__(16) double nn_sm[];
     nn_body<TX, TO, NQ, DOT>(A, (int64_t)blockIdx.x * kNnWarps + (threadIdx.x >> 5), (int64_t)gridDim.x * kNnWarps,
                              (int)blockIdx.y * NQ * 8, nn_sm);
 }

@@ -184,7 +184,7 @@ __device__ __forceinline__ void res_rows(const int* rp, const uint16_t* ci, cons
 // products 4.9, gathering temp 2.5, eta and the purge test 1.7.
 template <bool FP32, bool CL, bool SL = false, bool RES = false>
 __global__ void __launch_bounds__(kThreads, (CL || SL) ? 1 : 2) k_lanczos_block(const __grid_constant__ LzArgs a) {
-    extern __shared__ double lz_dyn[];  // SL: the x slice and the row accumulators; RES: lz_res_layout
+    extern __shared__ __align__(16) double lz_dyn[];  // SL: the x slice and the row accumulators; RES: lz_res_layout
     __shared__ double sh[32];
     __shared__ double cl_slot[CL ? 2 * kClSlots : 1];
     __shared__ int cl_flag;

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(384) k_chol_inv(const double* __restrict__ G, 
                                                   int* __restrict__ flags, int* __restrict__ shifted,
                                                   const int* __restrict__ cond, int* __restrict__ loose) {
     if (cond && *cond == 0) return;
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     chol_inv_body(G, nparts, c, shift_scale, R, Ri, flags, shifted, sm, loose);
 }
 
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kQrThreads, 1) k_cholqr_cluster(double* X, int
                                                                   double shift_scale, double* Rw, double* Rout,
                                                                   int* flags, const int* cond, int* loose) {
     if (cond && *cond == 0) return;  // the same for every CTA
-    extern __shared__ double qr_sm[];
+    extern __shared__ __align__(16) double qr_sm[];
     __shared__ int s_shifted, s_loose;
     cg::cluster_group cl = cg::this_cluster();
     const QrLayout L = qr_layout(c);
@@ -200,14 +200,14 @@ __global__ void k_colnorm(T* __restrict__ X, int64_t rows, int c) {
 __global__ void __launch_bounds__(960) k_jacobi_svd(const double* __restrict__ R, int trans, int c,
                                                      double* __restrict__ U, double* __restrict__ V,
                                                      double* __restrict__ sig, int* __restrict__ status) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     jacobi_svd_body<true>(R, trans != 0, c, U, V, sig, status, sm);
 }
 // c <= 64: the widths of most solves, with the registers of smaller blocks
 __global__ void __launch_bounds__(256) k_jacobi_svd64(const double* __restrict__ R, int trans, int c,
                                                       double* __restrict__ U, double* __restrict__ V,
                                                       double* __restrict__ sig, int* __restrict__ status) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     jacobi_svd_body<false>(R, trans != 0, c, U, V, sig, status, sm);
 }
 

@@ -38,7 +38,7 @@ template <typename VT>
 __global__ void __launch_bounds__(kSlThreads, 1)
     k_spmv_sliced(const __grid_constant__ SlicedOp a, const VT* __restrict__ val, const double* __restrict__ x,
                   double* __restrict__ y) {
-    extern __shared__ double sl_sm[];
+    extern __shared__ __align__(16) double sl_sm[];
     sliced_rows<VT, false>(a, val, x, 1.0, sl_sm, [&](int64_t r, double acc) { y[r] = acc; });
 }
 
