@@ -532,6 +532,7 @@ void randomized(const svdb_matrix* A, uint64_t target_rank, uint64_t n_oversampl
     const int64_t rank = std::min<int64_t>((int64_t)target_rank, std::min(m, n));
     int l = (int)(rank + (int64_t)n_oversamples);
     if (l <= 0) throw Error(SVDB_ERR_SHAPE, "randomized_svd: zero sample columns");
+    if (m == 0 || n == 0) throw Error(SVDB_ERR_SHAPE, "randomized_svd: the matrix has no rows or no columns");
     const DevCompressed& Acsr = csr_of(A);
     const DevCompressed& Acsc = csc_of(A);
     if (mixed) ensure_fp32(A);
