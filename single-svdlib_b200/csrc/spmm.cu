@@ -347,7 +347,9 @@ __global__ void k_slice16(const int64_t* __restrict__ rp, int64_t rows, unsigned
 // of more than kSegNnz entries, then those of each bin.  Above 64 entries a
 // class is a quarter octave of the length (by octaves A x of the Zipf operator
 // in k_spmv's comment took 136 us, against 130); below, one bin, so that rows
-// next to each other in memory, which share cache lines, stay together.
+// next to each other in memory, which share cache lines, stay together.  A class
+// ends at its upper length (2^e + q 2^(e-2), inclusive), so no class holds rows on
+// both sides of a bin's or the long rows' bound.
 constexpr int kSpmvKeyBits = 7;
 __global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, uint8_t* __restrict__ key,
                             int32_t* __restrict__ ids, unsigned long long* __restrict__ counts) {
@@ -359,8 +361,9 @@ __global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, uint8_
         int c = 0;  // 0: one block, c: bin c - 1
         while (c < kSpmvBins && len <= spmv_bin_len(c)) ++c;
         if (c < 2) {
-            const int e = min(63 - __clzll(len), 31);
-            key[r] = (uint8_t)(127 - 4 * e - (int)((len >> (e - 2)) & 3));
+            const int64_t k = len - 1;
+            const int e = min(63 - __clzll(k), 31);
+            key[r] = (uint8_t)(127 - 4 * e - (int)((k >> (e - 2)) & 3));
         } else {
             key[r] = (uint8_t)(104 + c);  // 65 entries: 103
         }
