@@ -281,6 +281,203 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
     }
 }
 
+// A block of cut rows: 8 >> cls warps per row, 1 << cls rows from cut.rows[p0];
+// class 0 walks one row of any length in rounds, the others' rows fit their warps.
+// Not inlined: the rest of k_spmm_cut then compiles as k_spmm_lean does (in one
+// loop with it, or inlined beside it, it cost the FP64 products 10-20 %).
+template <typename T, typename OT, int H, int NL, int U, bool BYTES>
+__device__ __noinline__ void cut_block(const int32_t* __restrict__ ci, const T* __restrict__ val,
+                                       const int64_t* __restrict__ ptr, const CutRows* cut, const T* __restrict__ X,
+                                       uint32_t ldx, int l, OT* __restrict__ Y, int ldy) {
+    using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int GL = 32 / H;  // lanes per group
+    constexpr int COLS = GL * NL * VEC;
+    using Slots = LeanSlots<T, H>;
+    extern __shared__ __align__(16) double cut_sums[];
+    __shared__ __align__(16) uint32_t s_off[kLeanWarps][32];
+    __shared__ __align__(16) T s_val[kLeanWarps][H * Slots::VS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / GL, gl = lane % GL;
+    bool active[NL];
+    uint32_t col[NL];
+#pragma unroll
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * VEC;
+        active[j] = c < l;
+        col[j] = active[j] ? (uint32_t)c : 0u;
+    }
+    const uint32_t scale = BYTES ? ldx * (uint32_t)sizeof(T) : ldx;
+    uint32_t* const oput = s_off[w] + Slots::off(lane);
+    T* const vput = s_val[w] + Slots::val(lane);
+    const uint32_t* const og = s_off[w] + g * Slots::PER;
+    const T* const vg = s_val[w] + g * Slots::VS;
+    int cls = 0, p0 = blockIdx.x;
+    for (; p0 >= cut->items(cls); ++cls) p0 -= cut->items(cls);
+    p0 = cut->first[cls] + (p0 << cls);
+    const int pend = cut->first[cls + 1], width = kLeanWarps >> cls, p = p0 + w / width;
+    int64_t beg = 0, n = 0;
+    if (p < pend) {
+        const int32_t r = __ldg(cut->rows + p);
+        beg = __ldg(ptr + r);
+        n = __ldg(ptr + r + 1) - beg;
+    }
+    const int rounds = cls == 0 ? (int)((n + cut->len * kLeanWarps - 1) / (cut->len * kLeanWarps)) : 1;
+    double carry = 0.0;
+    for (int q = 0; q < rounds; ++q) {
+        const int64_t at = (int64_t)(q * kLeanWarps + w % width) * cut->len, a = beg + at;
+        int left = (int)max((int64_t)0, min((int64_t)cut->len, n - at));
+        const int32_t* cp = ci + a + lane;
+        const T* vp = val + a + lane;
+        double acc[NL][VEC];
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[j][e] = 0.0;
+        int32_t myc = 0;
+        T myv = T(0);
+        if (lane < left) { myc = __ldg(cp); myv = __ldg(vp); }
+        for (; left > 0; left -= 32) {
+            __syncwarp();  // the previous chunk's entries have been read
+            *oput = (uint32_t)myc * scale;
+            *vput = myv;
+            __syncwarp();
+            cp += 32;
+            vp += 32;
+            if (lane + 32 < left) { myc = __ldg(cp); myv = __ldg(vp); }  // the next chunk's, while this one is used
+            CT cs[NL][VEC];
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
+            lean_chunk<T, H, NL, U, BYTES>(og, vg, left, g, X, col, active, cs);
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += (double)cs[j][e];
+        }
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += __shfl_xor_sync(0xffffffffu, acc[j][e], o);
+        if (g == 0) {
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) cut_sums[w * COLS + (j * GL + gl) * VEC + e] = acc[j][e];
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < (l << cls); t += kLeanWarps * 32) {  // at most once a thread in class 0
+            const int slot = t / l, c = t - slot * l;
+            double tot = carry;
+            for (int u = 0; u < width; ++u) tot += cut_sums[(slot * width + u) * COLS + c];
+            if (q + 1 < rounds) carry = tot;
+            else if (p0 + slot < pend) Y[(int64_t)__ldg(cut->rows + p0 + slot) * ldy + c] = (OT)tot;
+        }
+        __syncthreads();
+    }
+}
+
+// The same products where some rows are cut: rows of more than cut.len entries
+// are the first blocks' work, longest first: 8, 4 or 2 warps take a row's
+// segments, and the block adds their sums in segment order through shared memory
+// (dynamic, 8 x GL NL VEC doubles); the other blocks' warps take the other rows.
+// Written out as partials and added by a second kernel, a product of 10^5 to 10^6
+// nonzeros took an allocation and a launch more, which outlast its one kernel
+// (3,000 x 1,200, 0.26 M, l = 20, FP64, A X alone: 45 us a call, here 18).
+template <typename T, typename OT, int H, int NL, int U, int MINB, bool BYTES>
+__global__ void __launch_bounds__(kLeanWarps * 32, MINB)
+    k_spmm_cut(const int32_t* __restrict__ ci, const T* __restrict__ val, const int64_t* __restrict__ ptr, int64_t rows,
+               const __grid_constant__ CutRows cut, const T* __restrict__ X, uint32_t ldx, int l, OT* __restrict__ Y,
+               int ldy, int yvec) {
+    if ((int)blockIdx.x < cut.blocks) {
+        cut_block<T, OT, H, NL, U, BYTES>(ci, val, ptr, &cut, X, ldx, l, Y, ldy);
+        return;
+    }
+    using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int GL = 32 / H;   // lanes per group
+    using Slots = LeanSlots<T, H>;
+    __shared__ __align__(16) uint32_t s_off[kLeanWarps][32];
+    __shared__ __align__(16) T s_val[kLeanWarps][H * Slots::VS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / GL, gl = lane % GL;
+    bool active[NL];
+    uint32_t col[NL];
+#pragma unroll
+    for (int j = 0; j < NL; ++j) {
+        const int c = (j * GL + gl) * VEC;
+        active[j] = c < l;
+        col[j] = active[j] ? (uint32_t)c : 0u;
+    }
+    const uint32_t scale = BYTES ? ldx * (uint32_t)sizeof(T) : ldx;
+    uint32_t* const oput = s_off[w] + Slots::off(lane);
+    T* const vput = s_val[w] + Slots::val(lane);
+    const uint32_t* const og = s_off[w] + g * Slots::PER;
+    const T* const vg = s_val[w] + g * Slots::VS;
+    const int64_t gwarp = (int64_t)(blockIdx.x - cut.blocks) * kLeanWarps + w;
+    const int64_t nwarps = (int64_t)(gridDim.x - cut.blocks) * kLeanWarps;
+    for (int64_t rr = gwarp; rr < rows; rr += nwarps) {
+        const int64_t a = __ldg(ptr + rr);
+        const int64_t len = __ldg(ptr + rr + 1) - a;
+        if (len > cut.len) continue;  // a block's
+        int left = (int)len;
+        const int32_t* cp = ci + a + lane;
+        const T* vp = val + a + lane;
+        double acc[NL][VEC];
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[j][e] = 0.0;
+        int32_t myc = 0;
+        T myv = T(0);
+        if (lane < left) { myc = __ldg(cp); myv = __ldg(vp); }
+        for (; left > 0; left -= 32) {
+            __syncwarp();  // the previous chunk's entries have been read
+            *oput = (uint32_t)myc * scale;
+            *vput = myv;
+            __syncwarp();
+            cp += 32;
+            vp += 32;
+            if (lane + 32 < left) { myc = __ldg(cp); myv = __ldg(vp); }  // the next chunk's, while this one is used
+            CT cs[NL][VEC];
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
+            lean_chunk<T, H, NL, U, BYTES>(og, vg, left, g, X, col, active, cs);
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += (double)cs[j][e];
+        }
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) acc[j][e] += __shfl_xor_sync(0xffffffffu, acc[j][e], o);
+        if (g != 0) continue;
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+            if (!active[j]) continue;
+            const int here = l - (int)col[j];
+            OT* o = Y + rr * ldy + col[j];
+            if (yvec && here >= VEC) {
+                struct alignas(sizeof(OT) * VEC > 16 ? 16 : sizeof(OT) * VEC) Row { OT v[VEC]; };
+                Row t;
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) t.v[e] = (OT)acc[j][e];
+                *reinterpret_cast<Row*>(o) = t;
+            } else {
+                store_cols<OT, VEC>(o, here, acc[j]);
+            }
+        }
+    }
+}
+
 // rows split into several segments: add their partials in segment order
 template <typename OT>
 __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_t* __restrict__ multi_rows,
@@ -301,14 +498,27 @@ __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_
 }
 
 // ------------------------------------------------------------- the plan --
-// SpMM segment length of a structure: the power of two at which the resident
-// warps (148 SMs x 24) get at least four segments' worth of entries each, so
-// that one long row does not outlast the rest of the product.  At 2,048
-// throughout, A^T X of a 30,011 x 8,009 matrix (3.1 M nonzeros, columns up to
-// a few thousand entries, l = 40) took 196 us; 85 us at 128.
-static int64_t seg_len_for(int64_t nnz) {
-    int64_t len = nnz < 200000 ? 512 : 128;  // small products: the merge's launch costs more than a long row
-    while (len < kSegNnz && len * 4 * 148 * 24 < nnz) len *= 2;
+// SpMM segment length of a structure, a power of two.  Rows longer than it are
+// cut, so that one long row does not outlast the rest of the product.
+//  - Up to kCutNnz entries a cut row is one block's (k_spmm_cut): the length at
+//    which the resident warps (24 an SM) get two segments' worth of entries each,
+//    and no less than the mean row, or most rows would be cut.  At half of it the
+//    blocks' idle warps cost more than the shorter chains give (40,000 x 9,000,
+//    1.1 M, A^T X, l = 60, FP64, three streams: 42 us a call against 36), at twice
+//    the mean the chains are back (2,000 x 2,000, 0.47 M: 39 us against 25).
+//  - Above, cut rows are merged from partials (k_spmm_merge), whose allocation and
+//    launch no longer show: four segments a warp.  At 2,048 throughout, A^T X of a
+//    30,011 x 8,009 matrix (3.1 M, columns up to a few thousand entries, l = 40)
+//    took 196 us, at 256 85.
+// kCutNnz: A^T X, l = 60, FP64, alone / on three streams, by blocks and merged: at
+// 1.1 M 54 / 35 and 62 / 32 us, at 2.2 M 92 / 70 and 92 / 64, at 4.2 M 163 / 127
+// and 151 / 116.
+constexpr int64_t kCutNnz = 1 << 21;
+static int64_t seg_len_for(int64_t nnz, int64_t rows) {
+    const int64_t warps = (int64_t)device_props().sms * 24;
+    const bool blocks = nnz < kCutNnz;
+    int64_t len = 128;
+    while (len < kSegNnz && (len * (blocks ? 2 : 4) * warps < nnz || (blocks && len * rows < nnz))) len *= 2;
     return len;
 }
 __global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, int64_t* __restrict__ cnt) {
@@ -351,10 +561,11 @@ __global__ void k_slice16(const int64_t* __restrict__ rp, int64_t rows, unsigned
 // ends at its upper length (2^e + q 2^(e-2), inclusive), so no class holds rows on
 // both sides of a bin's or the long rows' bound.
 constexpr int kSpmvKeyBits = 7;
-__global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, uint8_t* __restrict__ key,
+constexpr int kKeyCounts = kSpmvBins + 1 + 4;  // and the rows of more than kCutMax, 4 seg, 2 seg, seg entries
+__global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, uint8_t* __restrict__ key,
                             int32_t* __restrict__ ids, unsigned long long* __restrict__ counts) {
-    __shared__ unsigned int sc[kSpmvBins + 1];
-    if (threadIdx.x <= kSpmvBins) sc[threadIdx.x] = 0;
+    __shared__ unsigned int sc[kKeyCounts];
+    if (threadIdx.x < kKeyCounts) sc[threadIdx.x] = 0;
     __syncthreads();
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t len = rp[r + 1] - rp[r];
@@ -369,9 +580,16 @@ __global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, uint8_
         }
         ids[r] = (int32_t)r;
         atomicAdd(sc + c, 1u);
+        if (len > seg) {
+            unsigned int* cut = sc + kSpmvBins + 1;
+            atomicAdd(cut + 3, 1u);
+            if (len > 2 * seg) atomicAdd(cut + 2, 1u);
+            if (len > 4 * seg) atomicAdd(cut + 1, 1u);
+            if (len > kCutMax) atomicAdd(cut, 1u);
+        }
     }
     __syncthreads();
-    if (threadIdx.x <= kSpmvBins && sc[threadIdx.x])
+    if (threadIdx.x < kKeyCounts && sc[threadIdx.x])
         atomicAdd(counts + 2 + threadIdx.x, (unsigned long long)sc[threadIdx.x]);
 }
 
@@ -389,12 +607,12 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
         p.nseg = p.nmulti = p.nlong = 0;
         return;
     }
-    const int64_t seg = seg_len_for(m.nnz);
+    const int64_t seg = seg_len_for(m.nnz, rows);
     p.multi_rows.alloc(rows, s);
     p.bin_rows.alloc(rows, s);
     // One scratch allocation for all temporaries: an allocation takes 10-25 us
     // where the pool's free blocks belong to other streams.
-    constexpr int kCounts = 3 + kSpmvBins;
+    constexpr int kCounts = 2 + kKeyCounts;
     size_t tb = 0, tb2 = 0;
     SVDB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int64_t*)nullptr, p.seg_first.p, rows + 1, s));
     SVDB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb2, (uint8_t*)nullptr, (uint8_t*)nullptr, (int32_t*)nullptr,
@@ -434,7 +652,7 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
         SVDB_CHECK_LAUNCH();
     }
     // SpMV order: the rows' length classes, longest first, by one stable sort
-    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, key, ids, nm);
+    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, seg, key, ids, nm);
     SVDB_CHECK_LAUNCH();
     SVDB_CUDA(cub::DeviceRadixSort::SortPairs(cub_tmp, tb2, key, skey, ids, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
     unsigned long long hm[kCounts];
@@ -454,6 +672,11 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.bins.off[kSpmvBins] = off;
     p.bins.items[kSpmvBins] = items;
     p.bins.rows = p.bin_rows.p;
+    // the cut rows head the same order (seg and kCutMax are class bounds)
+    p.cut.rows = p.bin_rows.p;
+    p.cut.len = (int)seg;
+    for (int k = 0; k < 4; ++k) p.cut.first[k] = (int)hm[3 + kSpmvBins + k];
+    p.cut.blocks = m.nnz < kCutNnz ? p.cut.items(0) + p.cut.items(1) + p.cut.items(2) : 0;
 }
 
 // ------------------------------------------------------------- launcher --
@@ -486,20 +709,34 @@ static bool lean_aligned(const DevCompressed& m, const T* X, int64_t ldx) {
            m.nminor * ldx < ((int64_t)1 << 31);
 }
 
+// k_spmm_cut takes every cut row: no partials, no merge
+static bool cut_in_blocks(const DevCompressed& m) { return m.plan.cut.blocks > 0 && m.plan.cut.first[0] == 0; }
+
 template <typename T, typename OT, int H, int NL, int U, int MINB>
 static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
                     double* part, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(T);
     // 8x the resident blocks: timed against the resident blocks only, 1.10
     // against 1.20 ms for A X of the 100k x 30k workload
-    const int blocks = nblk(m.plan.nseg * 32, kLeanWarps * 32, MINB * 8);
+    const int work = nblk(m.plan.nseg * 32, kLeanWarps * 32, MINB * 8);
     const int yvec = ldy % VEC == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
-    auto go = [&](auto kern) {
-        kern<<<blocks, kLeanWarps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p,
-                                                m.plan.nseg, X, (uint32_t)ldx, l, Y, ldy, yvec, part);
-    };
-    if (m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32)) go(k_spmm_lean<T, OT, H, NL, U, MINB, true>);
-    else go(k_spmm_lean<T, OT, H, NL, U, MINB, false>);
+    const bool bytes = m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32);
+    if (cut_in_blocks(m)) {
+        const CutRows& cut = m.plan.cut;
+        auto go = [&](auto kern) {
+            kern<<<cut.blocks + work, kLeanWarps * 32, (size_t)kLeanWarps * (32 / H) * NL * 16 / sizeof(T) * 8, s>>>(
+                m.idx.p, v, m.ptr.p, m.nmajor, cut, X, (uint32_t)ldx, l, Y, (int)ldy, yvec);
+        };
+        if (bytes) go(k_spmm_cut<T, OT, H, NL, U, MINB, true>);
+        else go(k_spmm_cut<T, OT, H, NL, U, MINB, false>);
+    } else {
+        auto go = [&](auto kern) {
+            kern<<<work, kLeanWarps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p,
+                                                  m.plan.nseg, X, (uint32_t)ldx, l, Y, ldy, yvec, part);
+        };
+        if (bytes) go(k_spmm_lean<T, OT, H, NL, U, MINB, true>);
+        else go(k_spmm_lean<T, OT, H, NL, U, MINB, false>);
+    }
     SVDB_CHECK_LAUNCH();
 }
 
@@ -535,7 +772,6 @@ __global__ void k_pad_rows(const T* __restrict__ in, T* __restrict__ out, uint32
 
 template <typename OT>
 static void merge_rows(const DevCompressed& m, const double* part, int l, OT* Y, int64_t ldy, cudaStream_t s) {
-    if (!m.plan.nmulti) return;
     k_spmm_merge<OT><<<nblk(m.plan.nmulti * 32, 256, 16), 256, 0, s>>>(m.plan.seg_first.p, m.plan.multi_rows.p,
                                                                       m.plan.nmulti, part, l, Y, ldy);
     SVDB_CHECK_LAUNCH();
@@ -564,23 +800,32 @@ static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t&
     return buf.p;
 }
 
+template <typename T, typename OT>
+static void lean_product(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
+                         cudaStream_t s) {
+    const int64_t merged = cut_in_blocks(m) ? 0 : m.plan.nmulti;
+    DevBuf<double> part;
+    if (merged) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
+    for (int c0 = 0; c0 < l; c0 += 128) {
+        const int lc = std::min(128, l - c0);
+        launch_lean<T, OT>(m, v, X + c0, lc, ldx, Y + c0, ldy, part.p, s);
+        if (merged) merge_rows(m, part.p, lc, Y + c0, ldy, s);
+    }
+}
+
 template <typename VT, typename XT, typename OT>
 static void spmm_impl(const DevCompressed& m, const VT* v, const XT* X, int l, OT* Y, cudaStream_t s) {
-    DevBuf<double> part;
-    if (m.plan.nmulti) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
     if constexpr (std::is_same<VT, XT>::value) {
         DevBuf<XT> buf;
         int64_t ldx = 0;
         const XT* Xa = lean_operand(m, X, l, ldx, buf, s);
         if (Xa) {
-            for (int c0 = 0; c0 < l; c0 += 128) {
-                const int lc = std::min(128, l - c0);
-                launch_lean<VT, OT>(m, v, Xa + c0, lc, ldx, Y + c0, l, part.p, s);
-                merge_rows(m, part.p, lc, Y + c0, l, s);
-            }
+            lean_product<VT, OT>(m, v, Xa, l, ldx, Y, l, s);
             return;
         }
     }
+    DevBuf<double> part;
+    if (m.plan.nmulti) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
     for (int c0 = 0; c0 < l; c0 += 128) {
         const int lc = std::min(128, l - c0);
         const XT* Xc = X + c0;
@@ -588,7 +833,7 @@ static void spmm_impl(const DevCompressed& m, const VT* v, const XT* X, int l, O
         if (lc <= 32) launch_seg<VT, XT, OT, 2, 2>(m, v, Xc, l, lc, Yc, l, part.p, s);
         else if (lc <= 64) launch_seg<VT, XT, OT, 4, 2>(m, v, Xc, l, lc, Yc, l, part.p, s);
         else launch_seg<VT, XT, OT, 4, 1>(m, v, Xc, l, lc, Yc, l, part.p, s);
-        merge_rows(m, part.p, lc, Yc, l, s);
+        if (part.p) merge_rows(m, part.p, lc, Yc, l, s);
     }
 }
 
@@ -865,10 +1110,7 @@ void spmm_f32_strided(const DevCompressed& m, const float* X, int l, int64_t ldx
     if (m.nmajor == 0) return;
     if (!spmm_f32_strided_ok(m, l, ldx) || (reinterpret_cast<uintptr_t>(X) % 16))
         throw Error(SVDB_ERR_ARG, "spmm_f32_strided: operand layout not supported");
-    DevBuf<double> part;
-    if (m.plan.nmulti) part.alloc(m.plan.nseg * (int64_t)l, s);
-    launch_lean<float, double>(m, m.val32.p, X, l, ldx, Y, l, part.p, s);
-    merge_rows(m, part.p, l, Y, l, s);
+    lean_product<float, double>(m, m.val32.p, X, l, ldx, Y, l, s);
 }
 
 template <typename XT, typename OT>

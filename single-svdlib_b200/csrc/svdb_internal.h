@@ -107,11 +107,21 @@ struct SpmvBins {
     int64_t off[kSpmvBins + 1];      // bin b: rows[off[b] .. off[b+1]); off[0] = nlong
     int64_t items[kSpmvBins + 1];    // warp items before bin b (1 << b rows per item)
 };
+// The rows of more than len entries as k_spmm_cut's blocks take them: rows[0 ..
+// first[0]) have more than kCutMax; rows[first[k] .. first[k + 1]) take 8 >> k
+// warps each, 1 << k of them a block.  blocks: 0 where all are merged from partials.
+constexpr int64_t kCutMax = 8 * kSegNnz;
+struct CutRows {
+    const int32_t* rows;  // bin_rows
+    int first[4], blocks, len;
+    __host__ __device__ int items(int k) const { return (first[k + 1] - first[k] + (1 << k) - 1) >> k; }
+};
 struct SegPlan {
     int64_t nseg = 0, nmulti = 0, nlong = 0;
     int64_t slice16_nnz = kSlice16Unknown;  // most entries in one of 16 equal row ranges (lz_resident.h)
     DevBuf<int32_t> bin_rows;
     SpmvBins bins{};
+    CutRows cut{};
     DevBuf<int64_t> seg_first;
     DevBuf<int32_t> seg_row;
     DevBuf<int64_t> seg_beg, seg_end;
