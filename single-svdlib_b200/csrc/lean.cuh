@@ -13,12 +13,10 @@ struct AccOf { using type = double; };
 template <>
 struct AccOf<float> { using type = float; };
 
-template <typename T>
-struct LeanVec;
-template <>
-struct alignas(16) LeanVec<float> { float v[4]; };
-template <>
-struct alignas(16) LeanVec<double> { double v[2]; };
+// VEC elements of a row read at once: 16 bytes, or single elements of rows that
+// are no whole 16-byte vectors
+template <typename T, int VEC = 16 / (int)sizeof(T)>
+struct alignas(sizeof(T) * VEC) LeanVec { T v[VEC]; };
 
 // Shared-memory slots of a chunk: its H groups' entries side by side, the
 // FP64 values' groups two slots apart so that they sit on different banks.
@@ -45,25 +43,25 @@ __device__ __forceinline__ void lean_values4(const T* p, T (&v)[4]) {  // four c
 // `cnt` staged ones of v X[off + col[j] ..].  A full chunk runs U gathers per
 // lane at a time, a shorter one masked batches of four.  BYTES: offsets are
 // bytes from X, else elements.
-template <typename T, int H, int NL, int U, bool BYTES>
+template <typename T, int H, int NL, int U, bool BYTES, int VEC = 16 / (int)sizeof(T)>
 __device__ __forceinline__ void lean_chunk(const uint32_t* og, const T* vg, int cnt, int g, const T* __restrict__ X,
                                            const uint32_t (&col)[NL], const bool (&active)[NL],
-                                           typename AccOf<T>::type (&cs)[NL][16 / sizeof(T)]) {
+                                           typename AccOf<T>::type (&cs)[NL][VEC]) {
     using CT = typename AccOf<T>::type;
-    constexpr int VEC = 16 / (int)sizeof(T);
+    using Vec = LeanVec<T, VEC>;
     constexpr int PER = LeanSlots<T, H>::PER;
     static_assert(U % 4 == 0 && U <= PER, "batches of whole quads");
     auto gather = [&](uint32_t off, int j) {
         if constexpr (BYTES)
-            return *reinterpret_cast<const LeanVec<T>*>(reinterpret_cast<const char*>(X) +
+            return *reinterpret_cast<const Vec*>(reinterpret_cast<const char*>(X) +
                                                         (off + col[j] * (uint32_t)sizeof(T)));
         else
-            return *reinterpret_cast<const LeanVec<T>*>(X + (off + col[j]));
+            return *reinterpret_cast<const Vec*>(X + (off + col[j]));
     };
     if (cnt >= 32) {
 #pragma unroll 1
         for (int qb = 0; qb < PER; qb += U) {  // one batch live at a time
-            LeanVec<T> xv[U][NL];
+            Vec xv[U][NL];
             T vv[U];
 #pragma unroll
             for (int q = 0; q < U; q += 4) {
@@ -77,7 +75,7 @@ __device__ __forceinline__ void lean_chunk(const uint32_t* og, const T* vg, int 
 #pragma unroll
                     for (int j = 0; j < NL; ++j) {
                         if (active[j]) xv[q + u][j] = gather(off, j);
-                        else xv[q + u][j] = LeanVec<T>{};
+                        else xv[q + u][j] = Vec{};
                     }
                 }
             }
@@ -92,7 +90,7 @@ __device__ __forceinline__ void lean_chunk(const uint32_t* og, const T* vg, int 
         const int mine = (cnt - g + H - 1) / H;  // entries of this group
 #pragma unroll 1
         for (int qb = 0; qb * H < cnt; qb += 4) {
-            LeanVec<T> xv[4][NL];
+            Vec xv[4][NL];
             T vv[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -102,7 +100,7 @@ __device__ __forceinline__ void lean_chunk(const uint32_t* og, const T* vg, int 
 #pragma unroll
                 for (int j = 0; j < NL; ++j) {
                     if (ok && active[j]) xv[u][j] = gather(off, j);
-                    else xv[u][j] = LeanVec<T>{};
+                    else xv[u][j] = Vec{};
                 }
             }
 #pragma unroll

@@ -285,12 +285,11 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
 // class 0 walks one row of any length in rounds, the others' rows fit their warps.
 // Not inlined: the rest of k_spmm_cut then compiles as k_spmm_lean does (in one
 // loop with it, or inlined beside it, it cost the FP64 products 10-20 %).
-template <typename T, typename OT, int H, int NL, int U, bool BYTES>
+template <typename T, typename OT, int VEC, int H, int NL, int U, bool BYTES>
 __device__ __noinline__ void cut_block(const int32_t* __restrict__ ci, const T* __restrict__ val,
                                        const int64_t* __restrict__ ptr, const CutRows* cut, const T* __restrict__ X,
                                        uint32_t ldx, int l, OT* __restrict__ Y, int ldy) {
     using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
-    constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int GL = 32 / H;  // lanes per group
     constexpr int COLS = GL * NL * VEC;
     using Slots = LeanSlots<T, H>;
@@ -350,7 +349,7 @@ __device__ __noinline__ void cut_block(const int32_t* __restrict__ ci, const T* 
             for (int j = 0; j < NL; ++j)
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
-            lean_chunk<T, H, NL, U, BYTES>(og, vg, left, g, X, col, active, cs);
+            lean_chunk<T, H, NL, U, BYTES, VEC>(og, vg, left, g, X, col, active, cs);
 #pragma unroll
             for (int j = 0; j < NL; ++j)
 #pragma unroll
@@ -387,17 +386,16 @@ __device__ __noinline__ void cut_block(const int32_t* __restrict__ ci, const T* 
 // Written out as partials and added by a second kernel, a product of 10^5 to 10^6
 // nonzeros took an allocation and a launch more, which outlast its one kernel
 // (3,000 x 1,200, 0.26 M, l = 20, FP64, A X alone: 45 us a call, here 18).
-template <typename T, typename OT, int H, int NL, int U, int MINB, bool BYTES>
+template <typename T, typename OT, int VEC, int H, int NL, int U, int MINB, bool BYTES>
 __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
     k_spmm_cut(const int32_t* __restrict__ ci, const T* __restrict__ val, const int64_t* __restrict__ ptr, int64_t rows,
                const __grid_constant__ CutRows cut, const T* __restrict__ X, uint32_t ldx, int l, OT* __restrict__ Y,
                int ldy, int yvec) {
     if ((int)blockIdx.x < cut.blocks) {
-        cut_block<T, OT, H, NL, U, BYTES>(ci, val, ptr, &cut, X, ldx, l, Y, ldy);
+        cut_block<T, OT, VEC, H, NL, U, BYTES>(ci, val, ptr, &cut, X, ldx, l, Y, ldy);
         return;
     }
     using CT = typename AccOf<T>::type;  // chunk sums: FP32 for float, FP64 for double
-    constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int GL = 32 / H;   // lanes per group
     using Slots = LeanSlots<T, H>;
     __shared__ __align__(16) uint32_t s_off[kLeanWarps][32];
@@ -447,7 +445,7 @@ __global__ void __launch_bounds__(kLeanWarps * 32, MINB)
             for (int j = 0; j < NL; ++j)
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) cs[j][e] = CT(0);
-            lean_chunk<T, H, NL, U, BYTES>(og, vg, left, g, X, col, active, cs);
+            lean_chunk<T, H, NL, U, BYTES, VEC>(og, vg, left, g, X, col, active, cs);
 #pragma unroll
             for (int j = 0; j < NL; ++j)
 #pragma unroll
@@ -502,7 +500,8 @@ __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_
 // cut, so that one long row does not outlast the rest of the product.
 //  - Up to kCutNnz entries a cut row is one block's (k_spmm_cut): the length at
 //    which the resident warps (24 an SM) get two segments' worth of entries each,
-//    and no less than the mean row, or most rows would be cut.  At half of it the
+//    and no less than the mean row, or most rows would be cut (unless there are
+//    too few rows to fill the warps).  At half of it the
 //    blocks' idle warps cost more than the shorter chains give (40,000 x 9,000,
 //    1.1 M, A^T X, l = 60, FP64, three streams: 42 us a call against 36), at twice
 //    the mean the chains are back (2,000 x 2,000, 0.47 M: 39 us against 25).
@@ -518,7 +517,8 @@ static int64_t seg_len_for(int64_t nnz, int64_t rows) {
     const int64_t warps = (int64_t)device_props().sms * 24;
     const bool blocks = nnz < kCutNnz;
     int64_t len = 128;
-    while (len < kSegNnz && (len * (blocks ? 2 : 4) * warps < nnz || (blocks && len * rows < nnz))) len *= 2;
+    while (len < kSegNnz && (len * (blocks ? 2 : 4) * warps < nnz || (blocks && rows * 4 >= warps && len * rows < nnz)))
+        len *= 2;
     return len;
 }
 __global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, int64_t* __restrict__ cnt) {
@@ -713,22 +713,23 @@ static bool lean_aligned(const DevCompressed& m, const T* X, int64_t ldx) {
 static bool cut_in_blocks(const DevCompressed& m) { return m.plan.cut.blocks > 0 && m.plan.cut.first[0] == 0; }
 
 template <typename T, typename OT, int H, int NL, int U, int MINB>
-static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
-                    double* part, cudaStream_t s) {
+static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
+                    int64_t ldy, double* part, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(T);
     // 8x the resident blocks: timed against the resident blocks only, 1.10
     // against 1.20 ms for A X of the 100k x 30k workload
     const int work = nblk(m.plan.nseg * 32, kLeanWarps * 32, MINB * 8);
     const int yvec = ldy % VEC == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     const bool bytes = m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32);
-    if (cut_in_blocks(m)) {
+    if (narrow || cut_in_blocks(m)) {
         const CutRows& cut = m.plan.cut;
         auto go = [&](auto kern) {
             kern<<<cut.blocks + work, kLeanWarps * 32, (size_t)kLeanWarps * (32 / H) * NL * 16 / sizeof(T) * 8, s>>>(
                 m.idx.p, v, m.ptr.p, m.nmajor, cut, X, (uint32_t)ldx, l, Y, (int)ldy, yvec);
         };
-        if (bytes) go(k_spmm_cut<T, OT, H, NL, U, MINB, true>);
-        else go(k_spmm_cut<T, OT, H, NL, U, MINB, false>);
+        if (narrow) go(k_spmm_cut<T, OT, 1, H, NL * VEC, 4, MINB, true>);  // four rows in flight: more spill
+        else if (bytes) go(k_spmm_cut<T, OT, VEC, H, NL, U, MINB, true>);
+        else go(k_spmm_cut<T, OT, VEC, H, NL, U, MINB, false>);
     } else {
         auto go = [&](auto kern) {
             kern<<<work, kLeanWarps * 32, 0, s>>>(m.idx.p, v, m.plan.seg_row.p, m.plan.seg_beg.p, m.plan.seg_end.p,
@@ -741,23 +742,24 @@ static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64
 }
 
 // l <= 128 columns of X (ldx apart) into Y (ldy apart).  Lane groups as narrow
-// as the columns allow, so that few lanes idle.
+// as the columns allow, so that few lanes idle.  narrow: X is read element by
+// element, VEC times the vectors a lane in the same groups.
 template <typename T, typename OT>
-static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
-                        double* part, cudaStream_t s) {
+static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
+                        int64_t ldy, double* part, cudaStream_t s) {
     if (m.plan.nseg <= 0) return;
     if constexpr (std::is_same<T, float>::value) {
-        if (l <= 16) lean_go<T, OT, 8, 1, 4, 4>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 32) lean_go<T, OT, 4, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 64) lean_go<T, OT, 2, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
-        else lean_go<T, OT, 1, 1, 8, 4>(m, v, X, l, ldx, Y, ldy, part, s);
+        if (l <= 16) lean_go<T, OT, 8, 1, 4, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
     } else {
-        if (l <= 8) lean_go<T, OT, 8, 1, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 16) lean_go<T, OT, 4, 1, 8, 3>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 32) lean_go<T, OT, 4, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 48) lean_go<T, OT, 4, 3, 4, 2>(m, v, X, l, ldx, Y, ldy, part, s);
-        else if (l <= 64) lean_go<T, OT, 2, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
-        else lean_go<T, OT, 1, 2, 4, 3>(m, v, X, l, ldx, Y, ldy, part, s);
+        if (l <= 8) lean_go<T, OT, 8, 1, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 16) lean_go<T, OT, 4, 1, 8, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 48) lean_go<T, OT, 4, 3, 4, 2>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
     }
 }
 
@@ -777,23 +779,47 @@ static void merge_rows(const DevCompressed& m, const double* part, int l, OT* Y,
     SVDB_CHECK_LAUNCH();
 }
 
-// The operand k_spmm_lean reads: X itself, or a copy in `buf` whose rows are
-// whole 16-byte vectors (odd l, unaligned X).  Null where it does not apply:
-// 2^31 elements or more, or fewer entries than rows of X (the copy would cost
-// more than the gathers); k_spmm_seg takes those as they are.  Rows padded
-// further, to whole 128-byte lines, were no faster (50,000 x 30,000, 28 M
-// nonzeros, l = 60: 805 against 812 us FP64, 865 against 870 FP32 at 100,000
+// The operand the lean kernels read: X itself, or a copy in `buf` where its rows
+// are no whole 16-byte vectors (odd l, unaligned X).  A copy is an allocation and
+// a launch, 10-17 us of a call that runs alone, so small products read X as it is,
+// element by element (narrow: k_spmm_cut in the same lane groups, the same bits):
+// up to 2^24 gathered elements, 2^25 above 64 columns, and at FP64 above 64 columns
+// always.  A X of 20,000 x 6,000, 1.07 M, alone / on three streams, narrow and
+// copied, us: l = 7 (2^23) FP32 27 / 13 and 37 / 13; l = 23 (2^24.5) FP32 39 / 22
+// and 42 / 17, FP64 43 / 27 and 54 / 26; l = 63 (2^26) FP32 50 / 31 and 51 / 24, FP64
+// 83 / 56 and 68 / 38; l = 101 (2^26.7) FP32 85 / 54 and 70 / 36, FP64 91 / 65 and
+// 107 / 66.  A copy that cannot be allocated is done without.  Null: k_spmm_seg
+// takes X as it is (also fewer entries than rows of X, and 2^31 elements or more).
+// Rows padded further, to whole 128-byte lines, were no faster (50,000 x 30,000,
+// 28 M nonzeros, l = 60: 805 against 812 us FP64, 865 against 870 FP32 at 100,000
 // rows): the gathers run at 15-17 TB/s of rows, near what L2 delivers.
 template <typename T>
-static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t& ldx, DevBuf<T>& buf,
+static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t& ldx, bool& narrow, DevBuf<T>& buf,
                              cudaStream_t s) {
-    if (lean_off()) return nullptr;
+    constexpr bool f32 = sizeof(T) == 4;
+    narrow = false;
     ldx = l;
+    if (lean_off()) return nullptr;
     if (lean_aligned(m, X, ldx)) return X;
+    const int64_t gathered = m.nnz * l;
+    const bool can = m.nnz < kCutNnz && m.plan.cut.first[0] == 0 &&
+                     m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32);
+    if (can && ((!f32 && l > 64) || gathered <= ((int64_t)1 << (l > 64 ? 25 : 24)) || m.nnz < m.nminor)) {
+        narrow = true;
+        return X;
+    }
     constexpr int64_t VEC = 16 / (int64_t)sizeof(T);
-    ldx = (l + VEC - 1) / VEC * VEC;
-    if (m.nnz < m.nminor || m.nminor * ldx >= ((int64_t)1 << 31)) return nullptr;
-    buf.alloc(std::max<int64_t>(m.nminor * ldx, 1), s);
+    const int64_t ldc = (l + VEC - 1) / VEC * VEC;
+    if (m.nnz < m.nminor || m.nminor * ldc >= ((int64_t)1 << 31)) return nullptr;
+    try {
+        buf.alloc(std::max<int64_t>(m.nminor * ldc, 1), s);
+    } catch (const Error& e) {
+        if (e.code != SVDB_ERR_OOM) throw;
+        cudaGetLastError();
+        narrow = can;
+        return can ? X : nullptr;
+    }
+    ldx = ldc;
     k_pad_rows<T><<<nblk(m.nminor * ldx, 256, 16), 256, 0, s>>>(X, buf.p, (uint32_t)(m.nminor * ldx), (uint32_t)l,
                                                                (uint32_t)ldx);
     SVDB_CHECK_LAUNCH();
@@ -801,14 +827,14 @@ static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t&
 }
 
 template <typename T, typename OT>
-static void lean_product(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, OT* Y, int64_t ldy,
-                         cudaStream_t s) {
-    const int64_t merged = cut_in_blocks(m) ? 0 : m.plan.nmulti;
+static void lean_product(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
+                         int64_t ldy, cudaStream_t s) {
+    const int64_t merged = narrow || cut_in_blocks(m) ? 0 : m.plan.nmulti;
     DevBuf<double> part;
     if (merged) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
     for (int c0 = 0; c0 < l; c0 += 128) {
         const int lc = std::min(128, l - c0);
-        launch_lean<T, OT>(m, v, X + c0, lc, ldx, Y + c0, ldy, part.p, s);
+        launch_lean<T, OT>(m, v, X + c0, lc, ldx, narrow, Y + c0, ldy, part.p, s);
         if (merged) merge_rows(m, part.p, lc, Y + c0, ldy, s);
     }
 }
@@ -818,9 +844,10 @@ static void spmm_impl(const DevCompressed& m, const VT* v, const XT* X, int l, O
     if constexpr (std::is_same<VT, XT>::value) {
         DevBuf<XT> buf;
         int64_t ldx = 0;
-        const XT* Xa = lean_operand(m, X, l, ldx, buf, s);
+        bool narrow = false;
+        const XT* Xa = lean_operand(m, X, l, ldx, narrow, buf, s);
         if (Xa) {
-            lean_product<VT, OT>(m, v, Xa, l, ldx, Y, l, s);
+            lean_product<VT, OT>(m, v, Xa, l, ldx, narrow, Y, l, s);
             return;
         }
     }
@@ -1110,7 +1137,7 @@ void spmm_f32_strided(const DevCompressed& m, const float* X, int l, int64_t ldx
     if (m.nmajor == 0) return;
     if (!spmm_f32_strided_ok(m, l, ldx) || (reinterpret_cast<uintptr_t>(X) % 16))
         throw Error(SVDB_ERR_ARG, "spmm_f32_strided: operand layout not supported");
-    lean_product<float, double>(m, m.val32.p, X, l, ldx, Y, l, s);
+    lean_product<float, double>(m, m.val32.p, X, l, ldx, false, Y, l, s);
 }
 
 template <typename XT, typename OT>
