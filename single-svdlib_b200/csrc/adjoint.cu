@@ -45,16 +45,15 @@ static int grid_for_work(int64_t work, int threads, int per_sm = 8) {
 // loads, a 31-shuffle transpose with two selects each over the whole warp,
 // about 20 warp instructions per entry) took 313 us for 4.3 M entries of
 // rank 64 at FP32.
-template <typename T>
-struct alignas(16) SdVec { T v[16 / sizeof(T)]; };
+template <typename T, int VEC>
+struct alignas(sizeof(T) * VEC) SdVec { T v[VEC]; };
 
-template <typename T, int GL, int NL, int U, int MINB>
+template <typename T, int VEC, int GL, int NL, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__ idx, const int32_t* __restrict__ seg_row,
                                                      const int64_t* __restrict__ seg_beg,
                                                      const int64_t* __restrict__ seg_end, int64_t nseg,
                                                      const T* __restrict__ left, const T* __restrict__ right, int rank,
                                                      T* __restrict__ out) {
-    constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int H = 32 / GL;
     static_assert(GL % U == 0, "whole batches");
     constexpr int SH = GL / U;  // lanes that end up with one entry of a batch; batches of a chunk
@@ -77,10 +76,10 @@ __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__
         int left_n = (int)(__ldg(seg_end + sg) - beg);
         const int32_t* ip = idx + beg + lane;
         int32_t cm = lane < left_n ? __ldg(ip) : 0;
-        SdVec<T> lv[NL];
+        SdVec<T, VEC> lv[NL];
 #pragma unroll
         for (int j = 0; j < NL; ++j)
-            lv[j] = active[j] ? *reinterpret_cast<const SdVec<T>*>(left + (int64_t)r * rank + col[j]) : SdVec<T>{};
+            lv[j] = active[j] ? *reinterpret_cast<const SdVec<T, VEC>*>(left + (int64_t)r * rank + col[j]) : SdVec<T, VEC>{};
         for (T* op = out + beg; left_n > 0; left_n -= 32, op += 32) {
             const int cnt = left_n < 32 ? left_n : 32;
             ip += 32;
@@ -88,7 +87,7 @@ __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__
             T res = T(0);
 #pragma unroll 1
             for (int b = 0; b < SH && b * U * H < cnt; ++b) {
-                SdVec<T> x[U][NL];
+                SdVec<T, VEC> x[U][NL];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int q = (b * U + u) * H + g;
@@ -96,8 +95,8 @@ __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__
                     const T* row = right + (uint64_t)c * (uint32_t)rank;
 #pragma unroll
                     for (int j = 0; j < NL; ++j) {
-                        if (q < cnt && active[j]) x[u][j] = *reinterpret_cast<const SdVec<T>*>(row + col[j]);
-                        else x[u][j] = SdVec<T>{};
+                        if (q < cnt && active[j]) x[u][j] = *reinterpret_cast<const SdVec<T, VEC>*>(row + col[j]);
+                        else x[u][j] = SdVec<T, VEC>{};
                     }
                 }
                 T p[U];
@@ -132,14 +131,71 @@ __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__
     }
 }
 
-// out (rows x ldo) = in (rows x rank), zero past column rank
+// A lane per column (rank <= 32 SLOTS), 4- or 8-byte loads, a butterfly transpose
+// over the whole warp per 32 entries: for small products at ranks above 64 that
+// are no whole 16-byte vectors, where the form above has too many loads a lane.
+template <typename T, int SLOTS>
+__global__ void __launch_bounds__(256) k_sddmm_lane(const int32_t* __restrict__ idx, const int32_t* __restrict__ seg_row,
+                                                    const int64_t* __restrict__ seg_beg,
+                                                    const int64_t* __restrict__ seg_end, int64_t nseg,
+                                                    const T* __restrict__ left, const T* __restrict__ right, int rank,
+                                                    T* __restrict__ out) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t sg = warp0; sg < nseg; sg += nwarps) {
+        int32_t r = seg_row[sg];
+        if (r < 0) r = -r - 1;
+        const int64_t beg = seg_beg[sg], end = seg_end[sg];
+        T lv[SLOTS];
+#pragma unroll
+        for (int j = 0; j < SLOTS; ++j) {
+            const int t = lane + 32 * j;
+            lv[j] = t < rank ? left[(int64_t)r * rank + t] : T(0);
+        }
+        for (int64_t p0 = beg; p0 < end; p0 += 32) {
+            const int cnt = (int)min((int64_t)32, end - p0);
+            const int cmine = lane < cnt ? idx[p0 + lane] : 0;
+            T p[32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+                const int c = __shfl_sync(full, cmine, q);
+                T acc = T(0);
+                if (q < cnt) {
+                    const T* rr = right + (int64_t)c * rank;
+#pragma unroll
+                    for (int j = 0; j < SLOTS; ++j) {
+                        const int t = lane + 32 * j;
+                        if (t < rank) acc = fma(lv[j], __ldg(rr + t), acc);
+                    }
+                }
+                p[q] = acc;
+            }
+#pragma unroll
+            for (int w = 16; w >= 1; w >>= 1) {
+                const bool upper = (lane & w) != 0;
+#pragma unroll
+                for (int i = 0; i < w; ++i) {
+                    const T send = upper ? p[i] : p[i + w];
+                    const T keep = upper ? p[i + w] : p[i];
+                    p[i] = keep + __shfl_xor_sync(full, send, w);
+                }
+            }
+            if (lane < cnt) out[p0 + lane] = p[0];
+        }
+    }
+}
+
+// out ((rl + rr) x ldo) = the rows of l, then of r (x rank), zero past column rank
 template <typename T>
-__global__ void k_sddmm_pad(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int rank, int ldo) {
-    const int64_t n = rows * ldo;
+__global__ void k_sddmm_pad(const T* __restrict__ l, int64_t rl, const T* __restrict__ r, int64_t rr, int rank,
+                            int ldo, T* __restrict__ out) {
+    const int64_t n = (rl + rr) * ldo;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / ldo;
-        const int c = (int)(i - r * ldo);
-        out[i] = c < rank ? in[r * rank + c] : T(0);
+        const int64_t q = i / ldo;
+        const int c = (int)(i - q * ldo);
+        out[i] = c < rank ? (q < rl ? l[q * rank + c] : r[(q - rl) * rank + c]) : T(0);
     }
 }
 
@@ -147,37 +203,67 @@ template <typename T>
 static void sddmm_launch(const DevCompressed& m, const T* left, const T* right, int rank, T* out, cudaStream_t s) {
     if (m.nnz == 0) return;
     if (rank > 256) throw Error(SVDB_ERR_UNSUPPORTED, "sddmm: rank above 256");
-    // factors whose rows are not whole 16-byte vectors are copied to rows that are
     constexpr int VEC = 16 / (int)sizeof(T);
-    DevBuf<T> lbuf, rbuf;
-    const int ld = (rank + VEC - 1) / VEC * VEC;
-    auto whole = [&](const T* x, int64_t rows, DevBuf<T>& buf) -> const T* {
-        if (ld == rank && reinterpret_cast<uintptr_t>(x) % 16 == 0) return x;
-        buf.alloc(rows * ld, s);
-        k_sddmm_pad<T><<<grid_for_work(rows * ld, 256, 16), 256, 0, s>>>(x, buf.p, rows, rank, ld);
-        SVDB_CHECK_LAUNCH();
-        return buf.p;
-    };
-    left = whole(left, m.nmajor, lbuf);
-    right = whole(right, m.nminor, rbuf);
+    constexpr bool f32 = sizeof(T) == 4;
     const SegPlan& pl = m.plan;
     const int blocks = grid_for_work(pl.nseg * 32, 256, 24);
+    int ld = (rank + VEC - 1) / VEC * VEC;
     auto go = [&](auto kern) {
         kern<<<blocks, 256, 0, s>>>(m.idx.p, pl.seg_row.p, pl.seg_beg.p, pl.seg_end.p, pl.nseg, left, right, ld, out);
     };
+    // Factors whose rows are no whole 16-byte vectors are copied to rows that are
+    // (one allocation, one launch: 25-40 us of a call that runs alone) where enough
+    // is gathered from them; else, and where the copy cannot be allocated, they are
+    // read element by element.  20,000 x 6,000, 1.06 M, FP32, alone / on three
+    // streams, element by element and copied: rank 23 (2^24.5) 49 / 28 and 61 / 25 us,
+    // rank 37 (2^25.2) 80 / 49 and 79 / 29, rank 63 (2^26) 85 / 52 and 81 / 29.
+    auto fits = [&](const T* x) { return ld == rank && reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+    const int64_t lrows = fits(left) ? 0 : m.nmajor, rrows = fits(right) ? 0 : m.nminor;
+    DevBuf<T> buf;
+    if (lrows + rrows) {
+        bool copied = m.nnz * rank > ((int64_t)1 << 25) && m.nnz > 4 * (lrows + rrows);
+        if (copied) {
+            try {
+                buf.alloc((lrows + rrows) * ld, s);
+            } catch (const Error& e) {
+                if (e.code != SVDB_ERR_OOM) throw;
+                cudaGetLastError();
+                copied = false;
+            }
+        }
+        if (!copied) {
+            ld = rank;
+            if (rank <= 4) go(k_sddmm<T, 1, 4, 1, 4, 4>);
+            else if (rank <= 8) go(k_sddmm<T, 1, 8, 1, 8, 4>);
+            else if (rank <= 16) go(k_sddmm<T, 1, 8, 2, f32 ? 2 : 8, f32 ? 6 : 4>);
+            else if (rank <= 32) go(k_sddmm<T, 1, 8, 4, 2, 4>);
+            else if (rank <= 64) go(k_sddmm<T, 1, 16, 4, 2, 4>);
+            else if (rank <= 96) go(k_sddmm_lane<T, 3>);
+            else if (rank <= 128) go(k_sddmm_lane<T, 4>);
+            else if (rank <= 192) go(k_sddmm_lane<T, 6>);
+            else go(k_sddmm_lane<T, 8>);
+            SVDB_CHECK_LAUNCH();
+            return;
+        }
+        k_sddmm_pad<T><<<grid_for_work((lrows + rrows) * ld, 256, 16), 256, 0, s>>>(left, lrows, right, rrows, rank, ld,
+                                                                                    buf.p);
+        SVDB_CHECK_LAUNCH();
+        if (lrows) left = buf.p;
+        if (rrows) right = buf.p + lrows * ld;
+    }
     // At least 64 contiguous bytes per load, two vectors per lane before the
     // group widens, and as many warps as the registers allow: warps count more
     // than entries in flight per warp (5.4 M entries, rank 64, FP32: 126 us with
     // two entries and six CTAs per SM, 144-174 with eight and two or three;
     // FP64: 240 us with four entries and four CTAs, 291 with (8, 4, 2) and three).
     const int nv = ld / VEC;  // vectors per row
-    if (nv <= 4) go(k_sddmm<T, 4, 1, 4, 4>);
-    else if (nv <= 8) go(k_sddmm<T, 8, 1, 8, 4>);
-    else if (nv <= 16) go(k_sddmm<T, 8, 2, 2, 6>);
-    else if (nv <= 24) go(k_sddmm<T, 8, 3, 2, 4>);
-    else if (nv <= 32) go(k_sddmm<T, 16, 2, 4, 4>);
-    else if (nv <= 64) go(k_sddmm<T, 32, 2, 4, 4>);
-    else go(k_sddmm<T, 32, 4, 2, 3>);
+    if (nv <= 4) go(k_sddmm<T, VEC, 4, 1, 4, 4>);
+    else if (nv <= 8) go(k_sddmm<T, VEC, 8, 1, 8, 4>);
+    else if (nv <= 16) go(k_sddmm<T, VEC, 8, 2, 2, 6>);
+    else if (nv <= 24) go(k_sddmm<T, VEC, 8, 3, 2, 4>);
+    else if (nv <= 32) go(k_sddmm<T, VEC, 16, 2, 4, 4>);
+    else if (nv <= 64) go(k_sddmm<T, VEC, 32, 2, 4, 4>);
+    else go(k_sddmm<T, VEC, 32, 4, 2, 3>);
     SVDB_CHECK_LAUNCH();
 }
 

@@ -513,12 +513,15 @@ __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_
 // 1.1 M 54 / 35 and 62 / 32 us, at 2.2 M 92 / 70 and 92 / 64, at 4.2 M 163 / 127
 // and 151 / 116.
 constexpr int64_t kCutNnz = 1 << 21;
-static int64_t seg_len_for(int64_t nnz, int64_t rows) {
-    const int64_t warps = (int64_t)device_props().sms * 24;
-    const bool blocks = nnz < kCutNnz;
+static int64_t seg_len_for(int64_t nnz) {
     int64_t len = 128;
-    while (len < kSegNnz && (len * (blocks ? 2 : 4) * warps < nnz || (blocks && rows * 4 >= warps && len * rows < nnz)))
-        len *= 2;
+    while (len < kSegNnz && len * 4 * device_props().sms * 24 < nnz) len *= 2;
+    return len;
+}
+static int64_t cut_len_for(int64_t nnz, int64_t rows) {
+    const int64_t warps = (int64_t)device_props().sms * 24;
+    int64_t len = 128;
+    while (len < kSegNnz && (len * 2 * warps < nnz || (rows * 4 >= warps && len * rows < nnz))) len *= 2;
     return len;
 }
 __global__ void k_seg_count(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, int64_t* __restrict__ cnt) {
@@ -561,8 +564,8 @@ __global__ void k_slice16(const int64_t* __restrict__ rp, int64_t rows, unsigned
 // ends at its upper length (2^e + q 2^(e-2), inclusive), so no class holds rows on
 // both sides of a bin's or the long rows' bound.
 constexpr int kSpmvKeyBits = 7;
-constexpr int kKeyCounts = kSpmvBins + 1 + 4;  // and the rows of more than kCutMax, 4 seg, 2 seg, seg entries
-__global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, int64_t seg, uint8_t* __restrict__ key,
+constexpr int kKeyCounts = kSpmvBins + 1 + 4;  // and the rows of more than kCutMax, 4, 2 and 1 cut_len entries
+__global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, int64_t cut_len, uint8_t* __restrict__ key,
                             int32_t* __restrict__ ids, unsigned long long* __restrict__ counts) {
     __shared__ unsigned int sc[kKeyCounts];
     if (threadIdx.x < kKeyCounts) sc[threadIdx.x] = 0;
@@ -580,11 +583,11 @@ __global__ void k_spmv_keys(const int64_t* __restrict__ rp, int64_t rows, int64_
         }
         ids[r] = (int32_t)r;
         atomicAdd(sc + c, 1u);
-        if (len > seg) {
+        if (len > cut_len) {
             unsigned int* cut = sc + kSpmvBins + 1;
             atomicAdd(cut + 3, 1u);
-            if (len > 2 * seg) atomicAdd(cut + 2, 1u);
-            if (len > 4 * seg) atomicAdd(cut + 1, 1u);
+            if (len > 2 * cut_len) atomicAdd(cut + 2, 1u);
+            if (len > 4 * cut_len) atomicAdd(cut + 1, 1u);
             if (len > kCutMax) atomicAdd(cut, 1u);
         }
     }
@@ -607,7 +610,7 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
         p.nseg = p.nmulti = p.nlong = 0;
         return;
     }
-    const int64_t seg = seg_len_for(m.nnz, rows);
+    const int64_t seg = seg_len_for(m.nnz), cut = cut_len_for(m.nnz, rows);
     p.multi_rows.alloc(rows, s);
     p.bin_rows.alloc(rows, s);
     // One scratch allocation for all temporaries: an allocation takes 10-25 us
@@ -652,7 +655,7 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
         SVDB_CHECK_LAUNCH();
     }
     // SpMV order: the rows' length classes, longest first, by one stable sort
-    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, seg, key, ids, nm);
+    k_spmv_keys<<<nblk(rows, 256, 16), 256, 0, s>>>(m.ptr.p, rows, cut, key, ids, nm);
     SVDB_CHECK_LAUNCH();
     SVDB_CUDA(cub::DeviceRadixSort::SortPairs(cub_tmp, tb2, key, skey, ids, p.bin_rows.p, rows, 0, kSpmvKeyBits, s));
     unsigned long long hm[kCounts];
@@ -672,9 +675,9 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.bins.off[kSpmvBins] = off;
     p.bins.items[kSpmvBins] = items;
     p.bins.rows = p.bin_rows.p;
-    // the cut rows head the same order (seg and kCutMax are class bounds)
+    // the cut rows head the same order (its length and kCutMax are class bounds)
     p.cut.rows = p.bin_rows.p;
-    p.cut.len = (int)seg;
+    p.cut.len = (int)cut;
     for (int k = 0; k < 4; ++k) p.cut.first[k] = (int)hm[3 + kSpmvBins + k];
     p.cut.blocks = m.nnz < kCutNnz ? p.cut.items(0) + p.cut.items(1) + p.cut.items(2) : 0;
 }
