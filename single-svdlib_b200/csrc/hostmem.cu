@@ -7,6 +7,7 @@
 // svdb_rec_free hands them back, a later result of a similar size takes them
 // again, and svdb_release_cached_memory returns them to the driver.  Smaller
 // buffers are plain malloc.
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -45,7 +46,7 @@ void* host_result_alloc(size_t bytes) {
     {
         std::lock_guard<std::mutex> lk(c.mu);
         auto it = c.idle.lower_bound(bytes);
-        if (it != c.idle.end() && it->first <= 2 * bytes + kPinnedGrain) {  // no more than about twice the size
+        if (it != c.idle.end() && it->first <= std::max(2 * bytes, kPinnedGrain)) {  // twice the size, or one grain
             void* p = it->second;
             const size_t cap = it->first;
             c.idle.erase(it);

@@ -9,6 +9,8 @@ constructed and keep a device handle for their lifetime.
 from __future__ import annotations
 
 import ctypes as C
+import mmap
+import os
 import threading
 import weakref
 from dataclasses import dataclass, field
@@ -138,53 +140,131 @@ class SvdRec:
 # Result buffers of 64 KB and more are page-locked memory that the library
 # reuses (csrc/hostmem.cu).  An array takes its buffer over and hands it back
 # when the last view of it dies: copying 86 MB of results into fresh pages took
-# about 20 ms beside 4 ms of solving.  At most _LENT_MAX bytes are out at a
-# time (page-locked memory is scarce, and a caller that keeps every result
-# would have each call page-lock anew); past that, and for small results, the
-# values are copied and the buffer is released at once.
-_LENT_MIN, _LENT_MAX = 64 << 10, 512 << 20
-_lent = 0
+# about 20 ms beside 4 ms of solving.
+#
+# Page-locking costs more than copying (1.3 ms for the 2 MB behind a small
+# result, against 0.2 ms a MB), so a caller that keeps its results must not have
+# every call page-lock anew: a call lends only while at most _KEPT_CALLS earlier
+# calls, the previous one aside, still have theirs out.  A loop that keeps the
+# results of 1,000 x 250 solves took 1.79 ms a call lent, 0.47 when it drops them.
+# At most _LENT_MAX bytes of results and _LENT_CAP of page-locked memory are out:
+# the library hands a result no more than twice its bytes, or one 2 MB grain.
+# What is not lent is copied, and the buffer is released at once.
+_LENT_MIN, _LENT_MAX, _LENT_CAP, _KEPT_CALLS = 64 << 10, 512 << 20, 1 << 30, 3
+_GRAIN = 2 << 20
+_lent = _lent_cap = _call = 0
+_out = {}    # address -> (bytes, capacity, call) of the lent buffers
+_calls = {}  # call -> how many of them
 _lent_mu = threading.RLock()  # a finaliser may run inside the locked region
 
 
-def _give_back(addr, nbytes):
-    global _lent
-    r = _abi.svdb_rec()
-    r.u = C.cast(addr, C.POINTER(C.c_double))
-    _abi.lib().svdb_rec_free(C.byref(r))
+def _give_back(addr, pid):
+    global _lent, _lent_cap
     with _lent_mu:
+        nbytes, cap, call = _out.pop(addr)
+        _calls[call] -= 1
+        if not _calls[call]:
+            del _calls[call]
         _lent -= nbytes
+        _lent_cap -= cap
+    if _pid == pid:  # a forked child's copy is its own memory
+        r = _abi.svdb_rec()
+        r.u = C.cast(addr, C.POINTER(C.c_double))
+        _abi.lib().svdb_rec_free(C.byref(r))
 
 
-def _take(r, name, count, shape, dtype):
+def _lend(addr, nbytes, call):
+    """Whether the buffer may leave with an array of results of `call`; counted if so."""
+    global _lent, _lent_cap
+    cap = max(2 * nbytes, _GRAIN)
+    with _lent_mu:
+        if _lent + nbytes > _LENT_MAX or _lent_cap + cap > _LENT_CAP:
+            return False
+        if sum(c < call - 1 for c in _calls) > _KEPT_CALLS:
+            return False
+        _out[addr] = (nbytes, cap, call)
+        _calls[call] = _calls.get(call, 0) + 1
+        _lent += nbytes
+        _lent_cap += cap
+    return True
+
+
+def _take(r, name, count, shape, dtype, call):
     """Array of the record's host buffer `name`; a lent buffer leaves the record."""
-    global _lent
     if count == 0:
         return np.zeros(shape, dtype=dtype)
     ptr = getattr(r, name)
-    nbytes = count * np.dtype(dtype).itemsize
-    with _lent_mu:
-        lend = nbytes >= _LENT_MIN and _lent + nbytes <= _LENT_MAX
-        if lend:
-            _lent += nbytes
-    if not lend:
+    nbytes = count * C.sizeof(ptr._type_)
+    addr = C.addressof(ptr.contents)
+    if nbytes < _LENT_MIN or not _lend(addr, nbytes, call):
         return np.ctypeslib.as_array(ptr, (count,)).copy().reshape(shape)
-    addr = C.cast(ptr, C.c_void_p).value
     buf = (ptr._type_ * count).from_address(addr)
-    weakref.finalize(buf, _give_back, addr, nbytes).atexit = False  # the process's end frees it anyway
+    weakref.finalize(buf, _give_back, addr, _pid).atexit = False  # the process's end frees it anyway
     setattr(r, name, None)
     return np.frombuffer(buf, dtype=dtype).reshape(shape)
 
 
-def rec_from_c(r) -> SvdRec:
-    """SvdRec from an svdb_rec (T = f64) or an svdb_rec_f32 (T = f32, float32 arrays)."""
+def next_call():
+    """Number of a library call, for the results it returns."""
+    global _call
+    with _lent_mu:
+        _call += 1
+        return _call
+
+
+# Page-locked memory is shared with a forked child: its writes would show in the
+# parent's arrays, and a buffer the parent reuses in the child's.  The child gets
+# private copies at the same addresses (heap buffers, which are never
+# page-aligned, are private already).
+_PAGE = mmap.PAGESIZE
+_fork_copies = []
+_pid = os.getpid()
+
+
+def _before_fork():
+    _lent_mu.acquire()
+    _fork_copies[:] = [(a, C.string_at(a, n)) for a, (n, _, _) in _out.items() if a % _PAGE == 0]
+
+
+def _after_fork_in_parent():
+    _fork_copies.clear()
+    _lent_mu.release()
+
+
+def _after_fork_in_child():
+    global _pid
+    _pid = os.getpid()
+    if _fork_copies:
+        libc = C.CDLL(None, use_errno=True)
+        libc.mmap.restype = C.c_void_p
+        libc.mmap.argtypes = [C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int, C.c_long]
+        fixed = 0x10  # MAP_FIXED
+        for a, data in _fork_copies:
+            size = (len(data) + _PAGE - 1) // _PAGE * _PAGE
+            got = libc.mmap(a, size, mmap.PROT_READ | mmap.PROT_WRITE, mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS | fixed,
+                            -1, 0)
+            if got == a:
+                C.memmove(a, data, len(data))
+    _fork_copies.clear()
+    _lent_mu.release()
+
+
+if hasattr(os, "register_at_fork"):
+    os.register_at_fork(before=_before_fork, after_in_parent=_after_fork_in_parent,
+                        after_in_child=_after_fork_in_child)
+
+
+def rec_from_c(r, call=None) -> SvdRec:
+    """SvdRec from an svdb_rec (T = f64) or an svdb_rec_f32 (T = f32, float32 arrays);
+    `call`: the next_call() of a library call that returns several."""
+    call = next_call() if call is None else call
     d = int(r.d)
     ur, uc, vr, vc = int(r.u_rows), int(r.u_cols), int(r.vt_rows), int(r.vt_cols)
     dtype = np.float32 if isinstance(r, _abi.svdb_rec_f32) else np.float64
 
-    u = _take(r, "u", ur * uc, (ur, uc), dtype)
-    s = _take(r, "s", d, (d,), dtype)
-    vt = _take(r, "vt", vr * vc, (vr, vc), dtype)
+    u = _take(r, "u", ur * uc, (ur, uc), dtype, call)
+    s = _take(r, "s", d, (d,), dtype, call)
+    vt = _take(r, "vt", vr * vc, (vr, vc), dtype, call)
     dg = r.diagnostics
     diag = Diagnostics(int(dg.non_zero), int(dg.dimensions), int(dg.iterations), bool(dg.transposed),
                        int(dg.lanczos_steps), int(dg.ritz_values_stabilized), int(dg.significant_values),

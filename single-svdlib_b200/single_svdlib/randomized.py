@@ -7,7 +7,7 @@ import enum
 import numpy as np
 
 from . import _abi
-from ._core import ShapeError, SvdRec, as_smat, check, options, rec_from_c
+from ._core import ShapeError, SvdRec, as_smat, check, next_call, options, rec_from_c
 
 
 class PowerIterationNormalizer(enum.Enum):
@@ -102,7 +102,8 @@ class RandomizedBatch:
         recs = (_abi.svdb_rec * self.count)()
         try:
             check(_abi.lib().svdb_batch_run(self._h, recs))
-            return [rec_from_c(recs[i]) for i in range(self.count)]
+            call = next_call()
+            return [rec_from_c(recs[i], call) for i in range(self.count)]
         finally:
             for i in range(self.count):
                 _abi.lib().svdb_rec_free(C.byref(recs[i]))
