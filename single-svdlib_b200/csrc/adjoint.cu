@@ -22,6 +22,7 @@
 
 #include "dense_tall.cuh"
 #include "device_common.cuh"
+#include "host_scratch.h"
 #include "ops.cuh"
 #include "svdb_internal.h"
 
@@ -435,10 +436,7 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
         if (!(sv[i] > 0.0) || !std::isfinite(sv[i]))
             throw Error(SVDB_ERR_ARG, "adjoint: singular values must be positive and finite");
 
-    cudaEvent_t e0, e1, e2;
-    SVDB_CUDA(cudaEventCreate(&e0));
-    SVDB_CUDA(cudaEventCreate(&e1));
-    SVDB_CUDA(cudaEventCreate(&e2));
+    ScopedEvent e0, e1, e2;
     SVDB_CUDA(cudaEventRecord(e0, s));
 
     DevBuf<double> U(m * k, s), V(n * k, s), GU(m * k, s), GV(n * k, s);
@@ -499,11 +497,8 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     SVDB_CUDA(cudaMemcpyAsync(R.p, Rhs.p, n * k * 8, cudaMemcpyDeviceToDevice, s));
     SVDB_CUDA(cudaMemcpyAsync(P.p, Rhs.p, n * k * 8, cudaMemcpyDeviceToDevice, s));
     // page-locked: the residual's copy does not hold the host, which enqueues on
-    struct HostBuf {
-        double* p;
-        ~HostBuf() { host_result_free(p); }
-    } hrr{(double*)host_result_alloc(64 << 10)};
-    double* rr = hrr.p;
+    HostScratch hrr(64 << 10, s);
+    double* rr = (double*)hrr.p;
     // column norms of rhs as the dots of R with itself (C1 = 0: the product adds nothing)
     SVDB_CUDA(cudaMemsetAsync(C1, 0, k * k * 8, s));
     gemm_tall<1>(cx, V.p, k, n, kk, C1, nullptr, kk, 0.0, R.p, k, 1.0, W.p, k);
@@ -523,8 +518,7 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     };
     double res = residual();
     uint64_t it = 0;
-    cudaEvent_t got;  // the residual's copy
-    SVDB_CUDA(cudaEventCreateWithFlags(&got, cudaEventDisableTiming));
+    ScopedEvent got(cudaEventDisableTiming);  // the residual's copy
     if (res > tol && it < max_it) spmm_dev<double, double>(Ar, false, P.p, kk, T.p, s);  // T = A P
     while (res > tol && it < max_it) {
         atb(cx, V.p, k, P.p, k, n, kk, kk, C1);                                           // C1 = V^T P
@@ -549,7 +543,6 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
         ++it;
         res = residual();
     }
-    cudaEventDestroy(got);
     o.cg_iterations = it;
     o.cg_residual = res;
 
@@ -617,9 +610,6 @@ void svd_adjoint(const svdb_matrix* A, int64_t k, const double* u, const double*
     cudaEventElapsedTime(&t2, e1, e2);
     o.time_ms_solve = t1;
     o.time_ms_sddmm = t2;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    cudaEventDestroy(e2);
     if (res > tol)
         throw Error(SVDB_ERR_NOCONV, "adjoint: block CG stopped at relative residual " + std::to_string(res) +
                                          " after " + std::to_string(it) + " iterations");

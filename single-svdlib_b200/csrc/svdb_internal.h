@@ -52,6 +52,16 @@ inline void allow_smem(F kern, size_t bytes) {
         SVDB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
+// An event of the current device, destroyed with its scope.
+struct ScopedEvent {
+    cudaEvent_t e = nullptr;
+    explicit ScopedEvent(unsigned flags = cudaEventDefault) { SVDB_CUDA(cudaEventCreateWithFlags(&e, flags)); }
+    ScopedEvent(const ScopedEvent&) = delete;
+    ScopedEvent& operator=(const ScopedEvent&) = delete;
+    ~ScopedEvent() { cudaEventDestroy(e); }
+    operator cudaEvent_t() const { return e; }
+};
+
 // --------------------------------------------------------- device memory ----
 // Owning device buffer, stream-ordered (cudaMallocAsync pool).
 template <typename T>
