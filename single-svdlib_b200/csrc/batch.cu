@@ -584,7 +584,10 @@ __global__ void __launch_bounds__(kBLeanWarps * 32, NL == 3 ? 2 : 3)
 
 // --------------------------------------------------------- CholeskyQR2 ----
 // Gram partials: block (chunk, b) sums X_b^T X_b over its rows on the FP64
-// matrix instruction (dense_tall.cuh), the tile blocks I <= J only.  At FP32
+// matrix instruction (dense_tall.cuh), the tile blocks I <= J only.  The number of
+// chunks depends on m alone, so that a subset's results do not depend on how many
+// others the batch has (one wave of CTAs over all subsets was 10 % faster for one
+// or two subsets of 20,000 rows, 2 % for sixteen).  At FP32
 // the chunks are sixteenths of the rows, each summed in row order by one warp
 // per tile block (rg = 1, small blocks, so that there are enough warps), and
 // the sixteen are added in one order whatever the batch: X R^-1 is rounded to
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_b_gram_part(con
 
 // G_b = sum of the subset's partials in chunk order (elements of tile blocks
 // below the diagonal are not read by the factorisation and stay undefined)
-constexpr int kGramChunks = 16;  // of a mixed batch
+constexpr int kGramChunks = 16;  // of a mixed batch, and at most at FP64
 __global__ void k_b_gram_reduce16(const double* __restrict__ part, int c, double* __restrict__ G,
                                   const int* __restrict__ cond) {
     const int64_t b = blockIdx.y;
@@ -1152,10 +1155,8 @@ void batch_create(const svdb_matrix* A, const uint64_t* col_off, const uint64_t*
         B->Om64.alloc(tc * ld, s); B->Y64.alloc(count * m * ld, s); B->Z64.alloc(tc * ld, s);
     }
     B->Bt.alloc(tc * ld, s);
-    // one CTA per SM over all subsets (four waves of short ones took 59 us, one
-    // 54, in the mixed solve of 16 subsets of 20,000 x 6,000), none of them below 256 rows
-    B->gram_parts = (int)std::max<int64_t>(
-        1, std::min<int64_t>((int64_t)device_props().sms / (int64_t)count, (m + 255) / 256));
+    // chunks of the FP64 Grams: none below 256 rows, whatever the number of subsets
+    B->gram_parts = (int)std::max<int64_t>(1, std::min<int64_t>(kGramChunks, (m + 255) / 256));
     B->part.alloc(count * std::max(B->gram_parts, B->mixed ? kGramChunks : 1) * l * l, s);
     for (DevBuf<double>* p : {&B->G, &B->R1, &B->R2, &B->R3, &B->Ri, &B->Rout, &B->Rtmp, &B->Ur, &B->Vr})
         p->alloc(count * l * l, s);
