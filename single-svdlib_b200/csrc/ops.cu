@@ -37,15 +37,12 @@ int group_for(double avg) {
 // bound on the blocks, 131, 124 and 111 compiled for five blocks an SM (48
 // registers in both types), 139, 133 and 117 for four, 161, 154 and 129 for
 // eight (spills).  Uniform 100,000 x 20,000 (20 M): 78 and 82 -> 60 and 73 us.
-// The last two arguments are unused and bring the arguments to 160 bytes.  A
-// small product is bound by the host's launches, and their cost went with the
-// arguments' size: 3.7-3.8 us per call at 160 and 224 bytes, 4.05 at 152,
-// 4.3-4.6 at 144, 176 and 192.
+// A small product is bound by the host's launches, whose cost follows the size
+// of the arguments (96 bytes: bins counted in 32 bits).
 template <typename VT>
 __global__ void __launch_bounds__(256, 5) k_spmv(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                               const VT* __restrict__ v, const __grid_constant__ SpmvBins bins,
-                                              const double* __restrict__ x, double* __restrict__ y, int64_t,
-                                              int64_t) {
+                                              const double* __restrict__ x, double* __restrict__ y) {
     __shared__ double sh[32];
     auto xl = [&](int32_t c) { return __ldg(x + c); };
     spmv_deal(blockIdx.x, gridDim.x, bins.off[0], [&](int64_t i) {
@@ -89,13 +86,13 @@ void spmv(const DevCompressed& m, bool fp32, const double* x, double* y, cudaStr
     if (allow_sliced && !sliced_off() && spmv_sliced(m, f, x, y, s)) return;
     // an item for every warp: a warp's second item lengthened a 5000 x 2000 product, whose chain of
     // loads is all its time, from 2.7 to 3.6 us
-    const int64_t work = std::max<int64_t>((m.plan.bins.items[kSpmvBins] + 7) / 8, m.plan.nlong);
+    const int64_t work = std::max<int64_t>(((int64_t)m.plan.bins.items[kSpmvBins] + 7) / 8, m.plan.nlong);
     if (f) {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<float>()));
-        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, x, y, 0, 0);
+        k_spmv<float><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val32.p, m.plan.bins, x, y);
     } else {
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(work, spmv_grid<double>()));
-        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, x, y, 0, 0);
+        k_spmv<double><<<blocks, 256, 0, s>>>(m.ptr.p, m.idx.p, m.val.p, m.plan.bins, x, y);
     }
     SVDB_CHECK_LAUNCH();
 }

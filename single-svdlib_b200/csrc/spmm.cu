@@ -667,13 +667,13 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     int64_t off = p.nlong, items = 0;
     for (int b = 0; b < kSpmvBins; ++b) {
         const int64_t cnt = (int64_t)hm[3 + b], rpw = (int64_t)1 << b;
-        p.bins.off[b] = off;
-        p.bins.items[b] = items;
+        p.bins.off[b] = (int32_t)off;
+        p.bins.items[b] = (int32_t)items;
         off += cnt;
         items += (cnt + rpw - 1) / rpw;
     }
-    p.bins.off[kSpmvBins] = off;
-    p.bins.items[kSpmvBins] = items;
+    p.bins.off[kSpmvBins] = (int32_t)off;
+    p.bins.items[kSpmvBins] = (int32_t)items;
     p.bins.rows = p.bin_rows.p;
     // the cut rows head the same order (its length and kCutMax are class bounds)
     p.cut.rows = p.bin_rows.p;

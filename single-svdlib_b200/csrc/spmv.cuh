@@ -65,12 +65,13 @@ __device__ __forceinline__ void spmv_binned(const int64_t* __restrict__ rp, cons
                                             const VT* __restrict__ v, const SpmvBins& bins, int64_t warp0,
                                             int64_t nwarps, XL xload, FIN fin) {
     const int lane = threadIdx.x & 31;
-    spmv_deal(warp0, nwarps, bins.items[kSpmvBins], [&](int64_t it) {
+    spmv_deal(warp0, nwarps, bins.items[kSpmvBins], [&](int64_t item) {
+        const int32_t it = (int32_t)item;
         int b = 0;
         while (b + 1 < kSpmvBins && it >= bins.items[b + 1]) ++b;
         const int G = 32 >> b;
         const int sub = lane & (G - 1);
-        const int64_t p = bins.off[b] + ((it - bins.items[b]) << b) + lane / G;
+        const int32_t p = bins.off[b] + ((it - bins.items[b]) << b) + lane / G;
         const bool valid = p < bins.off[b + 1];
         double acc = 0.0;
         int64_t r = 0;

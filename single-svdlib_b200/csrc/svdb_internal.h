@@ -114,8 +114,8 @@ constexpr int kSpmvBins = 5;
 __host__ __device__ constexpr int64_t spmv_bin_len(int b) { return b ? 128 >> b : kSegNnz; }
 struct SpmvBins {
     const int32_t* rows;             // bin_rows
-    int64_t off[kSpmvBins + 1];      // bin b: rows[off[b] .. off[b+1]); off[0] = nlong
-    int64_t items[kSpmvBins + 1];    // warp items before bin b (1 << b rows per item)
+    int32_t off[kSpmvBins + 1];      // bin b: rows[off[b] .. off[b+1]); off[0] = nlong
+    int32_t items[kSpmvBins + 1];    // warp items before bin b (1 << b rows per item)
 };
 // The rows of more than len entries as k_spmm_cut's blocks take them: rows[0 ..
 // first[0]) have more than kCutMax; rows[first[k] .. first[k + 1]) take 8 >> k
