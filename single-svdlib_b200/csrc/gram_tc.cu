@@ -21,7 +21,7 @@
 // reads its 32 TMEM lanes (tcgen05.ld 32x32b), warps 2-3 hand D's rows 64..127
 // over through shared memory, and warps 0-1 write the CTA's FP64 partial
 // D[i][j] + D[64+i][j] + D2[i][j]; the partials are summed in block order by
-// k_gram_reduce.  Waits give up after 2 s (g_gram_tc_err).
+// k_tn_reduce.  Waits give up after 2 s (g_gram_tc_err).
 #include <algorithm>
 
 #include "device_common.cuh"
