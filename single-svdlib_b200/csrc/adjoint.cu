@@ -105,9 +105,14 @@ __global__ void __launch_bounds__(256, MINB) k_sddmm(const int32_t* __restrict__
                 for (int u = 0; u < U; ++u) {
                     p[u] = T(0);
 #pragma unroll
-                    for (int j = 0; j < NL; ++j)
+                    for (int j = 0; j < NL; ++j) {
+                        // four columns a vector (FP32): a chain per vector, then their sum, which
+                        // rounds as often as a lane per column and a tree (one chain: 6 % further off)
+                        T t = VEC > 2 ? T(0) : p[u];
 #pragma unroll
-                        for (int e = 0; e < VEC; ++e) p[u] = fma(lv[j].v[e], x[u][j].v[e], p[u]);
+                        for (int e = 0; e < VEC; ++e) t = fma(lv[j].v[e], x[u][j].v[e], t);
+                        p[u] = VEC > 2 && j ? p[u] + t : t;
+                    }
                 }
 #pragma unroll
                 for (int n = U / 2, w = GL / 2; w >= 1; w >>= 1, n >>= 1) {
