@@ -506,7 +506,8 @@ __global__ void k_spmm_merge(const int64_t* __restrict__ seg_first, const int32_
 //    1.1 M, A^T X, l = 60, FP64, three streams: 42 us a call against 36), at twice
 //    the mean the chains are back (2,000 x 2,000, 0.47 M: 39 us against 25).
 //  - Above, cut rows are merged from partials (k_spmm_merge), whose allocation and
-//    launch no longer show: four segments a warp.  At 2,048 throughout, A^T X of a
+//    launch no longer outweigh the balance: four segments a warp (but where the
+//    rows are even enough: cut_in_blocks).  At 2,048 throughout, A^T X of a
 //    30,011 x 8,009 matrix (3.1 M, columns up to a few thousand entries, l = 40)
 //    took 196 us, at 256 85.
 // kCutNnz: A^T X, l = 60, FP64, alone / on three streams, by blocks and merged: at
@@ -679,7 +680,7 @@ void build_seg_plan(DevCompressed& m, cudaStream_t s) {
     p.cut.rows = p.bin_rows.p;
     p.cut.len = (int)cut;
     for (int k = 0; k < 4; ++k) p.cut.first[k] = (int)hm[3 + kSpmvBins + k];
-    p.cut.blocks = m.nnz < kCutNnz ? p.cut.items(0) + p.cut.items(1) + p.cut.items(2) : 0;
+    p.cut.blocks = m.nnz < 2 * kCutNnz ? p.cut.items(0) + p.cut.items(1) + p.cut.items(2) : 0;
 }
 
 // ------------------------------------------------------------- launcher --
@@ -712,11 +713,35 @@ static bool lean_aligned(const DevCompressed& m, const T* X, int64_t ldx) {
            m.nminor * ldx < ((int64_t)1 << 31);
 }
 
-// k_spmm_cut takes every cut row: no partials, no merge
-static bool cut_in_blocks(const DevCompressed& m) { return m.plan.cut.blocks > 0 && m.plan.cut.first[0] == 0; }
+// Of the structures that have rows of several segments, those whose products of l
+// columns k_spmm_cut does in one kernel, without partials and their merge:
+//  - below kCutNnz, where no row is longer than kCutMax;
+//  - up to 64 columns to twice that, where no row is longer than 4 cut.len;
+//  - above, where no row is longer than cut.len: every row is then one warp's.
+//    Above 64 columns only up to 512 entries: there a warp has one row of X in
+//    flight per vector, and the longer chains show.
+// In one kernel and merged, A X, alone / on one stream in turn: 45,477 x 21,986
+// (2.8 M, rows of up to 374) at l = 24, FP64, 67 / 60 and 88 / 64 us; 32,169 x 10,970
+// (3.9 M, up to 540) at l = 60, FP32, 82 / 74 and 96 / 80; 8,465 x 6,126 (2.3 M, up
+// to 910) at l = 44, FP32, 55 / 47 and 66 / 50; and where it is merged, 23,109 x
+// 11,277 (3.9 M, up to 964) at l = 120, FP32, 166 / 158 and 153 / 137; A^T X of
+// 12,889 x 6,080 (2.4 M, up to 3,705) at l = 64, FP32, 61 / 53 and 65 / 49.
+static bool cut_in_blocks(const DevCompressed& m, int l) {
+    const CutRows& cut = m.plan.cut;
+    if (m.plan.nmulti == 0 || cut.first[0] > 0) return false;
+    if (m.nnz < kCutNnz || (m.nnz < 2 * kCutNnz && l <= 64 && cut.first[1] == 0)) return true;
+    return cut.first[3] == 0 && (l <= 64 || cut.len <= 512);
+}
+
+// How launch_lean's kernels go over the rows
+enum class Rows {
+    kSegments,  // k_spmm_lean, a segment a warp; rows of several leave partials
+    kWhole,     // k_spmm_cut
+    kNarrow     // k_spmm_cut, X read element by element
+};
 
 template <typename T, typename OT, int H, int NL, int U, int MINB>
-static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
+static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, Rows form, OT* Y,
                     int64_t ldy, double* part, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(T);
     // 8x the resident blocks: timed against the resident blocks only, 1.10
@@ -724,13 +749,13 @@ static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64
     const int work = nblk(m.plan.nseg * 32, kLeanWarps * 32, MINB * 8);
     const int yvec = ldy % VEC == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     const bool bytes = m.nminor * ldx * (int64_t)sizeof(T) < ((int64_t)1 << 32);
-    if (narrow || cut_in_blocks(m)) {
+    if (form != Rows::kSegments) {
         const CutRows& cut = m.plan.cut;
         auto go = [&](auto kern) {
             kern<<<cut.blocks + work, kLeanWarps * 32, (size_t)kLeanWarps * (32 / H) * NL * 16 / sizeof(T) * 8, s>>>(
                 m.idx.p, v, m.ptr.p, m.nmajor, cut, X, (uint32_t)ldx, l, Y, (int)ldy, yvec);
         };
-        if (narrow) go(k_spmm_cut<T, OT, 1, H, NL * VEC, 4, MINB, true>);  // four rows in flight: more spill
+        if (form == Rows::kNarrow) go(k_spmm_cut<T, OT, 1, H, NL * VEC, 4, MINB, true>);  // four rows in flight: more spill
         else if (bytes) go(k_spmm_cut<T, OT, VEC, H, NL, U, MINB, true>);
         else go(k_spmm_cut<T, OT, VEC, H, NL, U, MINB, false>);
     } else {
@@ -745,24 +770,24 @@ static void lean_go(const DevCompressed& m, const T* v, const T* X, int l, int64
 }
 
 // l <= 128 columns of X (ldx apart) into Y (ldy apart).  Lane groups as narrow
-// as the columns allow, so that few lanes idle.  narrow: X is read element by
-// element, VEC times the vectors a lane in the same groups.
+// as the columns allow, so that few lanes idle.  kNarrow has VEC times the vectors
+// a lane in the same groups.
 template <typename T, typename OT>
-static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
+static void launch_lean(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, Rows form, OT* Y,
                         int64_t ldy, double* part, cudaStream_t s) {
     if (m.plan.nseg <= 0) return;
     if constexpr (std::is_same<T, float>::value) {
-        if (l <= 16) lean_go<T, OT, 8, 1, 4, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 32) lean_go<T, OT, 4, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 64) lean_go<T, OT, 2, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else lean_go<T, OT, 1, 1, 8, 4>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        if (l <= 16) lean_go<T, OT, 8, 1, 4, 4>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 1, 8, 4>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 1, 8, 4>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 1, 8, 4>(m, v, X, l, ldx, form, Y, ldy, part, s);
     } else {
-        if (l <= 8) lean_go<T, OT, 8, 1, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 16) lean_go<T, OT, 4, 1, 8, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 32) lean_go<T, OT, 4, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 48) lean_go<T, OT, 4, 3, 4, 2>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else if (l <= 64) lean_go<T, OT, 2, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
-        else lean_go<T, OT, 1, 2, 4, 3>(m, v, X, l, ldx, narrow, Y, ldy, part, s);
+        if (l <= 8) lean_go<T, OT, 8, 1, 4, 3>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 16) lean_go<T, OT, 4, 1, 8, 3>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 32) lean_go<T, OT, 4, 2, 4, 3>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 48) lean_go<T, OT, 4, 3, 4, 2>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else if (l <= 64) lean_go<T, OT, 2, 2, 4, 3>(m, v, X, l, ldx, form, Y, ldy, part, s);
+        else lean_go<T, OT, 1, 2, 4, 3>(m, v, X, l, ldx, form, Y, ldy, part, s);
     }
 }
 
@@ -832,12 +857,13 @@ static const T* lean_operand(const DevCompressed& m, const T* X, int l, int64_t&
 template <typename T, typename OT>
 static void lean_product(const DevCompressed& m, const T* v, const T* X, int l, int64_t ldx, bool narrow, OT* Y,
                          int64_t ldy, cudaStream_t s) {
-    const int64_t merged = narrow || cut_in_blocks(m) ? 0 : m.plan.nmulti;
+    const Rows form = narrow ? Rows::kNarrow : cut_in_blocks(m, l) ? Rows::kWhole : Rows::kSegments;
+    const int64_t merged = form == Rows::kSegments ? m.plan.nmulti : 0;
     DevBuf<double> part;
     if (merged) part.alloc(m.plan.nseg * (int64_t)std::min(l, 128), s);
     for (int c0 = 0; c0 < l; c0 += 128) {
         const int lc = std::min(128, l - c0);
-        launch_lean<T, OT>(m, v, X + c0, lc, ldx, narrow, Y + c0, ldy, part.p, s);
+        launch_lean<T, OT>(m, v, X + c0, lc, ldx, form, Y + c0, ldy, part.p, s);
         if (merged) merge_rows(m, part.p, lc, Y + c0, ldy, s);
     }
 }

@@ -119,7 +119,8 @@ struct SpmvBins {
 };
 // The rows of more than len entries as k_spmm_cut's blocks take them: rows[0 ..
 // first[0]) have more than kCutMax; rows[first[k] .. first[k + 1]) take 8 >> k
-// warps each, 1 << k of them a block.  blocks: 0 where all are merged from partials.
+// warps each, 1 << k of them a block.  blocks: 0 where there are none or all are
+// merged from partials.
 constexpr int64_t kCutMax = 8 * kSegNnz;
 struct CutRows {
     const int32_t* rows;  // bin_rows
